@@ -3417,6 +3417,8 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     SketchArgs a{};
     a.seq = d_seq;
     a.seq_off = dp.roff;
+    a.base0 = bp.roff[0];
+    a.base1 = bp.roff[(size_t)n];
     a.chunk_off = dp.chunk_off;
     a.n_seq = n;
     a.n_chunks = bp.chunk_off[(size_t)n];

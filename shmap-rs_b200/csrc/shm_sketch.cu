@@ -12,17 +12,15 @@
 #include "shm_common.cuh"
 #include "shm_prims.cuh"
 #include "shm_sketch.cuh"
+#include "shm_sketch_dev.cuh"
 #include "shm_tune.hpp"
 
 #include <cstdlib>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 namespace shm {
-
-struct SketchLuts {
-    uint64_t fw[256], rc[256], fw_k[256], rc_r1[256], rc_k1[256];
-};
 
 // Built on the host once per (k) exactly as src/sketch.rs:58-108 does.
 void build_luts(int32_t k, SketchLuts* L) {
@@ -263,8 +261,6 @@ struct PkTables {
     uint4 w1[4];       // one base: (fw, rc_k1)
 };
 
-__device__ __forceinline__ uint64_t u64_of(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
-
 __device__ void build_pk_tables(PkTables& P, const SketchLuts* __restrict__ L) {
     const unsigned char let[4] = {'A', 'C', 'T', 'G'};
     for (int e = threadIdx.x; e < 32 * 16; e += blockDim.x) {
@@ -306,11 +302,6 @@ __device__ void build_pk_tables(PkTables& P, const SketchLuts* __restrict__ L) {
 // before it, whatever it holds) is the warm-up's: that byte enters and
 // leaves through the same code, so it cancels.
 constexpr int FR_CAP = 32;
-
-// Code byte of four letters (the earliest in bits 0-1): the codes sit at
-// bits 0-1 of each byte after the shift and mask; the multiply gathers byte
-// i's code at bits 24 + 2i with no carry into them from the other products.
-__device__ __forceinline__ uint32_t codes4(uint32_t w) { return (((w >> 1) & 0x03030303u) * 0x01041040u) >> 24; }
 
 // Nonzero unless the four bytes of w are letters A, C, G, T of either case:
 // the byte that a letter of the same code would be (A, C, T, G = 0x41 +
@@ -813,22 +804,60 @@ __global__ void __launch_bounds__(SK_THREADS) k_sketch_pk(SketchArgs a, const Sk
 }
 
 SketchLuts* create_device_luts(int32_t k, cudaStream_t s) {
-    SketchLuts h;
-    build_luts(k, &h);
-    SketchLuts* d = nullptr;
-    SHM_CUDA(cudaMalloc(&d, sizeof(SketchLuts)));
+    SketchTabs h;
+    build_luts(k, &h.luts);
+    // what a group of four bases (codes A, C, T, G = 0..3) XORs into a window's hashes
+    const unsigned char let[4] = {'A', 'C', 'T', 'G'};
+    auto rl = [](uint64_t x, uint32_t n) { n &= 63; return n ? (x << n) | (x >> (64 - n)) : x; };
+    for (int g = 0; g < 8; g++)
+        for (int c = 0; c < 256; c++) {
+            uint64_t f = 0, r = 0;
+            for (int i = 4 * g; i < 4 * g + 4 && i < k; i++) {
+                const unsigned char b = let[(c >> (2 * (i & 3))) & 3];
+                f ^= rl(h.luts.fw[b], (uint32_t)(k - 1 - i));
+                r ^= rl(h.luts.rc[b], (uint32_t)i);
+            }
+            h.wt[g][c] = make_uint4((uint32_t)f, (uint32_t)(f >> 32), (uint32_t)r, (uint32_t)(r >> 32));
+        }
+    SketchTabs* d = nullptr;
+    SHM_CUDA(cudaMalloc(&d, sizeof(SketchTabs)));
     SHM_CUDA(cudaMemcpyAsync(d, &h, sizeof h, cudaMemcpyHostToDevice, s));
     SHM_CUDA(cudaStreamSynchronize(s));
-    return d;
+    return &d->luts;  // the first member
+}
+
+// The instances of the bit-plane kernels (an object each: shm_sketch_bits.cu).
+// They hold two words of bases a window (k <= 33) and tables of eight groups
+// of four bases (k <= 32); below 15 a k-mer says little about a genome's
+// place and the rolling kernels stay. At every hash ratio the bit planes are
+// the faster (0.092 Gbases, k = 25, ms on bit planes / rolled: letters 0.07 /
+// 0.16 at r = 0.01, 0.55 / 1.57 at 0.25, 2.65 / 7.49 at 1; packed 0.07 / 0.16,
+// 0.48 / 0.93, 2.32 / 5.54).
+constexpr int SKB_KMIN = 15, SKB_KMAX = 32;
+template <int K>
+void launch_sketch_bits_k(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s);
+template <int... I>
+static void launch_bits_of(int k, const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s,
+                           std::integer_sequence<int, I...>) {
+    (void)((k == SKB_KMIN + I ? (launch_sketch_bits_k<SKB_KMIN + I>(a, tabs, s), true) : false) || ...);
+}
+bool sketch_bits_takes(int32_t k) { return k >= SKB_KMIN && k <= SKB_KMAX; }
+void launch_sketch_bits(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s) {
+    launch_bits_of(a.k, a, tabs, s, std::make_integer_sequence<int, SKB_KMAX - SKB_KMIN + 1>{});
 }
 
 void launch_sketch(int mode, const SketchArgs& a, const SketchLuts* L, cudaStream_t s) {
     if (a.n_chunks == 0) return;
     const bool pk = a.pk_codes != nullptr;
     if (pk && mode != SK_APPEND) throw shm_cuda_error(cudaErrorInvalidValue);
+    // reads go through the bit planes where their k has an instance; other
     // packed reads roll in the rotated frame (k_sketch_pk); SHMAP_SKETCH_LETTERS=1
-    // rolls them through the letter tables instead (the same selections)
+    // rolls all of them from their letters instead (the same selections)
     static const bool letters = std::getenv("SHMAP_SKETCH_LETTERS") != nullptr;
+    if (mode == SK_APPEND && !letters && a.base1 > a.base0 && sketch_bits_takes(a.k)) {
+        launch_sketch_bits(a, (const SketchTabs*)L, s);
+        return;
+    }
     if (pk && !letters) {
         const uint64_t n_tiles = (a.n_chunks + SK_THREADS - 1) / SK_THREADS;
         k_sketch_pk<SK_APPEND><<<grid_for(n_tiles, 1, (int)tuning().sketch_ctas_per_sm), SK_THREADS, 0, s>>>(a, L);
@@ -911,7 +940,8 @@ void launch_fill_luts(SketchLuts* d, int32_t k, cudaStream_t s) {
 // reads packed on the host (packed != 0, the host-buffer path's layout) or
 // from their bytes. Read i's k-mers go unordered to out_h/out_rs from
 // cap_off[i] (at most cap_off[i+1] - cap_off[i] of them); out_cnt[i] gets
-// their number. Allocates its own device buffers.
+// their number. The device copy keeps offs[0] & 31 bytes before the first
+// read, so that it starts at that offset there. Allocates its own device buffers.
 #include "../host/pack.hpp"
 #include "shm_internal.hpp"
 
@@ -929,10 +959,11 @@ extern "C" int shm_internal_sketch_reads(int device, const uint8_t* seqs, const 
     };
     try {
         SHM_CUDA(cudaSetDevice(device));
-        const int64_t nb = offs[n] - offs[0];
+        const int64_t lead = offs[0] & 31, nb = offs[n] - offs[0] + lead;
+        const uint8_t* from = seqs + (offs[0] - lead);
         std::vector<int64_t> so((size_t)n + 1);
         std::vector<uint64_t> co((size_t)n + 1, 0);
-        for (int32_t i = 0; i <= n; i++) so[(size_t)i] = offs[i] - offs[0];
+        for (int32_t i = 0; i <= n; i++) so[(size_t)i] = offs[i] - offs[0] + lead;
         for (int32_t i = 0; i < n; i++) {
             const int64_t nw = so[(size_t)i + 1] - so[(size_t)i] - k + 1;
             co[(size_t)i + 1] = co[(size_t)i] + (nw > 0 ? (uint64_t)((nw + SKETCH_WIN - 1) / SKETCH_WIN) : 0);
@@ -955,7 +986,7 @@ extern "C" int shm_internal_sketch_reads(int device, const uint8_t* seqs, const 
         SHM_CUDA(cudaMemset(d_kc, 0, 4 * (size_t)std::max(n, 1)));
         if (packed) {
             std::vector<uint32_t> cw(packed_code_words(nb)), mw(packed_mask_words(nb));
-            pack_reads_host(seqs + offs[0], nb, cw.data(), mw.data());
+            pack_reads_host(from, nb, cw.data(), mw.data());
             auto* d_cw = (uint32_t*)dalloc(4 * cw.size());
             auto* d_mw = (uint32_t*)dalloc(4 * mw.size());
             SHM_CUDA(cudaMemcpy(d_cw, cw.data(), 4 * cw.size(), cudaMemcpyHostToDevice));
@@ -966,10 +997,12 @@ extern "C" int shm_internal_sketch_reads(int device, const uint8_t* seqs, const 
         } else {
             auto* d_seq = (uint8_t*)dalloc((size_t)nb + 32);
             SHM_CUDA(cudaMemset(d_seq, 0, (size_t)nb + 32));
-            if (nb) SHM_CUDA(cudaMemcpy(d_seq, seqs + offs[0], (size_t)nb, cudaMemcpyHostToDevice));
+            if (nb) SHM_CUDA(cudaMemcpy(d_seq, from, (size_t)nb, cudaMemcpyHostToDevice));
             a.seq = d_seq;
         }
         a.seq_off = d_so;
+        a.base0 = so[0];
+        a.base1 = so[(size_t)n];
         a.chunk_off = d_co;
         a.kmer_off = d_ko;
         a.kmer_cnt = d_kc;

@@ -39,12 +39,19 @@ struct SketchArgs {
     const uint32_t* pk_codes;
     const uint32_t* pk_mask;
     uint64_t pk_words;  // code words readable at pk_codes (those past it read as 0)
+    // SK_APPEND only: seq_off[0] and seq_off[n_seq] on the host, when the caller has
+    // them and `luts` is of create_device_luts (the bit-plane kernels take the call then)
+    int64_t base0, base1;
 };
 
 // The five lookup tables of src/sketch.rs:50-97 for one k, in device memory
 // (owned by the caller, released with cudaFree).
 struct SketchLuts;
 SketchLuts* create_device_luts(int32_t k, cudaStream_t s);
+// The bit-plane kernels (shm_sketch_bits.cuh) take an SK_APPEND call of this k.
+bool sketch_bits_takes(int32_t k);
+struct SketchTabs;
+void launch_sketch_bits(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s);
 void launch_sketch(int mode, const SketchArgs& a, const SketchLuts* luts, cudaStream_t s);
 
 // Builds the tables on the device into caller-provided device memory of

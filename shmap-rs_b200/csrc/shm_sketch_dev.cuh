@@ -1,0 +1,27 @@
+// Device pieces shared by the sketch kernels.
+#pragma once
+#include <stdint.h>
+
+namespace shm {
+
+struct SketchLuts {
+    uint64_t fw[256], rc[256], fw_k[256], rc_r1[256], rc_k1[256];
+};
+
+// The tables of one k as create_device_luts makes them: the byte tables, and
+// for the windows' full hashes a table per group of four bases (SKB kernels):
+// wt[g][codes] is what bases 4g .. 4g + 3 of a window XOR into (F, R), as (F
+// low, high, R low, high); bases past k contribute nothing.
+struct SketchTabs {
+    SketchLuts luts;
+    uint4 wt[8][256];
+};
+
+__device__ __forceinline__ uint64_t u64_of(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
+
+// Code byte of four letters (the earliest in bits 0-1): the codes sit at
+// bits 0-1 of each byte after the shift and mask; the multiply gathers byte
+// i's code at bits 24 + 2i with no carry into them from the other products.
+__device__ __forceinline__ uint32_t codes4(uint32_t w) { return (((w >> 1) & 0x03030303u) * 0x01041040u) >> 24; }
+
+}  // namespace shm
