@@ -106,6 +106,7 @@ struct MapCtx {
     int rchip_smem_set = 0;  // k_refine_chip's dynamic shared memory allowed
     int refine_smem_set = 0; // k_refine's
     int seedc_smem_set = 0;
+    int lcs_smem_set = 0;    // k_lcs_occ's
     // stage timing
     bool timing = false;
     double stage_ms[N_STAGES] = {};
