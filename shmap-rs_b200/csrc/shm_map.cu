@@ -2811,33 +2811,40 @@ __global__ void __launch_bounds__(RCHIP_WARPS * 32, 4) k_refine_chip(BatchView v
     uint16_t* cntA = (uint16_t*)(base + RCHIP_OFF_CNT);
     uint16_t* ring = (uint16_t*)(base + RCHIP_OFF_RING);
     uint32_t* smask = (uint32_t*)(base + RCHIP_OFF_MASK);
-    // work comes in chunks of RCHIP_CHUNK consecutive candidates (a read's
-    // candidates are consecutive) from a batch counter, the next chunk's
-    // number fetched while this one is refined; the seed table is rebuilt
-    // only when the read changes
-    const uint32_t ncand = v.coff[v.n];
+    // work comes in chunks of consecutive reads (pass 0 of two: a read's one
+    // lead) or consecutive candidates (a read's are consecutive) from a batch
+    // counter, the next chunk's number fetched while this one is refined; the
+    // seed table is rebuilt only when the read changes. A chunk's candidates
+    // are refined one after the other, so chunks grow to RCHIP_CHUNK only as
+    // the batch gives every warp several of them.
+    const bool leads = v.lead_on && pass == 0;
+    const uint32_t n_work = leads ? (uint32_t)v.n : v.coff[v.n];
+    const uint32_t chunk = min((uint32_t)RCHIP_CHUNK, max(1u, n_work / (4u * RCHIP_WARPS * gridDim.x)));
     uint32_t nxt = 0;
     if (lane == 0) nxt = atomicAdd(&v.mx->refine_next[pass], 1u);
     int32_t cur = -1;  // the read whose table is staged
     uint32_t T = 32;
     for (;;) {
-        const uint32_t ci0 = __shfl_sync(0xffffffffu, nxt, 0) * (uint32_t)RCHIP_CHUNK;
-        if (ci0 >= ncand) break;
+        const uint32_t ci0 = __shfl_sync(0xffffffffu, nxt, 0) * chunk;
+        if (ci0 >= n_work) break;
         if (lane == 0) nxt = atomicAdd(&v.mx->refine_next[pass], 1u);
         int32_t ql = -1;
-        bool onl = false;
-        if (lane < RCHIP_CHUNK && ci0 + lane < ncand) {
-            const uint32_t ji = v.cidx[ci0 + lane];
-            const BucketJob& Jl = v.jobs[ji];
-            ql = Jl.read;
-            onl = refine_on_chip(v.P, (uint32_t)v.r_m[ql], v.r_half[ql]) && refined_in(v, Jl, ji, pass);
+        uint32_t jl = UINT32_MAX;
+        if (lane < chunk && ci0 + lane < n_work) {
+            jl = leads ? v.r_lead[ci0 + lane] : v.cidx[ci0 + lane];
+            if (jl != UINT32_MAX) {
+                const BucketJob& Jl = v.jobs[jl];
+                ql = leads ? (int32_t)(ci0 + lane) : Jl.read;
+                if (!refine_on_chip(v.P, (uint32_t)v.r_m[ql], v.r_half[ql]) || !(leads || refined_in(v, Jl, jl, pass)))
+                    jl = UINT32_MAX;  // k_refine's, or not refined in this pass
+            }
         }
-        const unsigned on_mask = __ballot_sync(0xffffffffu, onl);
+        const unsigned on_mask = __ballot_sync(0xffffffffu, jl != UINT32_MAX);
         if (lane == 0 && on_mask) atomicAdd(&v.mx->refined, (unsigned long long)__popc(on_mask));
-        const uint32_t nc = min((uint32_t)RCHIP_CHUNK, ncand - ci0);
-        for (uint32_t j = 0; j < nc; j++) {
-            const int32_t q = __shfl_sync(0xffffffffu, ql, (int)j);
-            if (!__shfl_sync(0xffffffffu, onl, (int)j)) continue;  // k_refine's, or not refined in this pass
+        for (unsigned mk = on_mask; mk; mk &= mk - 1) {
+            const int src = __ffs(mk) - 1;
+            const int32_t q = __shfl_sync(0xffffffffu, ql, src);
+            const uint32_t ji = __shfl_sync(0xffffffffu, jl, src);
             const int32_t m = v.r_m[q], n_u = v.r_nu[q];  // n_u <= m <= RCHIP_M
             if (q != cur) {
                 const uint64_t kb = v.kcap_off[q];
@@ -2854,8 +2861,8 @@ __global__ void __launch_bounds__(RCHIP_WARPS * 32, 4) k_refine_chip(BatchView v
                 __syncwarp();
                 cur = q;
             }
-            refine_chip_one(v, v.jobs + v.cidx[ci0 + j], m, n_u, (int64_t)v.r_half[q], T, tslot, shash, sinfo, cntA,
-                            ring, D, smask, lane, lt);
+            refine_chip_one(v, v.jobs + ji, m, n_u, (int64_t)v.r_half[q], T, tslot, shash, sinfo, cntA, ring, D, smask,
+                            lane, lt);
             __syncwarp();
         }
     }
@@ -2906,14 +2913,29 @@ __global__ void __launch_bounds__(SWEEP_WARPS * 32) k_sweep(BatchView v, SweepCa
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int32_t gw = blockIdx.x * SWEEP_WARPS + w, nwarps = gridDim.x * SWEEP_WARPS;
     for (int32_t q = gw; q < v.n; q += nwarps) {
-        const uint32_t c0 = v.coff[q], nc = v.coff[q + 1] - c0;
+        const uint32_t c0 = v.coff[q];
+        uint32_t nc = v.coff[q + 1] - c0;
         const SweepCand* L;
-        if (nc <= SWEEP_CAP) {
-            for (uint32_t i = lane; i < nc; i += 32) {
-                uint32_t ji = v.cidx[c0 + i];
-                sm[w][i] = load_cand(v.jobs[ji], ji);
-            }
-            __syncwarp();
+        // Without a tie-break band both sweeps look only at candidates whose
+        // score is above a threshold of at least theta_low (pass 2's is best *
+        // (1 - d) with best > theta), so the others, candidates never refined
+        // among them, are left out: a read from a repeat has hundreds of
+        // candidates and a few that pass (150,000 hifi reads: 0.53 ms, one lane
+        // walking every candidate, against 0.13).
+        const bool cut = v.P.tiebreak == 0.0;
+        uint32_t kept = 0;
+        for (uint32_t i0 = 0; i0 < nc && kept <= SWEEP_CAP; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            const uint32_t ji = i < nc ? v.cidx[c0 + i] : 0u;
+            const bool keep = i < nc && (!cut || v.jobs[ji].score > v.P.theta_low);
+            const unsigned bal = __ballot_sync(0xffffffffu, keep);
+            const uint32_t at = kept + __popc(bal & ((1u << lane) - 1u));
+            if (keep && at < SWEEP_CAP) sm[w][at] = load_cand(v.jobs[ji], ji);
+            kept += __popc(bal);
+        }
+        __syncwarp();
+        if (kept <= SWEEP_CAP) {
+            nc = kept;
             for (uint32_t i = lane; i < nc; i += 32) {
                 const SweepCand me = sm[w][i];
                 uint32_t rank = 0;
@@ -3236,7 +3258,8 @@ struct BatchPlan {
     uint64_t* chunk_off;   // n+1
     uint64_t* kcap_off;    // n+1
     uint64_t* pht_off;     // n+1
-    uint32_t n_cap_512 = 0, n_cap_1024 = 0, n_cap_4096 = 0;  // reads whose capacity exceeds 512 / 1024 / 4096
+    // reads whose capacity exceeds 256 / 512 / 1024 / 4096
+    uint32_t n_cap_256 = 0, n_cap_512 = 0, n_cap_1024 = 0, n_cap_4096 = 0;
     uint32_t P_g = 0;                          // power of two >= every capacity above 4096
     uint64_t max_cap = 0;                      // largest k-mer capacity of a read
     int64_t max_len = 0;                       // longest read
@@ -3282,7 +3305,7 @@ static void plan_batch(uint8_t* h_plan, const int64_t* h_offs, int32_t n, int32_
     bp.P_g = 0;
     bp.max_cap = 0;
     bp.max_len = 0;
-    bp.n_cap_512 = bp.n_cap_1024 = bp.n_cap_4096 = 0;
+    bp.n_cap_256 = bp.n_cap_512 = bp.n_cap_1024 = bp.n_cap_4096 = 0;
     bp.roff[0] = base0;
     bp.chunk_off[0] = 0;
     bp.kcap_off[0] = 0;
@@ -3297,6 +3320,7 @@ static void plan_batch(uint8_t* h_plan, const int64_t* h_offs, int32_t n, int32_
         bp.max_cap = std::max(bp.max_cap, cap);
         bp.max_len = std::max(bp.max_len, L);
         bp.pht_off[i + 1] = bp.pht_off[i] + std::max<uint64_t>(16, pow2_host(2 * cap));
+        if (cap > 256) bp.n_cap_256++;
         if (cap > 512) bp.n_cap_512++;
         if (cap > 1024) bp.n_cap_1024++;
         if (cap > 4096) {
@@ -3642,10 +3666,10 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     T.begin(STG_SEEDPREP);  // one span: bins, the side stream's large bins, the join
     k_seed_bins<<<grid_for((size_t)n, 256, 8), 256, 0, s>>>(v, S.seed_lists.p, S.bin_cnt.p);
     SHM_CUDA(cudaGetLastError());
-    // the few reads with large sketches go on the side stream, so that their
-    // long per-read latency overlaps the bulk of the reads on the main stream
+    // the reads with larger sketches go on the side stream, so that their
+    // longer per-read latency overlaps that of the others on the main stream
     // (a read of bin b has capacity >= m, which bounds each bin's size on the host)
-    const bool side = bp.n_cap_512 > 0;
+    const bool side = bp.n_cap_256 > 0;
     if (side) {
         SHM_CUDA(cudaEventRecord(c->fork, s));
         SHM_CUDA(cudaStreamWaitEvent(c->side_stream, c->fork, 0));
@@ -3689,16 +3713,16 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
         SHM_CUDA(cudaGetLastError());
         count_launch();
     }
-    if (side) SHM_CUDA(cudaEventRecord(c->join, s2));
-    {
-        k_seedprep_c<256, 8><<<grid_for((size_t)n * 32, 256, 4), 256, 8 * seedc_bytes(256) + sgb, s>>>(v, LB, NB);
-        SHM_CUDA(cudaGetLastError());
-        count_launch();
-        k_seedprep_c<512, 4><<<grid_for((size_t)n * 32, 128, 4), 128, 4 * seedc_bytes(512) + sgb, s>>>(v, LB + n,
-                                                                                                      NB + 1);
+    if (bp.n_cap_256) {  // 256 < m <= 512
+        k_seedprep_c<512, 4><<<grid_for((size_t)bp.n_cap_256 * 32, 128, 4), 128, 4 * seedc_bytes(512) + sgb, s2>>>(
+            v, LB + n, NB + 1);
         SHM_CUDA(cudaGetLastError());
         count_launch();
     }
+    if (side) SHM_CUDA(cudaEventRecord(c->join, s2));
+    k_seedprep_c<256, 8><<<grid_for((size_t)n * 32, 256, 4), 256, 8 * seedc_bytes(256) + sgb, s>>>(v, LB, NB);
+    SHM_CUDA(cudaGetLastError());
+    count_launch();
     if (side) SHM_CUDA(cudaStreamWaitEvent(s, c->join, 0));
     T.end();
 
@@ -3910,17 +3934,32 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
                                           (int)(REFINE_WARPS * REFINE_SLICE)));
             c->refine_smem_set = 1;
         }
-        for (int pass = 0; pass < (v.lead_on ? 2 : 1); pass++) {
-            if (p.metric != SHM_BUCKET_SH) {
+        // the reads refined on chip and the others are disjoint, and a pass 1
+        // candidate looks at its own read's lead only: two chains, side by side
+        // (each ends in the tail of its longest windows; with the leads taken
+        // by read, 2,049 hifi reads: 0.32 ms one after the other, 0.15 so)
+        const int passes = v.lead_on ? 2 : 1;
+        const bool chip = p.metric != SHM_BUCKET_SH;
+        cudaStream_t sf = chip ? c->side_stream : s;
+        if (chip) {
+            SHM_CUDA(cudaEventRecord(c->fork, s));
+            SHM_CUDA(cudaStreamWaitEvent(sf, c->fork, 0));
+            for (int pass = 0; pass < passes; pass++) {
                 k_refine_chip<<<grid_for((size_t)n * 32, RCHIP_WARPS * 32, 4), RCHIP_WARPS * 32,
                                 RCHIP_WARPS * RCHIP_SLICE, s>>>(v, pass);
                 SHM_CUDA(cudaGetLastError());
                 count_launch();
             }
+        }
+        for (int pass = 0; pass < passes; pass++) {
             k_refine<<<(unsigned)std::max<size_t>(1, warps / REFINE_WARPS), REFINE_WARPS * 32,
-                       REFINE_WARPS * REFINE_SLICE, s>>>(v, rsc, pass);
+                       REFINE_WARPS * REFINE_SLICE, sf>>>(v, rsc, pass);
             SHM_CUDA(cudaGetLastError());
-            if (pass == 0 && v.lead_on) count_launch();  // the last launch is counted by the stage timer
+            if (pass + 1 < passes) count_launch();  // the last launch is counted by the stage timer
+        }
+        if (chip) {
+            SHM_CUDA(cudaEventRecord(c->join, sf));
+            SHM_CUDA(cudaStreamWaitEvent(s, c->join, 0));
         }
     }
     T.end();
