@@ -67,30 +67,31 @@ namespace shm {
 // cost order, the dearest first (a warp's cost grows with the window region,
 // twice the bucket half-length): half-lengths above FAR_EDGE0, above
 // FAR_EDGE1, the rest.
-constexpr int FAR_BINS = 3;
+constexpr int FAR_BINS = 3;  // (the queue's layout: next_far)
 constexpr int32_t FAR_EDGE0 = 1024, FAR_EDGE1 = 512;
 __host__ __device__ __forceinline__ int far_bin_of(int32_t half) {
     return half > FAR_EDGE0 ? 0 : (half > FAR_EDGE1 ? 1 : 2);
 }
 
+constexpr int BT2_RUN_BITS = 40;  // (the reads of a batch, 2^22 at most, fit the other 24)
 struct BatchMax {
     unsigned int m_max, nu_max, half_max, n_overflow;
     unsigned long long kmers, distinct, proc_seeds, hits, buckets, ext_seeds, refine_kmers;
     unsigned int refine_next[2];  // next candidate chunk k_refine_chip takes, per refinement pass
-    unsigned int n_far;        // candidates not refined on chip (listed in cfar)
-    unsigned int far_bin[FAR_BINS];  // candidates of cfar by cost bin (their read's bucket half-length)
-    unsigned int far_cur[FAR_BINS];  // placing them, binned, into cfar_q
-    unsigned int far_next[2];        // next candidate of cfar_q a refinement warp takes, per pass
+    unsigned int far_bin[FAR_BINS];  // those candidates by cost bin (their read's bucket half-length)
+    unsigned int far_next[2];        // next candidate of the refinement queue a warp takes, per pass
+    unsigned int n_jobs, n_cands;    // bucket jobs, candidates
     unsigned long long refined;      // candidates refined (the reads' leads and those that can still score)
     unsigned long long bt2_next;     // spare bucket-table slots handed out (second tables)
-    unsigned int bt2_n;              // reads given a second table (listed in bt2_list)
+    // reads given a second table (listed in bt2_list) << BT2_RUN_BITS, plus the
+    // runs of their hit words: one atomic gives a read its place and first run
+    unsigned long long bt2_pack;
 };
 
 // Small device-to-host reads of a batch, landing in pinned memory.
 struct HostReads {
     uint64_t totals[2];  // hit words, bucket-table slots
     BatchMax hm;         // after seed preparation
-    uint32_t nj, nc;     // bucket jobs, candidates
     uint32_t nbk;        // distinct buckets of every read (synchronous sizing)
     BatchMax fin;        // after the sweep
 };
@@ -129,7 +130,7 @@ struct BatchView {
     uint64_t bt_pool;   // slots of the first tables; bt2_spare more follow for second tables
     uint64_t bt2_spare;
     uint32_t* bt2_list; // the reads given a second table
-    uint64_t* bt2_off;  // their first runs of hit work items for k_contrib2 (exclusive prefix, nl + 1)
+    uint64_t* bt2_off;  // their first runs of hit words for k_contrib2 (ascending)
     uint64_t bt_cap;    // most slots a read's bucket table gets (a power of two >= 16)
     uint64_t* r_eb;     // per read: the bound on its distinct buckets (0 until its seeds are prepared)
     uint64_t ext_total; // reference k-mers (bases under -F): a read's buckets are at most ext_total / half + 2 n_seg + 2
@@ -138,8 +139,9 @@ struct BatchView {
     uint32_t* n_jobs;
     uint32_t job_cap;
     uint32_t *ccnt, *coff, *ccur, *cidx;
-    uint32_t* cfar;    // the jobs of the candidates not refined on chip (mx->n_far of them)
-    uint32_t* cfar_q;  // the same jobs by cost bin, dearest bin first: the refinement queue
+    // the jobs of the candidates not refined on chip, by cost bin (next_far):
+    // bin 0 from cfar_q's start, bin 2 from its end down, bin 1 in cfar
+    uint32_t *cfar, *cfar_q;
     uint32_t* r_lead;  // per read: its lead candidate's job (refined first), UINT32_MAX for none
     int32_t lead_on;   // candidates refined in two passes (the leads, then those that can still score)
     uint32_t* ovf_list;
@@ -1085,7 +1087,12 @@ __device__ __forceinline__ uint32_t ub_u32(const uint32_t* a, uint32_t n, uint32
 // and seed come from two binary searches, the rest by stepping through the
 // seed's hit list (sorted by gidx) and on to the next seed or read. The
 // previous hit's bucket and the current segment's bounds are carried along.
+// A run is CONTRIB_RUN words, fewer while there is not a run for every thread
+// of the grid (a run's hits are one dependent chain after the other).
 constexpr int CONTRIB_RUN = 8;
+__device__ __forceinline__ uint32_t contrib_run(uint64_t total) {
+    return (uint32_t)min((uint64_t)CONTRIB_RUN, max((uint64_t)1, total / ((uint64_t)gridDim.x * blockDim.x)));
+}
 
 __device__ __forceinline__ int32_t seg_step(const DevIndex& I, uint32_t g, int32_t seg, uint32_t& s_lo,
                                             uint32_t& s_hi) {
@@ -1200,72 +1207,29 @@ __device__ __forceinline__ void contrib_span(const BatchView& v, uint64_t w, con
 
 __global__ void __launch_bounds__(256) k_contrib(BatchView v) {
     const uint64_t total = v.hw_off[v.n];
-    const uint64_t nrun = (total + CONTRIB_RUN - 1) / CONTRIB_RUN;
+    const uint32_t run = contrib_run(total);
+    const uint64_t nrun = (total + run - 1) / run;
     const int lane = threadIdx.x & 31;
     // a warp takes 32 consecutive runs: the read of its first by a 32-way
     // search, each lane's own by walking on from there (runs of one warp
     // rarely cross more than a read or two)
     for (uint64_t r0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); r0 < nrun;
          r0 += (uint64_t)gridDim.x * blockDim.x) {
-        int32_t q = warp_last_le(v.hw_off, v.n + 1, r0 * CONTRIB_RUN, lane);
+        int32_t q = warp_last_le(v.hw_off, v.n + 1, r0 * run, lane);
         const uint64_t rn = r0 + (uint64_t)lane;
         if (rn >= nrun) continue;
-        const uint64_t w = rn * CONTRIB_RUN;
+        const uint64_t w = rn * run;
         while (v.hw_off[q + 1] <= w) q++;
-        contrib_span(v, w, min(w + CONTRIB_RUN, total), q);
+        contrib_span(v, w, min(w + run, total), q);
     }
 }
 
-// The runs of CONTRIB_RUN hit work items of the reads given a second bucket
-// table (k_bt_second), as an exclusive prefix over the list (one CTA; the
-// list is short unless many reads filled their tables).
-__global__ void __launch_bounds__(1024) k_bt2_scan(BatchView v) {
-    __shared__ unsigned long long wsum[32];
-    __shared__ unsigned long long carry;
-    const uint32_t nl = v.mx->bt2_n;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (uint32_t c0 = 0; c0 < nl; c0 += 1024) {
-        const uint32_t i = c0 + threadIdx.x;
-        unsigned long long x = 0;
-        if (i < nl) {
-            const int32_t q = (int32_t)v.bt2_list[i];
-            x = (v.hw_off[q + 1] - v.hw_off[q] + CONTRIB_RUN - 1) / CONTRIB_RUN;
-        }
-        unsigned long long inc = x;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long y = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += y;
-        }
-        if (lane == 31) wsum[wid] = inc;
-        __syncthreads();
-        if (wid == 0) {
-            unsigned long long t = wsum[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long y = __shfl_up_sync(0xffffffffu, t, o);
-                if (lane >= o) t += y;
-            }
-            wsum[lane] = t;  // inclusive over warps
-        }
-        __syncthreads();
-        const unsigned long long before = carry + (wid ? wsum[wid - 1] : 0ULL) + inc - x;
-        if (i < nl) v.bt2_off[i] = before;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += wsum[31];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) v.bt2_off[nl] = carry;
-}
-
-// Those runs over the whole grid: each finds its read in the list by the
-// prefix and contributes into the read's second table.
+// The hits of the reads given a second bucket table (k_bt_second), again: the
+// runs of all of them over the whole grid, each run's read by its first run.
 __global__ void __launch_bounds__(256) k_contrib2(BatchView v) {
-    const uint32_t nl = v.mx->bt2_n;
-    if (nl == 0) return;
-    const uint64_t nrun = v.bt2_off[nl];
+    const unsigned long long pack = v.mx->bt2_pack;
+    const uint32_t nl = (uint32_t)(pack >> BT2_RUN_BITS);
+    const uint64_t nrun = pack & (((uint64_t)1 << BT2_RUN_BITS) - 1);
     for (uint64_t rn = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; rn < nrun;
          rn += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t lo = 0, hi = nl;  // the last list entry whose first run is <= rn
@@ -1336,7 +1300,10 @@ __global__ void __launch_bounds__(256) k_bt_second(BatchView v) {
                 v.bt_tab[r] = make_ulonglong2(base, slots - 1);
                 v.r_seeded[r] = 0;
                 v.r_flags[r] = 0;
-                v.bt2_list[atomicAdd(&v.mx->bt2_n, 1u)] = (uint32_t)r;
+                const unsigned long long runs = (v.hw_off[r + 1] - v.hw_off[r] + CONTRIB_RUN - 1) / CONTRIB_RUN;
+                const unsigned long long pk = atomicAdd(&v.mx->bt2_pack, (1ULL << BT2_RUN_BITS) + runs);
+                v.bt2_list[pk >> BT2_RUN_BITS] = (uint32_t)r;
+                v.bt2_off[pk >> BT2_RUN_BITS] = pk & ((1ULL << BT2_RUN_BITS) - 1);
             }
         }
     }
@@ -1459,8 +1426,8 @@ __global__ void __launch_bounds__(256) k_extend(BatchView v) {
 }
 
 // ------------------------------------------------------------------ K6 candidates per read
-// Also lists the candidates k_refine takes (those not refined on chip), one
-// counter update per warp.
+// Also lists the candidates k_refine takes (those not refined on chip) by cost
+// bin, one counter update per warp and bin (within a bin, in any order).
 __global__ void k_cidx(BatchView v) {
     const uint32_t njobs = min(*v.n_jobs, v.job_cap);
     const int lane = threadIdx.x & 31;
@@ -1472,56 +1439,31 @@ __global__ void k_cidx(BatchView v) {
             v.cidx[v.coff[q] + atomicAdd(v.ccur + q, 1u)] = ji;
             far = !refine_on_chip(v.P, (uint32_t)v.r_m[q], v.r_half[q]);
         }
-        const unsigned fm = __ballot_sync(0xffffffffu, far);
-        if (fm) {
-            const int leader = __ffs(fm) - 1;
-            uint32_t at = 0;
-            if (lane == leader) at = atomicAdd(&v.mx->n_far, (uint32_t)__popc(fm));
-            at = __shfl_sync(0xffffffffu, at, leader);
-            if (far) v.cfar[at + __popc(fm & ((1u << lane) - 1u))] = ji;
-            const int bin = far ? far_bin_of(v.r_half[v.jobs[ji].read]) : -1;
+        const int bin = far ? far_bin_of(v.r_half[v.jobs[ji].read]) : -1;
 #pragma unroll
-            for (int b2 = 0; b2 < FAR_BINS; b2++) {
-                const unsigned bm = __ballot_sync(0xffffffffu, bin == b2);
-                if (bm && lane == __ffs(bm) - 1) atomicAdd(&v.mx->far_bin[b2], (uint32_t)__popc(bm));
-            }
-        }
-    }
-}
-
-// The refinement queue: cfar's candidates placed by cost bin, the dearest
-// bin first, so the longest refinements start first and the short ones fill
-// the end (within a bin, in any order).
-__global__ void k_far_bins(BatchView v) {
-    const uint32_t nfar = v.mx->n_far;
-    const int lane = threadIdx.x & 31;
-    uint32_t base[FAR_BINS];
-    base[0] = 0;
-    for (int b = 1; b < FAR_BINS; b++) base[b] = base[b - 1] + v.mx->far_bin[b - 1];
-    for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < nfar; i0 += gridDim.x * blockDim.x) {
-        const uint32_t i = i0 + (uint32_t)lane;
-        const uint32_t ji = i < nfar ? v.cfar[i] : 0u;
-        const int bin = i < nfar ? far_bin_of(v.r_half[v.jobs[ji].read]) : -1;
-#pragma unroll
-        for (int b = 0; b < FAR_BINS; b++) {
-            const unsigned bm = __ballot_sync(0xffffffffu, bin == b);
+        for (int b2 = 0; b2 < FAR_BINS; b2++) {
+            const unsigned bm = __ballot_sync(0xffffffffu, bin == b2);
             if (!bm) continue;
             const int leader = __ffs(bm) - 1;
             uint32_t at = 0;
-            if (lane == leader) at = atomicAdd(&v.mx->far_cur[b], (uint32_t)__popc(bm));
-            at = __shfl_sync(0xffffffffu, at, leader);
-            if (bin == b) v.cfar_q[base[b] + at + __popc(bm & ((1u << lane) - 1u))] = ji;
+            if (lane == leader) at = atomicAdd(&v.mx->far_bin[b2], (uint32_t)__popc(bm));
+            at = __shfl_sync(0xffffffffu, at, leader) + __popc(bm & ((1u << lane) - 1u));
+            if (bin == b2) *(b2 == 1 ? v.cfar + at : v.cfar_q + (b2 == 0 ? at : v.job_cap - 1 - at)) = ji;
         }
     }
 }
 
-// The next candidate of the refinement queue for this warp (UINT32_MAX when
-// the queue is empty).
+// The next candidate of the refinement queue for this warp, the dearest bin
+// first, so the longest refinements start first and the short ones fill the
+// end (UINT32_MAX when the queue is empty).
 __device__ __forceinline__ uint32_t next_far(const BatchView& v, int lane, int pass = 0) {
     uint32_t ci = 0;
     if (lane == 0) ci = atomicAdd(&v.mx->far_next[pass], 1u);
     ci = __shfl_sync(0xffffffffu, ci, 0);
-    return ci < v.mx->n_far ? v.cfar_q[ci] : UINT32_MAX;
+    const uint32_t n0 = v.mx->far_bin[0], n1 = v.mx->far_bin[1], n2 = v.mx->far_bin[2];
+    if (ci < n0) return v.cfar_q[ci];
+    if (ci - n0 < n1) return v.cfar[ci - n0];
+    return ci - n0 - n1 < n2 ? v.cfar_q[v.job_cap - 1 - (ci - n0 - n1)] : UINT32_MAX;
 }
 
 // ------------------------------------------------------------------ which candidates are refined
@@ -2520,8 +2462,7 @@ __device__ void refine_rarity_one(const BatchView& v, BucketJob* J, int32_t q, c
 __global__ void __launch_bounds__(REFINE_WARPS * 32, 4) k_refine_rarity(BatchView v, RefScratch rsc) {
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t nfar = v.mx->n_far;
+    const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int32_t* const base = rsc.base + (size_t)wid * rsc.per_warp;
     RarScratch R;
     R.cntA = base;
@@ -2531,8 +2472,6 @@ __global__ void __launch_bounds__(REFINE_WARPS * 32, 4) k_refine_rarity(BatchVie
     R.nxt = R.ring + rsc.ring_n;
     R.flag = R.nxt + rsc.wmax + 1;
     R.wt = (double*)(base + rsc.wt_at);
-    (void)nfar;
-    (void)nwarps;
     for (uint32_t jq; (jq = next_far(v, lane)) != UINT32_MAX;) {
         BucketJob* J = v.jobs + jq;
         refine_rarity_one(v, J, J->read, R, lane, lt);
@@ -2912,6 +2851,7 @@ __global__ void __launch_bounds__(SWEEP_WARPS * 32) k_sweep(BatchView v, SweepCa
     __shared__ SweepCand srt[SWEEP_WARPS][SWEEP_CAP];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int32_t gw = blockIdx.x * SWEEP_WARPS + w, nwarps = gridDim.x * SWEEP_WARPS;
+    if (gw == 0 && lane == 0) v.mx->n_cands = v.coff[v.n];
     for (int32_t q = gw; q < v.n; q += nwarps) {
         const uint32_t c0 = v.coff[q];
         uint32_t nc = v.coff[q + 1] - c0;
@@ -3137,30 +3077,27 @@ struct MapScratch {
     DevBuf<uint8_t> seqb[2];  // host-form batches: one mapped, the next arriving
     DevBuf<uint8_t> plan;  // BatchPlan's arrays on the device
     DevBuf<int32_t> seed_lists;  // N_SEED_BINS lists of n reads
-    DevBuf<uint32_t> bin_cnt;
     DevBuf<uint8_t> retry_seq;  // reads mapped again with exact bounds
     DevBuf<shm_map_record> retry_out;
     DevBuf<int64_t> retry_list;
     DevBuf<int32_t> retry_idx;
-    DevBuf<uint64_t> km_h, pht_key, hw, hw_off, bt_size, bt_off;
+    DevBuf<uint8_t> zero;  // the arrays a batch starts from zero (ZeroArena)
+    DevBuf<uint64_t> km_h, pht_key, hw_off, bt_off, scan_sums;
     DevBuf<SeedRec> sd;
     DevBuf<uint32_t> pk_codes[2], pk_mask[2];  // host-buffer batches, packed (host/pack.hpp)
     DevBuf<uint32_t> pk_list[2];               // their nonzero mask words as uploaded (index, word)
     DevBuf<uint32_t> dpk_codes, dpk_mask;      // device-resident batches, packed on the device
     DevBuf<uint64_t> sd_h;
-    DevBuf<uint32_t> kcnt, km_rs, sd_hpre, pht_val, r_seeded, n_jobs, ccnt, coff, ccur,
-        cidx, cfar, cfar_q, sort_scr, ovf_list, r_flags;
+    DevBuf<uint32_t> km_rs, sd_hpre, pht_val, coff, cidx, cfar, cfar_q, sort_scr;
     DevBuf<uint32_t> lcs_pos, lcs_cnt;  // bucket_LCS only
     DevBuf<uint32_t> r_lead;
-    DevBuf<int32_t> r_i32, ref_scr;
+    DevBuf<int32_t> ref_scr;
     DevBuf<int64_t> r_smatch;
-    DevBuf<uint64_t> r_eb;
     DevBuf<BSlot> bt;
     DevBuf<uint32_t> bt_list, bt2_list;
     DevBuf<ulonglong2> bt_tab;
     DevBuf<uint64_t> bt2_off;
     DevBuf<BucketJob> jobs;
-    DevBuf<BatchMax> mx;
     DevBuf<SweepCand> sweep_scr;
     DevBuf<uint8_t> seed_gscr;
     DevBuf<shm_map_record> out;
@@ -3288,15 +3225,46 @@ static uint8_t* pinned_stage(MapCtx* c, size_t bytes) {
     return c->h_pinned;
 }
 
+// The arrays of a batch that start from zero, in one allocation.
+struct ZeroArena {
+    uint64_t *hw, *bt_size, *r_eb;                         // n each
+    BatchMax* mx;
+    uint32_t *kcnt, *r_seeded, *r_flags, *ccnt, *ccur;     // n each
+    int32_t* r_i32;                                        // 8 n
+    uint32_t* bin_cnt;                                     // N_SEED_BINS
+    static size_t words(int32_t n) { return 19 * (size_t)n + sizeof(BatchMax) / 4 + N_SEED_BINS; }
+    void carve(uint8_t* base, int32_t n) {
+        hw = (uint64_t*)base;
+        bt_size = hw + n;
+        r_eb = bt_size + n;
+        mx = (BatchMax*)(r_eb + n);
+        kcnt = (uint32_t*)(mx + 1);
+        r_seeded = kcnt + n;
+        r_flags = r_seeded + n;
+        ccnt = r_flags + n;
+        ccur = ccnt + n;
+        r_i32 = (int32_t*)(ccur + n);
+        bin_cnt = (uint32_t*)(r_i32 + 8 * (size_t)n);
+    }
+};
+static_assert(sizeof(BatchMax) % 8 == 0, "the arena's arrays follow it");
+
+// The start of a batch: words [0, n) of src (device-accessible: a mapped
+// pinned block) to dst, and words [0, nz) of zero cleared. (A batch was 41
+// stream operations, a dozen of them clearings: a call of one read spent a
+// third of its 0.30 ms between them. 22 operations and shorter runs of
+// contributions make it 0.23 ms.)
+__global__ void k_begin(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, size_t n,
+                        uint32_t* __restrict__ zero, size_t nz) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        dst[i] = src[i];
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nz; i += (size_t)gridDim.x * blockDim.x)
+        zero[i] = 0;
+}
+
 // Written into pinned memory at h_plan (BatchPlan::layout(n) bytes). caps =
 // null: capacities from the estimate; else caps[i] k-mers for read i (the
 // counts a previous pass found).
-// words [0, n) of src (device-accessible, e.g. a mapped pinned block) to dst.
-__global__ void k_copy_words(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        dst[i] = src[i];
-}
-
 // roff starts at base0: the batch's first base in the buffer its sketch reads
 // (only differences of roff are read elsewhere).
 static void plan_batch(uint8_t* h_plan, const int64_t* h_offs, int32_t n, int32_t k, double h_frac,
@@ -3338,10 +3306,11 @@ struct Overflow {
 };
 
 // Where a batch's results land on the host (pinned): the small reads, then
-// its overflow list (up to n pairs read, m).
+// its overflow list (up to n entries of four words).
 struct BatchSlot {
     HostReads* R;
-    uint32_t* ovf;
+    uint32_t* ovf;      // written by the sweep through its device mapping, ovf_dev (overflows are few)
+    uint32_t* ovf_dev;
     int32_t i0, n;
     int64_t bases;
     uint32_t job_cap;  // set by run_batch: more jobs than this and the batch is mapped again
@@ -3411,6 +3380,7 @@ static std::vector<BatchSlot> batch_slots(MapCtx* c, const std::vector<std::pair
         sl.R = (HostReads*)at;
         at += (sizeof(HostReads) + 63) / 64 * 64;
         sl.ovf = (uint32_t*)at;
+        SHM_CUDA(cudaHostGetDevicePointer((void**)&sl.ovf_dev, at, 0));
         at += (16 * (size_t)(j - i) + 63) / 64 * 64;
         sl.i0 = i;
         sl.n = j - i;
@@ -3432,12 +3402,12 @@ static void collect_batch(MapCtx* c, const BatchSlot& sl, std::vector<Overflow>&
     c->work[W_PROC_SEEDS] += (int64_t)fin.proc_seeds;
     c->work[W_HITS] += (int64_t)fin.hits;
     c->work[W_BUCKETS] += (int64_t)fin.buckets;
-    c->work[W_JOBS] += R.nj;
+    c->work[W_JOBS] += fin.n_jobs;
     c->work[W_EXT_SEEDS] += (int64_t)fin.ext_seeds;
-    c->work[W_CANDS] += R.nc;
+    c->work[W_CANDS] += fin.n_cands;
     c->work[W_REFINE_KMERS] += (int64_t)fin.refine_kmers;
     c->work[W_REFINED] += (int64_t)fin.refined;
-    c->work[W_BT2_READS] += (int64_t)fin.bt2_n;
+    c->work[W_BT2_READS] += (int64_t)(fin.bt2_pack >> BT2_RUN_BITS);
     const size_t at = ovf.size();
     for (uint32_t i = 0; i < fin.n_overflow && i < (uint32_t)sl.n; i++)
         ovf.push_back(Overflow{sl.i0 + (int32_t)sl.ovf[4 * i], sl.ovf[4 * i + 1],
@@ -3478,21 +3448,26 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     // engine, or (plan_mapped) by a kernel reading the block through its
     // device mapping: then it does not queue behind the other host-to-device
     // copies of the copy engine (the packing threads' pieces)
+    // the same launch clears the arrays that start from zero
     S.plan.reserve(bp.bytes + 64);
+    S.zero.reserve(4 * ZeroArena::words(n));
+    ZeroArena Z;
+    Z.carve(S.zero.p, n);
     void* d_src = nullptr;
+    size_t words = (bp.bytes + 3) / 4;  // the block is padded to 64 bytes
     if (tuning().plan_mapped && cudaHostGetDevicePointer(&d_src, h_plan, 0) == cudaSuccess) {
-        const size_t words = (bp.bytes + 3) / 4;  // the block is padded to 64 bytes
-        k_copy_words<<<grid_for(words, 256, 4), 256, 0, s>>>((uint32_t*)S.plan.p, (const uint32_t*)d_src, words);
-        SHM_CUDA(cudaGetLastError());
-        count_launch();
         c->work[W_H2D_BYTES] += (int64_t)bp.bytes;
     } else {
         cudaGetLastError();
         copy_async(c, S.plan.p, h_plan, bp.bytes, cudaMemcpyHostToDevice, s);
+        words = 0;
     }
+    k_begin<<<grid_for(std::max(words, ZeroArena::words(n)), 256, 4), 256, 0, s>>>(
+        (uint32_t*)S.plan.p, (const uint32_t*)d_src, words, (uint32_t*)S.zero.p, ZeroArena::words(n));
+    SHM_CUDA(cudaGetLastError());
+    count_launch();
     BatchPlan dp;
     dp.carve(S.plan.p, n);
-    S.kcnt.reserve((size_t)n);
     S.km_h.reserve(kcap + 1);
     S.km_rs.reserve(kcap + 1);
     S.sd.reserve(kcap + 1);
@@ -3500,32 +3475,10 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     S.sd_hpre.reserve(kcap + 1);
     S.pht_key.reserve(phtn);
     S.pht_val.reserve(phtn);
-    S.r_i32.reserve((size_t)n * 8);
     S.r_smatch.reserve((size_t)n);
-    S.r_seeded.reserve((size_t)n);
-    S.r_flags.reserve((size_t)n);
-    S.hw.reserve((size_t)n);
     S.hw_off.reserve((size_t)n + 1);
-    S.bt_size.reserve((size_t)n);
     S.bt_off.reserve((size_t)n + 1);
-    S.ccnt.reserve((size_t)n);
     S.coff.reserve((size_t)n + 1);
-    S.ccur.reserve((size_t)n);
-    S.ovf_list.reserve(4 * (size_t)n);
-    S.r_eb.reserve((size_t)n);
-    S.n_jobs.reserve(1);
-    S.mx.reserve(1);
-    SHM_CUDA(cudaMemsetAsync(S.kcnt.p, 0, sizeof(uint32_t) * (size_t)n, s));
-    SHM_CUDA(cudaMemsetAsync(S.r_seeded.p, 0, sizeof(uint32_t) * (size_t)n, s));
-    SHM_CUDA(cudaMemsetAsync(S.r_flags.p, 0, sizeof(uint32_t) * (size_t)n, s));
-    SHM_CUDA(cudaMemsetAsync(S.r_eb.p, 0, sizeof(uint64_t) * (size_t)n, s));
-    SHM_CUDA(cudaMemsetAsync(S.ccnt.p, 0, sizeof(uint32_t) * (size_t)n, s));
-    SHM_CUDA(cudaMemsetAsync(S.ccur.p, 0, sizeof(uint32_t) * (size_t)n, s));
-    SHM_CUDA(cudaMemsetAsync(S.n_jobs.p, 0, sizeof(uint32_t), s));
-    SHM_CUDA(cudaMemsetAsync(S.mx.p, 0, sizeof(BatchMax), s));
-    SHM_CUDA(cudaMemsetAsync(S.r_i32.p, 0, sizeof(int32_t) * (size_t)n * 8, s));
-    SHM_CUDA(cudaMemsetAsync(S.hw.p, 0, sizeof(uint64_t) * (size_t)n, s));
-    SHM_CUDA(cudaMemsetAsync(S.bt_size.p, 0, sizeof(uint64_t) * (size_t)n, s));
     H.mark("upload");
 
     BatchView v{};
@@ -3583,7 +3536,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     v.seq = d_seq;
     v.roff = dp.roff;
     v.kcap_off = dp.kcap_off;
-    v.kcnt = S.kcnt.p;
+    v.kcnt = Z.kcnt;
     v.km_h = S.km_h.p;
     v.km_rs = S.km_rs.p;
     v.sd = S.sd.p;
@@ -3592,7 +3545,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     v.pht_off = dp.pht_off;
     v.pht_key = S.pht_key.p;
     v.pht_val = S.pht_val.p;
-    int32_t* ri = S.r_i32.p;
+    int32_t* ri = Z.r_i32;
     v.r_status = ri;
     v.r_m = ri + n;
     v.r_nu = ri + 2 * (size_t)n;
@@ -3602,23 +3555,23 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     v.r_half = ri + 6 * (size_t)n;
     v.r_maxseed = ri + 7 * (size_t)n;
     v.r_smatch = S.r_smatch.p;
-    v.r_seeded = S.r_seeded.p;
-    v.r_flags = S.r_flags.p;
+    v.r_seeded = Z.r_seeded;
+    v.r_flags = Z.r_flags;
     // synchronous sizing: tables of at most bt_lim slots a read (0: the full bound);
     // queued sizing: at most fast_bt_read_cap() a read, from a pool of fast_bt_slots() a read
     v.bt_cap = exact ? (bt_lim ? bt_lim : ((uint64_t)1 << 62)) : fast_bt_read_cap();
-    v.r_eb = S.r_eb.p;
+    v.r_eb = Z.r_eb;
     v.ext_total = p.abs_pos ? (uint64_t)ix->stats.total_nucls : (uint64_t)ix->dev.n_kmers;
-    v.hw = S.hw.p;
+    v.hw = Z.hw;
     v.hw_off = S.hw_off.p;
-    v.bt_size = S.bt_size.p;
+    v.bt_size = Z.bt_size;
     v.bt_off = S.bt_off.p;
-    v.n_jobs = S.n_jobs.p;
-    v.ccnt = S.ccnt.p;
+    v.n_jobs = &Z.mx->n_jobs;
+    v.ccnt = Z.ccnt;
     v.coff = S.coff.p;
-    v.ccur = S.ccur.p;
-    v.ovf_list = S.ovf_list.p;
-    v.mx = S.mx.p;
+    v.ccur = Z.ccur;
+    v.ovf_list = sl.ovf_dev;
+    v.mx = Z.mx;
     v.out = d_out;
 
     // K1
@@ -3634,7 +3587,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     a.thr = ix->dev.thr;
     a.r_offset = 0;
     a.kmer_off = dp.kcap_off;
-    a.kmer_cnt = S.kcnt.p;
+    a.kmer_cnt = Z.kcnt;
     a.out_h = S.km_h.p;
     a.out_rs = S.km_rs.p;
     const int64_t batch_bytes = h_offs[n] - h_offs[0];
@@ -3658,13 +3611,11 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
 
     // K2: bins by the actual sketch sizes, then one launch per bin (each
     // reads its own count on the device; empty bins return at once)
-    S.bin_cnt.reserve(N_SEED_BINS);
     S.seed_lists.reserve((size_t)N_SEED_BINS * (size_t)n);
-    SHM_CUDA(cudaMemsetAsync(S.bin_cnt.p, 0, sizeof(uint32_t) * N_SEED_BINS, s));
     const int32_t* LB = S.seed_lists.p;
-    const uint32_t* NB = S.bin_cnt.p;
+    const uint32_t* NB = Z.bin_cnt;
     T.begin(STG_SEEDPREP);  // one span: bins, the side stream's large bins, the join
-    k_seed_bins<<<grid_for((size_t)n, 256, 8), 256, 0, s>>>(v, S.seed_lists.p, S.bin_cnt.p);
+    k_seed_bins<<<grid_for((size_t)n, 256, 8), 256, 0, s>>>(v, S.seed_lists.p, Z.bin_cnt);
     SHM_CUDA(cudaGetLastError());
     // the reads with larger sketches go on the side stream, so that their
     // longer per-read latency overlaps that of the others on the main stream
@@ -3726,8 +3677,8 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     if (side) SHM_CUDA(cudaStreamWaitEvent(s, c->join, 0));
     T.end();
 
-    exclusive_scan_u64(S.hw.p, S.hw_off.p, (size_t)n, s);
-    exclusive_scan_u64(S.bt_size.p, S.bt_off.p, (size_t)n, s);
+    S.scan_sums.reserve(scan_sums_words((size_t)n));
+    exclusive_scan2<uint64_t>(Z.hw, S.hw_off.p, Z.bt_size, S.bt_off.p, (size_t)n, S.scan_sums.p, s);
     HostReads& R = *sl.R;
     const bool debug = std::getenv("SHMAP_DEBUG") != nullptr;
     // Sizes after seeding. Exact mode: wait for the bucket tables' total and
@@ -3738,7 +3689,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     if (exact || debug) {
         copy_async(c, &R.totals[0], S.hw_off.p + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
         copy_async(c, &R.totals[1], S.bt_off.p + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
-        copy_async(c, &R.hm, S.mx.p, sizeof(BatchMax), cudaMemcpyDeviceToHost, s);
+        copy_async(c, &R.hm, Z.mx, sizeof(BatchMax), cudaMemcpyDeviceToHost, s);
         H.mark("enq1");
         SHM_CUDA(cudaStreamSynchronize(s));
         H.mark("sync1");
@@ -3751,10 +3702,10 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
                 std::vector<int32_t> ri((size_t)n * 8);
                 std::vector<uint32_t> kc((size_t)n);
                 std::vector<uint64_t> hw((size_t)n), bs((size_t)n);
-                SHM_CUDA(cudaMemcpy(ri.data(), S.r_i32.p, sizeof(int32_t) * ri.size(), cudaMemcpyDeviceToHost));
-                SHM_CUDA(cudaMemcpy(kc.data(), S.kcnt.p, sizeof(uint32_t) * kc.size(), cudaMemcpyDeviceToHost));
-                SHM_CUDA(cudaMemcpy(hw.data(), S.hw.p, sizeof(uint64_t) * hw.size(), cudaMemcpyDeviceToHost));
-                SHM_CUDA(cudaMemcpy(bs.data(), S.bt_size.p, sizeof(uint64_t) * bs.size(), cudaMemcpyDeviceToHost));
+                SHM_CUDA(cudaMemcpy(ri.data(), Z.r_i32, sizeof(int32_t) * ri.size(), cudaMemcpyDeviceToHost));
+                SHM_CUDA(cudaMemcpy(kc.data(), Z.kcnt, sizeof(uint32_t) * kc.size(), cudaMemcpyDeviceToHost));
+                SHM_CUDA(cudaMemcpy(hw.data(), Z.hw, sizeof(uint64_t) * hw.size(), cudaMemcpyDeviceToHost));
+                SHM_CUDA(cudaMemcpy(bs.data(), Z.bt_size, sizeof(uint64_t) * bs.size(), cudaMemcpyDeviceToHost));
                 for (int32_t q = 0; q < n; q++)
                     std::fprintf(stderr,
                                  "[shmap]  read %d kcnt=%u status=%d m=%d nu=%d nproc=%d S=%d S0=%d half=%d maxseed=%d "
@@ -3788,7 +3739,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     S.bt_list.reserve(bt_slots_alloc + spare + 1);
     S.bt_tab.reserve((size_t)n);
     S.bt2_list.reserve((size_t)n);
-    S.bt2_off.reserve((size_t)n + 1);
+    S.bt2_off.reserve((size_t)n);
     H.mark("bt_res");
     v.bt = S.bt.p;
     v.bt_list = S.bt_list.p;
@@ -3798,7 +3749,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     v.bt_pool = bt_slots_alloc;
     v.bt2_spare = spare;
     T.begin(STG_AUX);
-    k_bt_init<<<wide, 256, 0, s>>>(S.bt.p, S.bt_off.p, n, bt_slots_alloc, S.r_flags.p, S.bt_tab.p);
+    k_bt_init<<<wide, 256, 0, s>>>(S.bt.p, S.bt_off.p, n, bt_slots_alloc, Z.r_flags, S.bt_tab.p);
     SHM_CUDA(cudaGetLastError());
     T.end();
     T.begin(STG_CONTRIB);
@@ -3811,10 +3762,6 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
         SHM_CUDA(cudaGetLastError());
         T.end();
         T.begin(STG_CONTRIB);
-        k_bt2_scan<<<1, 1024, 0, s>>>(v);
-        SHM_CUDA(cudaGetLastError());
-        T.end();
-        T.begin(STG_CONTRIB);
         k_contrib2<<<wide, 256, 0, s>>>(v);
         SHM_CUDA(cudaGetLastError());
         T.end();
@@ -3822,7 +3769,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     H.mark("contrib");
     if (exact) {  // the distinct buckets of every read, counted: they bound the jobs
         S.sort_scr.reserve((size_t)n + 1);
-        exclusive_scan_u32(S.r_seeded.p, S.sort_scr.p, (size_t)n, s);
+        exclusive_scan_u32(Z.r_seeded, S.sort_scr.p, (size_t)n, s);
         copy_async(c, &R.nbk, S.sort_scr.p + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
         SHM_CUDA(cudaStreamSynchronize(s));
         job_cap = R.nbk + 1;
@@ -3843,7 +3790,8 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
         T.end();
     }
     H.mark("extend");
-    exclusive_scan_u32(S.ccnt.p, S.coff.p, (size_t)n, s);
+    S.scan_sums.reserve(scan_sums_words((size_t)n));
+    exclusive_scan2<uint32_t>(Z.ccnt, S.coff.p, nullptr, nullptr, (size_t)n, (uint32_t*)S.scan_sums.p, s);
     H.mark("scan");
     S.cidx.reserve((size_t)job_cap + 1);
     S.cfar.reserve((size_t)job_cap + 1);
@@ -3865,9 +3813,6 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     T.begin(STG_AUX);
     k_cidx<<<wide, 256, 0, s>>>(v);
     SHM_CUDA(cudaGetLastError());
-    k_far_bins<<<wide, 256, 0, s>>>(v);
-    SHM_CUDA(cudaGetLastError());
-    count_launch();
     if (v.lead_on) {
         k_lead<<<grid_for((size_t)n * 32, 256, 8), 256, 0, s>>>(v);
         SHM_CUDA(cudaGetLastError());
@@ -3968,18 +3913,15 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     SHM_CUDA(cudaGetLastError());
     T.end();
 
-    copy_async(c, &R.fin, S.mx.p, sizeof(BatchMax), cudaMemcpyDeviceToHost, s);
-    copy_async(c, &R.nj, S.n_jobs.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    copy_async(c, &R.nc, S.coff.p + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    copy_async(c, sl.ovf, S.ovf_list.p, 4 * sizeof(uint32_t) * (size_t)n, cudaMemcpyDeviceToHost, s);
+    copy_async(c, &R.fin, Z.mx, sizeof(BatchMax), cudaMemcpyDeviceToHost, s);
     H.mark("enq_rest");
     if (debug) {
         SHM_CUDA(cudaStreamSynchronize(s));
-        std::fprintf(stderr, "[shmap] jobs=%u (cap %u) candidates=%u overflow=%u\n", R.nj, job_cap, R.nc,
+        std::fprintf(stderr, "[shmap] jobs=%u (cap %u) candidates=%u overflow=%u\n", R.fin.n_jobs, job_cap, R.fin.n_cands,
                      R.fin.n_overflow);
-        if (R.nj && R.nj <= 16) {
-            std::vector<BucketJob> jb(R.nj);
-            SHM_CUDA(cudaMemcpy(jb.data(), S.jobs.p, sizeof(BucketJob) * R.nj, cudaMemcpyDeviceToHost));
+        if (R.fin.n_jobs && R.fin.n_jobs <= 16) {
+            std::vector<BucketJob> jb(R.fin.n_jobs);
+            SHM_CUDA(cudaMemcpy(jb.data(), S.jobs.p, sizeof(BucketJob) * R.fin.n_jobs, cudaMemcpyDeviceToHost));
             for (auto& j : jb)
                 std::fprintf(stderr,
                              "[shmap]  job read=%d seg=%d bb=%d m0=%d matches=%d codir=%d r=[%d,%d] sh=%.6f cand=%d "
@@ -4073,7 +4015,7 @@ static void retry_group(MapCtx* c, const IndexStorage* ix, const shm_params& p, 
     run_batch(c, ix, p, S.retry_seq.p, o.data(), n, S.retry_out.p, caps.data(), exact, pin + plan_at, T, sl[0],
               nullptr, nullptr, bt_lim);
     SHM_CUDA(cudaStreamSynchronize(s));
-    if (!exact && sl[0].R->nj > sl[0].job_cap) {  // too many bucket jobs for the queued sizes: counted this time
+    if (!exact && sl[0].R->fin.n_jobs > sl[0].job_cap) {  // too many bucket jobs for the queued sizes: counted this time
         run_batch(c, ix, p, S.retry_seq.p, o.data(), n, S.retry_out.p, caps.data(), true, pin + plan_at, T, sl[0],
                   nullptr, nullptr, fast_bt_read_cap());
         SHM_CUDA(cudaStreamSynchronize(s));
@@ -4216,7 +4158,7 @@ void map_device(MapCtx* c, const IndexStorage* ix, const shm_params& p, const ui
     SHM_CUDA(cudaStreamSynchronize(c->stream));
     // a batch with more bucket jobs than its capacity is mapped again, its jobs counted first
     for (size_t b = 0; b < batches.size(); b++) {
-        if (slots[b].R->nj <= slots[b].job_cap) continue;
+        if (slots[b].R->fin.n_jobs <= slots[b].job_cap) continue;
         const auto [i, j] = batches[b];
         run_batch(c, ix, p, d_seq + (h_offs[i] - h_offs[0]), h_offs + i, j - i, d_out + i, nullptr, true, plans[b], T,
                   slots[b], nullptr, nullptr, fast_bt_read_cap());
@@ -4599,7 +4541,7 @@ static bool map_host_stream(MapCtx* c, const IndexStorage* ix, const shm_params&
     // a batch with more bucket jobs than its capacity is mapped again, its jobs counted first
     bool changed = false;
     for (size_t b = 0; b < batches.size(); b++) {
-        if (slots[b].R->nj <= slots[b].job_cap) continue;
+        if (slots[b].R->fin.n_jobs <= slots[b].job_cap) continue;
         changed = true;
         const auto [i, j] = batches[b];
         const int64_t nb = offs[j] - offs[i];
@@ -4834,7 +4776,7 @@ bool map_host(MapCtx* c, const IndexStorage* ix, const shm_params& p, const uint
     // a batch with more bucket jobs than its capacity is mapped again, its jobs counted first
     bool changed = false;
     for (size_t b = 0; b < batches.size(); b++) {
-        if (slots[b].R->nj <= slots[b].job_cap) continue;
+        if (slots[b].R->fin.n_jobs <= slots[b].job_cap) continue;
         changed = true;
         const auto [i, j] = batches[b];
         const int64_t nb = offs[j] - offs[i];

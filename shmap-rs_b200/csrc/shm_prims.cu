@@ -144,6 +144,69 @@ static void exclusive_scan_impl(const T* in, T* out, size_t n, cudaStream_t s) {
     SHM_CUDA(cudaFreeAsync(sums, s));
 }
 
+// Two arrays at once (blockIdx.y), two launches at any size: a block of the
+// second adds up the sums of the blocks before it itself.
+template <class T>
+__global__ void k_scan2_reduce(const T* __restrict__ a, const T* __restrict__ b, size_t n, T* __restrict__ sums) {
+    __shared__ T wt[32];
+    __shared__ T tot;
+    const T* in = blockIdx.y ? b : a;
+    const size_t base = (size_t)blockIdx.x * SCAN_TILE + (size_t)threadIdx.x * SCAN_ITEMS;
+    T s = 0;
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; i++)
+        if (base + i < n) s += in[base + i];
+    block_exclusive_scan<T>(s, wt, &tot);
+    if (threadIdx.x == 0) sums[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = tot;
+}
+template <class T>
+__global__ void k_scan2_apply(const T* __restrict__ a, T* __restrict__ ao, const T* __restrict__ b, T* __restrict__ bo,
+                              size_t n, const T* __restrict__ sums) {
+    __shared__ T wt[32];
+    __shared__ T tot;
+    const T* in = blockIdx.y ? b : a;
+    T* out = blockIdx.y ? bo : ao;
+    T before = 0;
+    for (uint32_t i = threadIdx.x; i < blockIdx.x; i += SCAN_THREADS) before += sums[(size_t)blockIdx.y * gridDim.x + i];
+    block_exclusive_scan<T>(before, wt, &tot);
+    before = tot;
+    __syncthreads();
+    const size_t base = (size_t)blockIdx.x * SCAN_TILE + (size_t)threadIdx.x * SCAN_ITEMS;
+    T loc[SCAN_ITEMS];
+    T s = 0;
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; i++) {
+        loc[i] = (base + i < n) ? in[base + i] : T(0);
+        s += loc[i];
+    }
+    T off = before + block_exclusive_scan<T>(s, wt, &tot);
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; i++) {
+        if (base + i < n) out[base + i] = off;
+        off += loc[i];
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = before + tot;
+}
+
+size_t scan_sums_words(size_t n) { return 2 * ((n + SCAN_TILE - 1) / SCAN_TILE) + 2; }
+
+template <class T>
+void exclusive_scan2(const T* a, T* ao, const T* b, T* bo, size_t n, T* sums, cudaStream_t s) {
+    const dim3 grid((unsigned)std::max<size_t>(1, (n + SCAN_TILE - 1) / SCAN_TILE), b ? 2 : 1);
+    if (grid.x > 1) {
+        k_scan2_reduce<T><<<grid, SCAN_THREADS, 0, s>>>(a, b, n, sums);
+        SHM_CUDA(cudaGetLastError());
+        count_launch();
+    }
+    k_scan2_apply<T><<<grid, SCAN_THREADS, 0, s>>>(a, ao, b, bo, n, sums);
+    SHM_CUDA(cudaGetLastError());
+    count_launch();
+}
+template void exclusive_scan2<uint32_t>(const uint32_t*, uint32_t*, const uint32_t*, uint32_t*, size_t, uint32_t*,
+                                        cudaStream_t);
+template void exclusive_scan2<uint64_t>(const uint64_t*, uint64_t*, const uint64_t*, uint64_t*, size_t, uint64_t*,
+                                        cudaStream_t);
+
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, cudaStream_t s) {
     exclusive_scan_impl<uint32_t>(in, out, n, s);
 }

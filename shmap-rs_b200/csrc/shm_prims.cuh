@@ -11,6 +11,14 @@ namespace shm {
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, cudaStream_t s);
 void exclusive_scan_u64(const uint64_t* in, uint64_t* out, size_t n, cudaStream_t s);
 
+// The same for arrays a and (unless null) b of one length, in at most two
+// launches, with sums[scan_sums_words(n)] of scratch from the caller: for the
+// per-read arrays of a batch (a block of the second launch reads the sums of
+// all blocks before it, so not for many millions of elements).
+size_t scan_sums_words(size_t n);
+template <class T>
+void exclusive_scan2(const T* a, T* ao, const T* b, T* bo, size_t n, T* sums, cudaStream_t s);
+
 // Stable sort by key bits [0, key_bits). Sorts (k0,v0) using (k1,v1) as the
 // ping-pong buffer; returns true if the result ended in (k1,v1).
 bool radix_sort_pairs(uint64_t* k0, uint32_t* v0, uint64_t* k1, uint32_t* v1, size_t n, int key_bits,
