@@ -29,7 +29,6 @@ namespace shm {
 constexpr int SKETCH_WIN = 128;          // windows rolled by one thread
 constexpr int MIN_HALFLEN = 5;           // src/buckets.rs:15
 constexpr uint64_t EMPTY_KEY = ~0ULL;    // empty slot of the per-read hash tables
-constexpr int SEED_SMEM_MAX = 4096;      // largest sketch sorted in shared memory
 
 // Per-read status codes written into the output record.
 enum ReadStatus : int32_t {

@@ -329,11 +329,40 @@ __device__ __forceinline__ bool seed_prologue(const BatchView& v, int32_t q, uin
     return true;
 }
 
-// One CTA per read. Arrays (P = power of two >= the read's k-mer capacity):
-// A/B element keys, GA/GB group hash and occs<<1|strand, GF first index then
-// count(), GD hit-list start, E rarest-first sort keys. A and B are dead once
-// the groups are formed, so E lives in A's place and GD in B's: 28 bytes an
-// element, two CTAs an SM at P = 4096.
+// What every seed-preparation form ends with, by one thread.
+__device__ __forceinline__ void seed_epilogue(const BatchView& v, int32_t q, uint32_t m, uint32_t n_u, uint32_t n_proc,
+                                              int32_t S, uint32_t S0, uint64_t smatch, uint32_t mxs, int32_t halflen,
+                                              uint64_t ebound) {
+    v.r_status[q] = ST_UNMAPPED;
+    v.r_nu[q] = (int32_t)n_u;
+    v.r_nproc[q] = (int32_t)n_proc;
+    v.r_S[q] = S;
+    v.r_S0[q] = (int32_t)S0;
+    v.r_smatch[q] = (int64_t)smatch;
+    v.r_maxseed[q] = (int32_t)mxs;
+    v.r_half[q] = halflen;
+    if (smatch >= 0xffffffffULL) {
+        v.r_status[q] = ST_OVERFLOW;
+    } else {
+        v.hw[q] = smatch;
+        const uint64_t eb = genome_bucket_cap(v, ebound, halflen);
+        v.r_eb[q] = eb;
+        v.bt_size[q] = smatch ? bt_slots(v, eb) : 0;
+    }
+    atomicMax(&v.mx->m_max, m);
+    atomicMax(&v.mx->nu_max, n_u);
+    atomicMax(&v.mx->half_max, (uint32_t)halflen);
+    atomicAdd(&v.mx->kmers, (unsigned long long)m);
+    atomicAdd(&v.mx->distinct, (unsigned long long)n_u);
+    atomicAdd(&v.mx->proc_seeds, (unsigned long long)n_proc);
+    atomicAdd(&v.mx->hits, (unsigned long long)smatch);
+}
+
+// One CTA per read, for sketches that fit no shared memory. Arrays in global
+// scratch (P = power of two >= the read's k-mer capacity): A/B element keys,
+// GA/GB group hash and occs<<1|strand, GF first index then count(), GD hit-list
+// start, E rarest-first sort keys. A and B are dead once the groups are
+// formed, so E lives in A's place and GD in B's: 28 bytes an element.
 struct SeedArrays {
     uint64_t *A, *GA, *E;
     uint32_t *B, *GB, *GF, *GD;
@@ -462,41 +491,14 @@ __device__ void seedprep_one(const BatchView& v, int32_t q, uint32_t P, const Se
     const uint64_t smatch = block_reduce_sum<uint64_t>(l_sm, sw64, &t64);
     const uint64_t ebound = block_reduce_sum<uint64_t>(l_eb, sw64, &t64);
     const uint32_t mxs = block_reduce_max(l_max, sw32);
-    if (tid == 0) {
-        v.r_status[q] = ST_UNMAPPED;
-        v.r_nu[q] = (int32_t)n_u;
-        v.r_nproc[q] = (int32_t)n_proc;
-        v.r_S[q] = S;
-        v.r_S0[q] = (int32_t)S0;
-        v.r_smatch[q] = (int64_t)smatch;
-        v.r_maxseed[q] = (int32_t)mxs;
-        v.r_half[q] = halflen;
-        if (smatch >= 0xffffffffULL) {
-            v.r_status[q] = ST_OVERFLOW;
-        } else {
-            v.hw[q] = smatch;
-            const uint64_t eb = genome_bucket_cap(v, ebound, halflen);
-            v.r_eb[q] = eb;
-            v.bt_size[q] = smatch ? bt_slots(v, eb) : 0;
-        }
-        atomicMax(&v.mx->m_max, m);
-        atomicMax(&v.mx->nu_max, n_u);
-        atomicMax(&v.mx->half_max, (uint32_t)halflen);
-        atomicAdd(&v.mx->kmers, (unsigned long long)m);
-        atomicAdd(&v.mx->distinct, (unsigned long long)n_u);
-        atomicAdd(&v.mx->proc_seeds, (unsigned long long)n_proc);
-        atomicAdd(&v.mx->hits, (unsigned long long)smatch);
-    }
+    if (tid == 0) seed_epilogue(v, q, m, n_u, n_proc, S, S0, smatch, mxs, halflen, ebound);
 }
 
-constexpr int SEEDP_THREADS = 512;  // a CTA per read: two CTAs an SM (112 KB of shared memory each at P = 4096)
-template <bool GLOBAL>
+constexpr int SEEDP_THREADS = 512;
 __global__ void __launch_bounds__(SEEDP_THREADS) k_seedprep(BatchView v, const int32_t* __restrict__ list,
-                                                  const uint32_t* __restrict__ n_list_d, uint32_t P, uint8_t* gscr,
-                                                  size_t gscr_per_cta) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    uint8_t* base = GLOBAL ? gscr + (size_t)blockIdx.x * gscr_per_cta : smem;
-    SeedArrays S_ = carve(base, P);
+                                                            const uint32_t* __restrict__ n_list_d, uint32_t P,
+                                                            uint8_t* gscr, size_t gscr_per_cta) {
+    SeedArrays S_ = carve(gscr + (size_t)blockIdx.x * gscr_per_cta, P);
     const int32_t n_list = (int32_t)*n_list_d;
     for (int32_t li = blockIdx.x; li < n_list; li += gridDim.x) {
         seedprep_one(v, list[li], P, S_);
@@ -506,9 +508,9 @@ __global__ void __launch_bounds__(SEEDP_THREADS) k_seedprep(BatchView v, const i
 
 // Seed-preparation bins by the actual sketch size m of each read (reads past
 // their k-mer capacity go to bin 0, whose prologue marks them overflowed):
-// m <= 256, 512 and 1024 the counting form (a warp per read), m <= 4096 a
-// CTA per read in shared memory, larger a CTA with global scratch.
-constexpr int N_SEED_BINS = 5;
+// m <= 256, 512 and 1024 the counting form with a warp per read, m <= 2048,
+// 4096 and 8192 with a CTA per read, larger a CTA sorting in global scratch.
+constexpr int N_SEED_BINS = 7;
 __global__ void k_seed_bins(BatchView v, int32_t* __restrict__ lists, uint32_t* __restrict__ bin_cnt) {
     const int lane = threadIdx.x & 31;
     for (int32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < v.n; base += gridDim.x * blockDim.x) {
@@ -517,7 +519,7 @@ __global__ void k_seed_bins(BatchView v, int32_t* __restrict__ lists, uint32_t* 
         if (q < v.n) {
             const uint32_t m = v.kcnt[q];
             const uint32_t cap = (uint32_t)(v.kcap_off[q + 1] - v.kcap_off[q]);
-            b = m > cap ? 0 : m <= 256 ? 0 : m <= 512 ? 1 : m <= 1024 ? 2 : m <= 4096 ? 3 : 4;
+            b = m > cap ? 0 : m <= 256 ? 0 : m <= 512 ? 1 : m <= 1024 ? 2 : m <= 2048 ? 3 : m <= 4096 ? 4 : m <= 8192 ? 5 : 6;
         }
         const unsigned same = __match_any_sync(0xffffffffu, b);
         const int leader = __ffs(same) - 1;
@@ -884,31 +886,7 @@ __device__ void seedprep_count(const BatchView& v, int32_t q, uint32_t C, uint8_
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l_eb += __shfl_xor_sync(0xffffffffu, l_eb, o);
-    if (lane == 0) {
-        v.r_status[q] = ST_UNMAPPED;
-        v.r_nu[q] = (int32_t)n_u;
-        v.r_nproc[q] = (int32_t)l_np;
-        v.r_S[q] = S;
-        v.r_S0[q] = (int32_t)l_s0;
-        v.r_smatch[q] = (int64_t)l_sm;
-        v.r_maxseed[q] = (int32_t)l_max;
-        v.r_half[q] = halflen;
-        if (l_sm >= 0xffffffffULL) {
-            v.r_status[q] = ST_OVERFLOW;
-        } else {
-            v.hw[q] = l_sm;
-            const uint64_t eb = genome_bucket_cap(v, l_eb, halflen);
-            v.r_eb[q] = eb;
-            v.bt_size[q] = l_sm ? bt_slots(v, eb) : 0;
-        }
-        atomicMax(&v.mx->m_max, m);
-        atomicMax(&v.mx->nu_max, n_u);
-        atomicMax(&v.mx->half_max, (uint32_t)halflen);
-        atomicAdd(&v.mx->kmers, (unsigned long long)m);
-        atomicAdd(&v.mx->distinct, (unsigned long long)n_u);
-        atomicAdd(&v.mx->proc_seeds, (unsigned long long)l_np);
-        atomicAdd(&v.mx->hits, (unsigned long long)l_sm);
-    }
+    if (lane == 0) seed_epilogue(v, q, m, n_u, l_np, S, l_s0, l_sm, l_max, halflen, l_eb);
 }
 
 template <uint32_t C, int W>
@@ -927,6 +905,257 @@ __global__ void __launch_bounds__(W * 32, 4) k_seedprep_c(BatchView v, const int
     for (int32_t li = blockIdx.x * W + wib; li < n; li += gridDim.x * W) {
         seedprep_count(v, list[li], C, base, segs);
         __syncwarp();
+    }
+}
+
+// The counting form with a CTA of NT threads per read, for sketches of up to C
+// k-mers (work linear in m, where a bitonic sort of them took 66 to 91 stages
+// of barriers and 160,000 warp instructions a read of 1,500 k-mers: 12,500
+// dense reads 4.5 ms, so _PENDING_). Shared memory as seedprep_count's, with
+// the radix digits counted per warp: each warp orders a contiguous part of the
+// groups, its digit offsets after those of the warps before it.
+template <uint32_t C, int NT>
+struct SeedCta {
+    static constexpr int NW = NT / 32, ND = 1 << SEEDC_DIGIT;
+    uint64_t Sh[C];
+    uint32_t Srs[C], Rc[C + 1], Ra[C];
+    uint16_t P0[C], P1[C];
+    uint32_t RH[ND * NW];
+    uint32_t sw32[32], t32;
+    uint64_t sw64[32], t64;
+};
+
+// Exclusive scan, in place, of X[0..n) by a CTA of NT threads (n a multiple
+// of NT or below it); every thread owns consecutive words.
+template <int NT>
+__device__ __forceinline__ void block_scan_words(uint32_t* X, uint32_t n, uint32_t* sw, uint32_t* tot) {
+    const uint32_t per = (n + NT - 1) / NT, b0 = min(n, (uint32_t)threadIdx.x * per), b1 = min(n, b0 + per);
+    uint32_t sum = 0;
+    for (uint32_t j = b0; j < b1; j++) sum += X[j];
+    uint32_t run = block_scan_excl<uint32_t>(sum, sw, tot);
+    for (uint32_t j = b0; j < b1; j++) {
+        const uint32_t c = X[j];
+        X[j] = run;
+        run += c;
+    }
+    __syncthreads();
+}
+
+template <uint32_t C, int NT>
+__device__ void seedprep_cta(const BatchView& v, int32_t q, SeedCta<C, NT>& T) {
+    constexpr int NW = NT / 32, ND = 1 << SEEDC_DIGIT;
+    constexpr uint32_t PER = C / NT;  // elements a thread
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    uint32_t m;
+    uint64_t kb;
+    int32_t S, halflen;
+    if (!seed_prologue(v, q, C, tid == 0, m, kb, S, halflen)) return;
+    // the k-mers into buckets of an order-preserving map of the hash, then
+    // into hash order by insertion (about one k-mer a bucket)
+    const uint32_t Ht = max((uint32_t)NT, (uint32_t)pow2_ceil(m));  // <= C
+    const uint64_t mul = v.P.slot_mul[31 - __clz(Ht)];
+    for (uint32_t i = tid; i < Ht; i += NT) T.Rc[i] = 0;
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t i = tid; i < m; i += NT) atomicAdd(&T.Rc[(uint32_t)__umul64hi(v.km_h[kb + i], mul)], 1u);
+    __syncthreads();
+    block_scan_words<NT>(T.Rc, Ht, T.sw32, &T.t32);
+#pragma unroll 4
+    for (uint32_t i = tid; i < m; i += NT) {
+        const uint64_t h = v.km_h[kb + i];
+        const uint32_t pos = atomicAdd(&T.Rc[(uint32_t)__umul64hi(h, mul)], 1u);
+        T.Sh[pos] = h;
+        T.Srs[pos] = v.km_rs[kb + i];
+    }
+    __syncthreads();
+    for (uint32_t b = tid; b < Ht; b += NT) {  // bucket b spans [Rc[b-1], Rc[b])
+        const uint32_t s0 = b ? T.Rc[b - 1] : 0u, e1 = T.Rc[b];
+        for (uint32_t x = s0 + 1; x < e1; x++) {
+            const uint64_t hx = T.Sh[x];
+            const uint32_t rx = T.Srs[x];
+            uint32_t y = x;
+            while (y > s0 && T.Sh[y - 1] > hx) {
+                T.Sh[y] = T.Sh[y - 1];
+                T.Srs[y] = T.Srs[y - 1];
+                y--;
+            }
+            T.Sh[y] = hx;
+            T.Srs[y] = rx;
+        }
+    }
+    __syncthreads();
+    // groups of equal hashes, compacted in place (src/shmap/seeding.rs:45-67):
+    // a thread's elements are in registers before anything is written; Rc gets
+    // each group's first element, Srs its smallest r << 1 | strand
+    uint64_t eh[PER];
+    uint32_t er[PER], first = 0, nf = 0;
+    const uint32_t e0 = (uint32_t)tid * PER;
+    {
+        uint64_t hp = e0 > 0 && e0 < m ? T.Sh[e0 - 1] : 0;
+#pragma unroll
+        for (uint32_t j = 0; j < PER; j++) {
+            const uint32_t e = e0 + j;
+            eh[j] = e < m ? T.Sh[e] : 0;
+            er[j] = e < m ? T.Srs[e] : 0;
+            if (e < m && (e == 0 || eh[j] != hp)) {
+                first |= 1u << j;
+                nf++;
+            }
+            hp = eh[j];
+        }
+    }
+    const uint32_t gbase = block_scan_excl<uint32_t>(nf, T.sw32, &T.t32);  // (its barriers: every element is read)
+    const uint32_t n_u = T.t32;
+    {
+        uint32_t g = gbase;
+#pragma unroll
+        for (uint32_t j = 0; j < PER; j++)
+            if (first >> j & 1u) {
+                T.Sh[g] = eh[j];
+                T.Srs[g] = er[j];
+                T.Rc[g] = e0 + j;
+                g++;
+            }
+    }
+    if (tid == 0) T.Rc[n_u] = m;
+    __syncthreads();
+    {
+        uint32_t g = gbase;
+#pragma unroll
+        for (uint32_t j = 0; j < PER; j++) {
+            if (first >> j & 1u) g++;
+            else if (e0 + j < m) atomicMin(&T.Srs[g - 1], er[j]);
+        }
+    }
+    __syncthreads();
+    for (uint32_t g = tid; g < n_u; g += NT)  // the representative: seeding.rs:56
+        T.Srs[g] = ((T.Rc[g + 1] - T.Rc[g]) << 1) | (T.Srs[g] & 1u);
+    __syncthreads();
+    if (v.P.os) S = (int32_t)n_u;  // mod.rs:732-736
+
+    // count() probes (index.rs:204-213)
+    uint32_t maxc = 0;
+    for (uint32_t g0 = 0; g0 < n_u; g0 += NT * SEEDC_U) {
+        uint64_t hh[SEEDC_U];
+        bool on[SEEDC_U];
+        uint32_t a[SEEDC_U], cnt[SEEDC_U];
+#pragma unroll
+        for (int u = 0; u < SEEDC_U; u++) {
+            const uint32_t g = g0 + NT * u + tid;
+            on[u] = g < n_u;
+            hh[u] = on[u] ? T.Sh[g] : 0;
+        }
+        idx_lookup_u<SEEDC_U>(v.I, hh, on, a, cnt);
+#pragma unroll
+        for (int u = 0; u < SEEDC_U; u++) {
+            const uint32_t g = g0 + NT * u + tid;
+            if (on[u]) {
+                T.Rc[g] = cnt[u];
+                T.Ra[g] = a[u];
+                maxc = max(maxc, cnt[u]);
+            }
+        }
+    }
+    maxc = block_reduce_max(maxc, T.sw32);
+
+    // rarest first, stable over hash order (seeding.rs:71)
+    const uint16_t* ord = nullptr;  // null: identity
+    uint16_t* pout = T.P0;
+    const uint32_t part = ((n_u + NW - 1) / NW + 31) / 32 * 32;
+    const uint32_t i0 = min(n_u, (uint32_t)wid * part), i1 = min(n_u, i0 + part);
+    for (int sh = 0; sh < 32 && (maxc >> sh) != 0; sh += SEEDC_DIGIT) {
+        for (uint32_t i = tid; i < ND * NW; i += NT) T.RH[i] = 0;
+        __syncthreads();
+        for (uint32_t i = i0 + lane; i < i1; i += 32) {
+            const uint32_t g = ord ? ord[i] : i;
+            atomicAdd(&T.RH[((T.Rc[g] >> sh) & (ND - 1)) * NW + wid], 1u);
+        }
+        __syncthreads();
+        block_scan_words<NT>(T.RH, ND * NW, T.sw32, &T.t32);
+        for (uint32_t c0 = i0; c0 < i1; c0 += 32) {
+            const uint32_t i = c0 + lane;
+            const bool valid = i < i1;
+            const uint32_t g = valid ? (ord ? ord[i] : i) : 0u;
+            const uint32_t d = valid ? (T.Rc[g] >> sh) & (ND - 1) : ND + (uint32_t)lane;
+            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            const int leader = __ffs(peers) - 1;
+            uint32_t at = (valid && lane == leader) ? T.RH[d * NW + wid] : 0u;
+            at = __shfl_sync(0xffffffffu, at, leader);
+            if (valid) pout[at + __popc(peers & lt)] = (uint16_t)g;
+            __syncwarp();
+            if (valid && lane == leader) T.RH[d * NW + wid] = at + __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        ord = pout;
+        pout = pout == T.P0 ? T.P1 : T.P0;
+    }
+
+    // seeding prefix (seeding.rs:101), as in seedprep_count
+    const bool pht = v.P.metric != MET_BUCKET_SH;  // (these reads are never on chip)
+    if (pht) {
+        const uint64_t pb = v.pht_off[q], pe = v.pht_off[q + 1];
+        for (uint64_t i = pb + tid; i < pe; i += NT) v.pht_val[i] = 0xffffffffu;
+    }
+    uint32_t po_carry = 0, l_np = 0, l_s0 = 0, l_max = 0;
+    uint64_t pc_carry = 0, l_sm = 0, l_eb = 0;
+    for (uint32_t c0 = 0; c0 < n_u; c0 += NT) {
+        const uint32_t i = c0 + tid;
+        const bool valid = i < n_u;
+        const uint32_t g = valid ? (ord ? ord[i] : i) : 0u;
+        const uint32_t cnt = valid ? T.Rc[g] : 0u;
+        const uint32_t os = valid ? T.Srs[g] : 0u, occs = os >> 1;
+        const uint32_t po = po_carry + block_scan_excl<uint32_t>(occs, T.sw32, &T.t32);
+        const uint64_t pc = pc_carry + block_scan_excl<uint64_t>((uint64_t)cnt, T.sw64, &T.t64);
+        if (valid) {
+            v.sd[kb + i] = SeedRec{T.Ra[g], cnt, os, po};
+            if ((int64_t)po < (int64_t)S) {
+                v.sd_hpre[kb + i] = (uint32_t)pc;
+                l_np++;
+                l_s0 += occs;
+                l_sm += cnt;
+                l_max = max(l_max, cnt);
+            }
+        }
+        po_carry += T.t32;
+        pc_carry += T.t64;
+        __syncthreads();  // the totals are read before the next scan writes them
+    }
+    const uint32_t n_proc = block_reduce_sum<uint32_t>(l_np, T.sw32, &T.t32);
+    const uint32_t S0 = block_reduce_sum<uint32_t>(l_s0, T.sw32, &T.t32);
+    const uint64_t smatch = block_reduce_sum<uint64_t>(l_sm, T.sw64, &T.t64);
+    const uint32_t mxs = block_reduce_max(l_max, T.sw32);
+    for (uint32_t c0 = 0; c0 < n_u; c0 += NT * SEEDC_U) {
+        uint64_t hh[SEEDC_U];
+        uint32_t a[SEEDC_U], cnt[SEEDC_U], ii[SEEDC_U];
+        bool on[SEEDC_U], proc[SEEDC_U];
+#pragma unroll
+        for (int u = 0; u < SEEDC_U; u++) {
+            ii[u] = c0 + NT * u + tid;
+            on[u] = ii[u] < n_u;
+            proc[u] = ii[u] < n_proc;  // the processed seeds are a prefix of the order
+            const uint32_t g = on[u] ? (ord ? ord[ii[u]] : ii[u]) : 0u;
+            hh[u] = on[u] ? T.Sh[g] : 0;
+            a[u] = on[u] ? T.Ra[g] : 0u;
+            cnt[u] = on[u] ? T.Rc[g] : 0u;
+        }
+        l_eb += seed_bucket_bound_u<SEEDC_U>(v, a, cnt, proc, halflen, v.I.seg_off);
+        if (pht) pht_insert_u<SEEDC_U>(v, q, hh, ii, on);
+    }
+    const uint64_t ebound = block_reduce_sum<uint64_t>(l_eb, T.sw64, &T.t64);
+    if (tid == 0) seed_epilogue(v, q, m, n_u, n_proc, S, S0, smatch, mxs, halflen, ebound);
+}
+
+template <uint32_t C, int NT>
+__global__ void __launch_bounds__(NT) k_seedprep_cta(BatchView v, const int32_t* __restrict__ list,
+                                                     const uint32_t* __restrict__ n_list) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    SeedCta<C, NT>& T = *(SeedCta<C, NT>*)smem;
+    const int32_t n = (int32_t)*n_list;
+    for (int32_t li = blockIdx.x; li < n; li += gridDim.x) {
+        seedprep_cta<C, NT>(v, list[li], T);
+        __syncthreads();
     }
 }
 
@@ -3195,9 +3424,9 @@ struct BatchPlan {
     uint64_t* chunk_off;   // n+1
     uint64_t* kcap_off;    // n+1
     uint64_t* pht_off;     // n+1
-    // reads whose capacity exceeds 256 / 512 / 1024 / 4096
-    uint32_t n_cap_256 = 0, n_cap_512 = 0, n_cap_1024 = 0, n_cap_4096 = 0;
-    uint32_t P_g = 0;                          // power of two >= every capacity above 4096
+    // reads whose capacity exceeds 256 / 512 / ...
+    uint32_t n_cap_256 = 0, n_cap_512 = 0, n_cap_1024 = 0, n_cap_2048 = 0, n_cap_4096 = 0, n_cap_8192 = 0;
+    uint32_t P_g = 0;                          // power of two >= every capacity above 8192
     uint64_t max_cap = 0;                      // largest k-mer capacity of a read
     int64_t max_len = 0;                       // longest read
     size_t bytes = 0;
@@ -3273,7 +3502,7 @@ static void plan_batch(uint8_t* h_plan, const int64_t* h_offs, int32_t n, int32_
     bp.P_g = 0;
     bp.max_cap = 0;
     bp.max_len = 0;
-    bp.n_cap_256 = bp.n_cap_512 = bp.n_cap_1024 = bp.n_cap_4096 = 0;
+    bp.n_cap_256 = bp.n_cap_512 = bp.n_cap_1024 = bp.n_cap_2048 = bp.n_cap_4096 = bp.n_cap_8192 = 0;
     bp.roff[0] = base0;
     bp.chunk_off[0] = 0;
     bp.kcap_off[0] = 0;
@@ -3291,8 +3520,10 @@ static void plan_batch(uint8_t* h_plan, const int64_t* h_offs, int32_t n, int32_
         if (cap > 256) bp.n_cap_256++;
         if (cap > 512) bp.n_cap_512++;
         if (cap > 1024) bp.n_cap_1024++;
-        if (cap > 4096) {
-            bp.n_cap_4096++;
+        if (cap > 2048) bp.n_cap_2048++;
+        if (cap > 4096) bp.n_cap_4096++;
+        if (cap > 8192) {
+            bp.n_cap_8192++;
             bp.P_g = std::max<uint32_t>(bp.P_g, (uint32_t)pow2_host(cap));
         }
     }
@@ -3626,24 +3857,38 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
         SHM_CUDA(cudaStreamWaitEvent(c->side_stream, c->fork, 0));
     }
     cudaStream_t s2 = c->side_stream;
-    if (bp.P_g) {  // m > 4096: CTA per read, global scratch
+    if (bp.P_g) {  // m > 8192: CTA per read, global scratch
         const size_t bytes = SEED_BYTES_PER_ELEM * bp.P_g;
-        const int grid = (int)std::min<size_t>(bp.n_cap_4096, 296);
+        const int grid = (int)std::min<size_t>(bp.n_cap_8192, 296);
         S.seed_gscr.reserve(bytes * (size_t)grid);
-        k_seedprep<true><<<grid, 256, 0, s2>>>(v, LB + 4 * (size_t)n, NB + 4, bp.P_g, S.seed_gscr.p, bytes);
+        k_seedprep<<<grid, 256, 0, s2>>>(v, LB + 6 * (size_t)n, NB + 6, bp.P_g, S.seed_gscr.p, bytes);
         SHM_CUDA(cudaGetLastError());
         count_launch();
     }
-    if (bp.n_cap_1024) {  // 1024 < m <= 4096: CTA per read
-        const uint32_t P = 4096;
-        const size_t bytes = SEED_BYTES_PER_ELEM * P;
-        if ((int)bytes > c->seed_smem_set) {
-            SHM_CUDA(cudaFuncSetAttribute(k_seedprep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-            c->seed_smem_set = (int)bytes;
-        }
-        k_seedprep<false><<<grid_for((size_t)bp.n_cap_1024 * SEEDP_THREADS, SEEDP_THREADS, 2), SEEDP_THREADS, bytes,
-                            s2>>>(v, LB + 3 * (size_t)n,
-                                                                                               NB + 3, P, nullptr, 0);
+    if (bp.n_cap_1024 && !c->seed_cta_set) {
+        SHM_CUDA(cudaFuncSetAttribute(k_seedprep_cta<2048, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(SeedCta<2048, 256>)));
+        SHM_CUDA(cudaFuncSetAttribute(k_seedprep_cta<4096, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(SeedCta<4096, 512>)));
+        SHM_CUDA(cudaFuncSetAttribute(k_seedprep_cta<8192, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(SeedCta<8192, 1024>)));
+        c->seed_cta_set = 1;
+    }
+    if (bp.n_cap_4096) {  // 4096 < m <= 8192: one CTA an SM
+        k_seedprep_cta<8192, 1024><<<grid_for((size_t)bp.n_cap_4096, 1, 1), 1024, sizeof(SeedCta<8192, 1024>), s2>>>(
+            v, LB + 5 * (size_t)n, NB + 5);
+        SHM_CUDA(cudaGetLastError());
+        count_launch();
+    }
+    if (bp.n_cap_2048) {  // 2048 < m <= 4096: two
+        k_seedprep_cta<4096, 512><<<grid_for((size_t)bp.n_cap_2048, 1, 2), 512, sizeof(SeedCta<4096, 512>), s2>>>(
+            v, LB + 4 * (size_t)n, NB + 4);
+        SHM_CUDA(cudaGetLastError());
+        count_launch();
+    }
+    if (bp.n_cap_1024) {  // 1024 < m <= 2048: four
+        k_seedprep_cta<2048, 256><<<grid_for((size_t)bp.n_cap_1024, 1, 4), 256, sizeof(SeedCta<2048, 256>), s2>>>(
+            v, LB + 3 * (size_t)n, NB + 3);
         SHM_CUDA(cudaGetLastError());
         count_launch();
     }

@@ -102,7 +102,7 @@ struct MapCtx {
     size_t h_pack_cap = 0;
     // work counters (always on): see WORK_NAMES
     int64_t work[16] = {};
-    int seed_smem_set = 0;   // dynamic shared memory the seed kernels have been allowed so far
+    int seed_cta_set = 0;    // k_seedprep_cta's dynamic shared memory allowed
     int rchip_smem_set = 0;  // k_refine_chip's dynamic shared memory allowed
     int refine_smem_set = 0; // k_refine's
     int seedc_smem_set = 0;
