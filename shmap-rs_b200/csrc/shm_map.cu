@@ -508,8 +508,13 @@ __global__ void __launch_bounds__(SEEDP_THREADS) k_seedprep(BatchView v, const i
 
 // Seed-preparation bins by the actual sketch size m of each read (reads past
 // their k-mer capacity go to bin 0, whose prologue marks them overflowed):
-// m <= 256, 512 and 1024 the counting form with a warp per read, m <= 2048,
-// 4096 and 8192 with a CTA per read, larger a CTA sorting in global scratch.
+// m <= 256 the counting form with a warp per read, m <= 512, 1024, 2048, 4096
+// and 8192 with a CTA of 128 to 1024 threads, larger a CTA sorting in global
+// scratch. (Reads of 257-512 k-mers took a warp each before, whose 12 KB of
+// shared memory left 16 warps an SM: the stage of 120,000 hifi reads 2.50 ms
+// so, 2.33 with a CTA of 128 threads, of 2,049 reads 0.14 and 0.10; with CTAs
+// for the smaller reads too 2.53 and 0.12. CTAs of half the threads are
+// slower: 2.82, and 0.775 against 0.742 for 30,000 ONT-like reads.)
 constexpr int N_SEED_BINS = 7;
 __global__ void k_seed_bins(BatchView v, int32_t* __restrict__ lists, uint32_t* __restrict__ bin_cnt) {
     const int lane = threadIdx.x & 31;
@@ -653,7 +658,8 @@ constexpr int SEEDC_DIGIT = 7;
 __host__ __device__ constexpr size_t seedc_bytes(uint32_t C) { return 24 * (size_t)C + 4 * (1u << SEEDC_DIGIT); }
 constexpr int SEEDC_U = 4;       // groups a lane probes at once
 constexpr int SEEDC_SEGS = 1024;  // references with at most this many segments keep seg_off in shared memory
-static_assert(1024 <= 65536, "group indices of the largest bin fit 16 bits");
+constexpr uint32_t SEEDC_C = 256;  // k-mers of the largest read a warp takes
+constexpr int SEEDC_WARPS = 8;
 inline size_t seedc_seg_bytes(int32_t n_seg) {
     return n_seg <= SEEDC_SEGS ? (4 * (size_t)(n_seg + 1) + 15) / 16 * 16 : 0;
 }
@@ -889,34 +895,34 @@ __device__ void seedprep_count(const BatchView& v, int32_t q, uint32_t C, uint8_
     if (lane == 0) seed_epilogue(v, q, m, n_u, l_np, S, l_s0, l_sm, l_max, halflen, l_eb);
 }
 
-template <uint32_t C, int W>
-__global__ void __launch_bounds__(W * 32, 4) k_seedprep_c(BatchView v, const int32_t* __restrict__ list,
-                                                       const uint32_t* __restrict__ n_list) {
+__global__ void __launch_bounds__(SEEDC_WARPS * 32, 4) k_seedprep_c(BatchView v, const int32_t* __restrict__ list,
+                                                                   const uint32_t* __restrict__ n_list) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int wib = threadIdx.x >> 5;
-    uint8_t* base = smem + (size_t)wib * seedc_bytes(C);
-    uint32_t* s_seg = (uint32_t*)(smem + (size_t)W * seedc_bytes(C));  // seg_off (seedc_seg_bytes)
+    uint8_t* base = smem + (size_t)wib * seedc_bytes(SEEDC_C);
+    uint32_t* s_seg = (uint32_t*)(smem + (size_t)SEEDC_WARPS * seedc_bytes(SEEDC_C));  // seg_off (seedc_seg_bytes)
     const int32_t n = (int32_t)*n_list;
     const bool staged = v.I.n_seg <= SEEDC_SEGS;
     if (staged)
         for (int i = threadIdx.x; i <= v.I.n_seg; i += blockDim.x) s_seg[i] = __ldg(v.I.seg_off + i);
     __syncthreads();
     const uint32_t* segs = staged ? s_seg : v.I.seg_off;
-    for (int32_t li = blockIdx.x * W + wib; li < n; li += gridDim.x * W) {
-        seedprep_count(v, list[li], C, base, segs);
+    for (int32_t li = blockIdx.x * SEEDC_WARPS + wib; li < n; li += gridDim.x * SEEDC_WARPS) {
+        seedprep_count(v, list[li], SEEDC_C, base, segs);
         __syncwarp();
     }
 }
 
 // The counting form with a CTA of NT threads per read, for sketches of up to C
 // k-mers (work linear in m, where a bitonic sort of them took 66 to 91 stages
-// of barriers and 160,000 warp instructions a read of 1,500 k-mers: 12,500
-// dense reads 4.5 ms, so _PENDING_). Shared memory as seedprep_count's, with
+// of barriers and 160,000 warp instructions a read of 1,500 k-mers: the stage
+// of 12,500 dense reads 6.7 ms, 2.5 so). Shared memory as seedprep_count's, with
 // the radix digits counted per warp: each warp orders a contiguous part of the
 // groups, its digit offsets after those of the warps before it.
 template <uint32_t C, int NT>
 struct SeedCta {
     static constexpr int NW = NT / 32, ND = 1 << SEEDC_DIGIT;
+    static_assert(C <= 65536, "group indices fit 16 bits");
     uint64_t Sh[C];
     uint32_t Srs[C], Rc[C + 1], Ra[C];
     uint16_t P0[C], P1[C];
@@ -1093,7 +1099,8 @@ __device__ void seedprep_cta(const BatchView& v, int32_t q, SeedCta<C, NT>& T) {
     }
 
     // seeding prefix (seeding.rs:101), as in seedprep_count
-    const bool pht = v.P.metric != MET_BUCKET_SH;  // (these reads are never on chip)
+    const bool chip = refine_on_chip(v.P, m, halflen);
+    const bool pht = !chip && v.P.metric != MET_BUCKET_SH;
     if (pht) {
         const uint64_t pb = v.pht_off[q], pe = v.pht_off[q + 1];
         for (uint64_t i = pb + tid; i < pe; i += NT) v.pht_val[i] = 0xffffffffu;
@@ -1110,6 +1117,7 @@ __device__ void seedprep_cta(const BatchView& v, int32_t q, SeedCta<C, NT>& T) {
         const uint64_t pc = pc_carry + block_scan_excl<uint64_t>((uint64_t)cnt, T.sw64, &T.t64);
         if (valid) {
             v.sd[kb + i] = SeedRec{T.Ra[g], cnt, os, po};
+            if (chip) v.sd_h[kb + i] = T.Sh[g];
             if ((int64_t)po < (int64_t)S) {
                 v.sd_hpre[kb + i] = (uint32_t)pc;
                 l_np++;
@@ -3866,8 +3874,8 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
         count_launch();
     }
     if (bp.n_cap_1024 && !c->seed_cta_set) {
-        SHM_CUDA(cudaFuncSetAttribute(k_seedprep_cta<2048, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sizeof(SeedCta<2048, 256>)));
+        SHM_CUDA(cudaFuncSetAttribute(k_seedprep_cta<2048, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(SeedCta<2048, 512>)));
         SHM_CUDA(cudaFuncSetAttribute(k_seedprep_cta<4096, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)sizeof(SeedCta<4096, 512>)));
         SHM_CUDA(cudaFuncSetAttribute(k_seedprep_cta<8192, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3887,36 +3895,31 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
         count_launch();
     }
     if (bp.n_cap_1024) {  // 1024 < m <= 2048: four
-        k_seedprep_cta<2048, 256><<<grid_for((size_t)bp.n_cap_1024, 1, 4), 256, sizeof(SeedCta<2048, 256>), s2>>>(
+        k_seedprep_cta<2048, 512><<<grid_for((size_t)bp.n_cap_1024, 1, 4), 512, sizeof(SeedCta<2048, 512>), s2>>>(
             v, LB + 3 * (size_t)n, NB + 3);
         SHM_CUDA(cudaGetLastError());
         count_launch();
     }
     const size_t sgb = seedc_seg_bytes(v.I.n_seg);
     if (!c->seedc_smem_set) {
-        const int sg = (int)seedc_seg_bytes(SEEDC_SEGS);
-        SHM_CUDA(cudaFuncSetAttribute(k_seedprep_c<256, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(8 * seedc_bytes(256)) + sg));
-        SHM_CUDA(cudaFuncSetAttribute(k_seedprep_c<512, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(4 * seedc_bytes(512)) + sg));
-        SHM_CUDA(cudaFuncSetAttribute(k_seedprep_c<1024, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(4 * seedc_bytes(1024)) + sg));
+        SHM_CUDA(cudaFuncSetAttribute(k_seedprep_c, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(SEEDC_WARPS * seedc_bytes(SEEDC_C) + seedc_seg_bytes(SEEDC_SEGS))));
         c->seedc_smem_set = 1;
     }
-    if (bp.n_cap_512) {  // 512 < m <= 1024
-        k_seedprep_c<1024, 4><<<grid_for((size_t)bp.n_cap_512 * 32, 128, 1), 128, 4 * seedc_bytes(1024) + sgb, s2>>>(
+    if (bp.n_cap_512) {  // 512 < m <= 1024: seven
+        k_seedprep_cta<1024, 256><<<grid_for((size_t)bp.n_cap_512, 1, 7), 256, sizeof(SeedCta<1024, 256>), s2>>>(
             v, LB + 2 * (size_t)n, NB + 2);
         SHM_CUDA(cudaGetLastError());
         count_launch();
     }
-    if (bp.n_cap_256) {  // 256 < m <= 512
-        k_seedprep_c<512, 4><<<grid_for((size_t)bp.n_cap_256 * 32, 128, 4), 128, 4 * seedc_bytes(512) + sgb, s2>>>(
+    if (bp.n_cap_256) {  // 256 < m <= 512: fourteen
+        k_seedprep_cta<512, 128><<<grid_for((size_t)bp.n_cap_256, 1, 14), 128, sizeof(SeedCta<512, 128>), s2>>>(
             v, LB + n, NB + 1);
         SHM_CUDA(cudaGetLastError());
         count_launch();
     }
     if (side) SHM_CUDA(cudaEventRecord(c->join, s2));
-    k_seedprep_c<256, 8><<<grid_for((size_t)n * 32, 256, 4), 256, 8 * seedc_bytes(256) + sgb, s>>>(v, LB, NB);
+    k_seedprep_c<<<grid_for((size_t)n * 32, 256, 4), 256, SEEDC_WARPS * seedc_bytes(SEEDC_C) + sgb, s>>>(v, LB, NB);
     SHM_CUDA(cudaGetLastError());
     count_launch();
     if (side) SHM_CUDA(cudaStreamWaitEvent(s, c->join, 0));
