@@ -118,8 +118,7 @@ struct BatchView {
     uint64_t* sd_h;     // per read, the hash of each seed (reads refined on chip only)
     uint32_t* sd_hpre;  // hit words before each processed seed
     const uint64_t* pht_off;
-    uint64_t* pht_key;
-    uint32_t* pht_val;
+    ulonglong2* pht;    // per read, its seeds by hash (PhtRef)
     int32_t *r_status, *r_m, *r_nu, *r_nproc, *r_S, *r_S0, *r_half, *r_maxseed;
     int64_t* r_smatch;
     uint32_t* r_seeded;
@@ -251,17 +250,105 @@ __device__ __forceinline__ bool refine_on_chip(const DevParams& P, uint32_t m, i
     return !P.ap && !bucket_metric(P) && !P.rarity && m <= (uint32_t)RCHIP_M && halflen <= RCHIP_M;
 }
 
-// The sketch hashes are uniform in [0, thr], so their low bits pick the slot.
-__device__ __forceinline__ void pht_insert(const BatchView& v, int32_t q, uint64_t h, uint32_t idx) {
-    const uint64_t base = v.pht_off[q];
-    const uint64_t mask = v.pht_off[q + 1] - base - 1;
-    uint64_t i = h & mask;
-    for (;;) {
-        if (atomicCAS(v.pht_val + base + i, 0xffffffffu, idx) == 0xffffffffu) {
-            v.pht_key[base + i] = h;
-            return;
+// A read's seeds by hash: open addressing over the first pow2_ceil(4 n_u)
+// slots (at least 16) of its room, which its k-mer capacity sized, or all of
+// the room (at least 2 n_u). The sketch hashes are uniform in [0, thr], so
+// their low bits pick the slot; most windows of a noisy read's k-mers are not
+// in the table, and with twice as many slots as seeds their probes ran on:
+// 30,000 ONT-like reads refine in 1.19 ms so, in 0.90 with four times. A slot is
+// the hash and what its readers need of the seed in one 16-byte word: the
+// index, the offset of its occurrences and occurrences << 1 | strand, 21, 21
+// and 22 bits while the read has fewer than 2^21 k-mers, else the index alone
+// (the rest from sd). Separate keys and indices over the whole room, then the
+// seed record, were three sectors a found k-mer: 12,500 dense reads refined in
+// 4.8 ms, in 3.6 so.
+constexpr unsigned long long PHT_EMPTY = ~0ULL;
+constexpr uint32_t PHT_PACK_M = 1u << 21;
+struct PhtRef {
+    ulonglong2* t;
+    uint64_t mask;
+    const SeedRec* sd;
+    bool packed;
+};
+__device__ __forceinline__ PhtRef pht_of(const BatchView& v, int32_t q, uint32_t m, uint32_t n_u) {
+    const uint64_t off = v.pht_off[q], room = v.pht_off[q + 1] - off;
+    return PhtRef{v.pht + off, min(room, max((uint64_t)16, pow2_ceil(4ULL * n_u))) - 1, v.sd + v.kcap_off[q],
+                  m < PHT_PACK_M};
+}
+__device__ __forceinline__ unsigned long long pht_value(const PhtRef& P, uint32_t s, uint32_t os, uint32_t ooff) {
+    return P.packed ? (unsigned long long)s | (unsigned long long)ooff << 21 | (unsigned long long)os << 42 : s;
+}
+
+// Inserts U seeds of one lane; the compare-and-swaps of the U probes are
+// issued together.
+template <int U>
+__device__ __forceinline__ void pht_insert_u(const PhtRef& P, const uint64_t (&h)[U], const unsigned long long (&val)[U],
+                                             const bool (&on)[U]) {
+    uint64_t i[U];
+    bool pend[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        i[u] = h[u] & P.mask;
+        pend[u] = on[u];
+    }
+    for (;;) {  // (at least twice as many slots as seeds: every insert ends)
+        bool more = false;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (!pend[u]) continue;
+            if (atomicCAS(&P.t[i[u]].y, PHT_EMPTY, val[u]) == PHT_EMPTY) {
+                P.t[i[u]].x = h[u];
+                pend[u] = false;
+            } else {
+                i[u] = (i[u] + 1) & P.mask;
+                more = true;
+            }
         }
-        i = (i + 1) & mask;
+        if (!more) break;
+    }
+}
+
+// Looks U hashes of one lane up, the probes issued together: s[u] = the seed
+// index, or -1 when absent (or !on[u]), with its os and ooff.
+template <int U>
+__device__ __forceinline__ void pht_find_u(const PhtRef& P, const uint64_t (&h)[U], const bool (&on)[U],
+                                           int32_t (&s)[U], uint32_t (&os)[U], uint32_t (&ooff)[U]) {
+    uint64_t i[U];
+    bool pend[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        i[u] = h[u] & P.mask;
+        pend[u] = on[u];
+        s[u] = -1;
+        os[u] = ooff[u] = 0;
+    }
+    for (;;) {  // the table keeps empty slots (at least twice as many slots as seeds): every probe ends
+        ulonglong2 e[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) e[u] = pend[u] ? __ldg(P.t + i[u]) : make_ulonglong2(0, PHT_EMPTY);
+        bool more = false;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (!pend[u]) continue;
+            if (e[u].y == PHT_EMPTY) {
+                pend[u] = false;
+            } else if (e[u].x == h[u]) {
+                pend[u] = false;
+                if (P.packed) {
+                    s[u] = (int32_t)(e[u].y & (PHT_PACK_M - 1));
+                    ooff[u] = (uint32_t)(e[u].y >> 21) & (PHT_PACK_M - 1);
+                    os[u] = (uint32_t)(e[u].y >> 42);
+                } else {
+                    s[u] = (int32_t)e[u].y;
+                    os[u] = P.sd[s[u]].os;
+                    ooff[u] = P.sd[s[u]].ooff;
+                }
+            } else {
+                i[u] = (i[u] + 1) & P.mask;
+                more = true;
+            }
+        }
+        if (!more) break;
     }
 }
 
@@ -462,9 +549,9 @@ __device__ void seedprep_one(const BatchView& v, int32_t q, uint32_t P, const Se
     uint32_t po = block_scan_excl<uint32_t>(so, sw32, &t32);
     uint64_t pc = block_scan_excl<uint64_t>(sc, sw64, &t64);
     const bool pht = v.P.metric != MET_BUCKET_SH;  // bucket_SH looks nothing up (these reads are never on chip)
+    const PhtRef T = pht_of(v, q, m, n_u);
     if (pht) {  // the read's probe table starts empty
-        const uint64_t pb = v.pht_off[q], pe = v.pht_off[q + 1];
-        for (uint64_t i = pb + tid; i < pe; i += nt) v.pht_val[i] = 0xffffffffu;
+        for (uint64_t i = tid; i <= T.mask; i += nt) T.t[i] = make_ulonglong2(0, PHT_EMPTY);
         __syncthreads();
     }
     uint32_t l_np = 0, l_s0 = 0, l_max = 0;
@@ -482,7 +569,12 @@ __device__ void seedprep_one(const BatchView& v, int32_t q, uint32_t P, const Se
             l_max = max(l_max, cnt);
             l_eb += seed_bucket_bound(v, S_.GD[g], cnt, halflen);
         }
-        if (pht) pht_insert(v, q, S_.GA[g], i);
+        if (pht) {
+            const uint64_t hh[1] = {S_.GA[g]};
+            const unsigned long long val[1] = {pht_value(T, i, os, po)};
+            const bool on[1] = {true};
+            pht_insert_u<1>(T, hh, val, on);
+        }
         po += occs;
         pc += cnt;
     }
@@ -573,37 +665,6 @@ __device__ __forceinline__ void idx_lookup_u(const DevIndex& I, const uint64_t (
         } else if (ac.w >> 31) {
             idx_lookup_dir(I, h[u], a[u], cnt[u]);
         }
-    }
-}
-
-// pht_insert for U seeds of one lane; the compare-and-swaps of the U probes
-// are issued together.
-template <int U>
-__device__ __forceinline__ void pht_insert_u(const BatchView& v, int32_t q, const uint64_t (&h)[U],
-                                             const uint32_t (&idx)[U], const bool (&on)[U]) {
-    const uint64_t base = v.pht_off[q];
-    const uint64_t mask = v.pht_off[q + 1] - base - 1;
-    uint64_t i[U];
-    bool pend[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-        i[u] = h[u] & mask;
-        pend[u] = on[u];
-    }
-    for (;;) {  // the table has at least twice as many slots as seeds: every insert ends
-        bool more = false;
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            if (!pend[u]) continue;
-            if (atomicCAS(v.pht_val + base + i[u], 0xffffffffu, idx[u]) == 0xffffffffu) {
-                v.pht_key[base + i[u]] = h[u];
-                pend[u] = false;
-            } else {
-                i[u] = (i[u] + 1) & mask;
-                more = true;
-            }
-        }
-        if (!more) break;
     }
 }
 
@@ -833,9 +894,9 @@ __device__ void seedprep_count(const BatchView& v, int32_t q, uint32_t C, uint8_
     // (seeding.rs:101); the processed seeds are a prefix of the order
     const bool chip = refine_on_chip(v.P, m, halflen);
     const bool pht = !chip && v.P.metric != MET_BUCKET_SH;  // bucket_SH looks nothing up
+    const PhtRef T = pht_of(v, q, m, n_u);
     if (pht) {  // the read's probe table starts empty (written before the inserts below)
-        const uint64_t pb = v.pht_off[q], pe = v.pht_off[q + 1];
-        for (uint64_t i = pb + lane; i < pe; i += 32) v.pht_val[i] = 0xffffffffu;
+        for (uint64_t i = lane; i <= T.mask; i += 32) T.t[i] = make_ulonglong2(0, PHT_EMPTY);
         __syncwarp();
     }
     uint32_t po_carry = 0, l_np = 0, l_s0 = 0, l_max = 0;
@@ -871,6 +932,7 @@ __device__ void seedprep_count(const BatchView& v, int32_t q, uint32_t C, uint8_
         l_sm += __shfl_xor_sync(0xffffffffu, l_sm, o);
         l_max = max(l_max, __shfl_xor_sync(0xffffffffu, l_max, o));
     }
+    __syncwarp();
     // bucket bounds of the processed seeds and the probe table, SEEDC_U seeds a
     // lane at once (both are independent of the order they are done in)
     for (uint32_t c0 = 0; c0 < n_u; c0 += 32 * SEEDC_U) {
@@ -888,7 +950,15 @@ __device__ void seedprep_count(const BatchView& v, int32_t q, uint32_t C, uint8_
             cnt[u] = on[u] ? Rc[g] : 0u;
         }
         l_eb += seed_bucket_bound_u<SEEDC_U>(v, a, cnt, proc, halflen, segs);
-        if (pht) pht_insert_u<SEEDC_U>(v, q, hh, ii, on);
+        if (pht) {  // (the records written above, by lanes of this warp)
+            unsigned long long val[SEEDC_U];
+#pragma unroll
+            for (int u = 0; u < SEEDC_U; u++) {
+                const SeedRec sr = on[u] ? v.sd[kb + ii[u]] : SeedRec{0u, 0u, 0u, 0u};
+                val[u] = pht_value(T, ii[u], sr.os, sr.ooff);
+            }
+            pht_insert_u<SEEDC_U>(T, hh, val, on);
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l_eb += __shfl_xor_sync(0xffffffffu, l_eb, o);
@@ -913,6 +983,24 @@ __global__ void __launch_bounds__(SEEDC_WARPS * 32, 4) k_seedprep_c(BatchView v,
     }
 }
 
+// Inserts seed i (hash hs) into an open-addressing table of T 16-bit slots in
+// shared memory (i + 1, 0 = empty; T a power of two): a compare-and-swap on the word
+// that holds the slot.
+__device__ __forceinline__ void slot_insert(uint16_t* tslot, uint32_t T, uint64_t hs, uint32_t i) {
+    uint32_t sl = (uint32_t)hs & (T - 1);
+    for (;;) {
+        uint32_t* w = (uint32_t*)tslot + (sl >> 1);
+        const uint32_t sh = (sl & 1u) * 16u;
+        uint32_t old = *(volatile uint32_t*)w;
+        while (((old >> sh) & 0xffffu) == 0) {
+            const uint32_t got = atomicCAS(w, old, old | ((i + 1u) << sh));
+            if (got == old) return;
+            old = got;  // the other slot of the word changed: look again
+        }
+        sl = (sl + 1) & (T - 1);
+    }
+}
+
 // The counting form with a CTA of NT threads per read, for sketches of up to C
 // k-mers (work linear in m, where a bitonic sort of them took 66 to 91 stages
 // of barriers and 160,000 warp instructions a read of 1,500 k-mers: the stage
@@ -924,7 +1012,8 @@ struct SeedCta {
     static constexpr int NW = NT / 32, ND = 1 << SEEDC_DIGIT;
     static_assert(C <= 65536, "group indices fit 16 bits");
     uint64_t Sh[C];
-    uint32_t Srs[C], Rc[C + 1], Ra[C];
+    uint32_t Srs[C], Rc[2 * C + 1];  // (Ra: Rc's second half)
+    __device__ __forceinline__ uint32_t* Ra() { return Rc + C + 1; }
     uint16_t P0[C], P1[C];
     uint32_t RH[ND * NW];
     uint32_t sw32[32], t32;
@@ -1058,7 +1147,7 @@ __device__ void seedprep_cta(const BatchView& v, int32_t q, SeedCta<C, NT>& T) {
             const uint32_t g = g0 + NT * u + tid;
             if (on[u]) {
                 T.Rc[g] = cnt[u];
-                T.Ra[g] = a[u];
+                T.Ra()[g] = a[u];
                 maxc = max(maxc, cnt[u]);
             }
         }
@@ -1101,10 +1190,6 @@ __device__ void seedprep_cta(const BatchView& v, int32_t q, SeedCta<C, NT>& T) {
     // seeding prefix (seeding.rs:101), as in seedprep_count
     const bool chip = refine_on_chip(v.P, m, halflen);
     const bool pht = !chip && v.P.metric != MET_BUCKET_SH;
-    if (pht) {
-        const uint64_t pb = v.pht_off[q], pe = v.pht_off[q + 1];
-        for (uint64_t i = pb + tid; i < pe; i += NT) v.pht_val[i] = 0xffffffffu;
-    }
     uint32_t po_carry = 0, l_np = 0, l_s0 = 0, l_max = 0;
     uint64_t pc_carry = 0, l_sm = 0, l_eb = 0;
     for (uint32_t c0 = 0; c0 < n_u; c0 += NT) {
@@ -1116,8 +1201,9 @@ __device__ void seedprep_cta(const BatchView& v, int32_t q, SeedCta<C, NT>& T) {
         const uint32_t po = po_carry + block_scan_excl<uint32_t>(occs, T.sw32, &T.t32);
         const uint64_t pc = pc_carry + block_scan_excl<uint64_t>((uint64_t)cnt, T.sw64, &T.t64);
         if (valid) {
-            v.sd[kb + i] = SeedRec{T.Ra[g], cnt, os, po};
+            v.sd[kb + i] = SeedRec{T.Ra()[g], cnt, os, po};
             if (chip) v.sd_h[kb + i] = T.Sh[g];
+            pout[i] = (uint16_t)po;  // (below m <= C)
             if ((int64_t)po < (int64_t)S) {
                 v.sd_hpre[kb + i] = (uint32_t)pc;
                 l_np++;
@@ -1134,22 +1220,41 @@ __device__ void seedprep_cta(const BatchView& v, int32_t q, SeedCta<C, NT>& T) {
     const uint32_t S0 = block_reduce_sum<uint32_t>(l_s0, T.sw32, &T.t32);
     const uint64_t smatch = block_reduce_sum<uint64_t>(l_sm, T.sw64, &T.t64);
     const uint32_t mxs = block_reduce_max(l_max, T.sw32);
-    for (uint32_t c0 = 0; c0 < n_u; c0 += NT * SEEDC_U) {
-        uint64_t hh[SEEDC_U];
-        uint32_t a[SEEDC_U], cnt[SEEDC_U], ii[SEEDC_U];
-        bool on[SEEDC_U], proc[SEEDC_U];
+    for (uint32_t c0 = 0; c0 < n_proc; c0 += NT * SEEDC_U) {  // the processed seeds are a prefix of the order
+        uint32_t a[SEEDC_U], cnt[SEEDC_U];
+        bool proc[SEEDC_U];
 #pragma unroll
         for (int u = 0; u < SEEDC_U; u++) {
-            ii[u] = c0 + NT * u + tid;
-            on[u] = ii[u] < n_u;
-            proc[u] = ii[u] < n_proc;  // the processed seeds are a prefix of the order
-            const uint32_t g = on[u] ? (ord ? ord[ii[u]] : ii[u]) : 0u;
-            hh[u] = on[u] ? T.Sh[g] : 0;
-            a[u] = on[u] ? T.Ra[g] : 0u;
-            cnt[u] = on[u] ? T.Rc[g] : 0u;
+            const uint32_t i = c0 + NT * u + tid;
+            proc[u] = i < n_proc;
+            const uint32_t g = proc[u] ? (ord ? ord[i] : i) : 0u;
+            a[u] = proc[u] ? T.Ra()[g] : 0u;
+            cnt[u] = proc[u] ? T.Rc[g] : 0u;
         }
         l_eb += seed_bucket_bound_u<SEEDC_U>(v, a, cnt, proc, halflen, v.I.seg_off);
-        if (pht) pht_insert_u<SEEDC_U>(v, q, hh, ii, on);
+    }
+    if (pht) {
+        // the probe table is laid out as seed numbers in shared memory (in
+        // Rc's and Ra's place, which the bounds were the last to read) and written out
+        // whole: clearing and filling it in device memory by compare-and-swap
+        // took a sector a slot
+        const PhtRef H = pht_of(v, q, m, n_u);
+        const uint32_t slots = (uint32_t)H.mask + 1;  // <= 4 C
+        uint16_t* const tslot = (uint16_t*)T.Rc;
+        __syncthreads();
+        for (uint32_t i = tid; i < slots / 2; i += NT) T.Rc[i] = 0;
+        __syncthreads();
+        for (uint32_t i = tid; i < n_u; i += NT) slot_insert(tslot, slots, T.Sh[ord ? ord[i] : i], i);
+        __syncthreads();
+        for (uint32_t x = tid; x < slots; x += NT) {
+            const uint32_t i1 = tslot[x];
+            ulonglong2 e = make_ulonglong2(0, PHT_EMPTY);
+            if (i1) {
+                const uint32_t i = i1 - 1, g = ord ? ord[i] : i;
+                e = make_ulonglong2(T.Sh[g], pht_value(H, i, T.Srs[g], pout[i]));
+            }
+            H.t[x] = e;
+        }
     }
     const uint64_t ebound = block_reduce_sum<uint64_t>(l_eb, T.sw64, &T.t64);
     if (tid == 0) seed_epilogue(v, q, m, n_u, n_proc, S, S0, smatch, mxs, halflen, ebound);
@@ -1777,49 +1882,46 @@ struct RefScratch {
     size_t wt_at;     // rarity: ints from a warp's base to its f64 weights (even)
 };
 
-// pht_lookup for U hashes of one lane, the probes issued together; s[u] =
-// the seed index, or -1 when absent (or !on[u]).
-template <int U>
-__device__ __forceinline__ void pht_lookup_u(const BatchView& v, int32_t q, const uint64_t (&h)[U], const bool (&on)[U],
-                                             int32_t (&s)[U]) {
-    const uint64_t base = v.pht_off[q];
-    const uint64_t mask = v.pht_off[q + 1] - base - 1;
-    uint64_t i[U];
-    bool pend[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-        i[u] = h[u] & mask;
-        pend[u] = on[u];
-        s[u] = -1;
-    }
-    for (;;) {  // the table keeps empty slots (at least twice as many slots as seeds): every probe ends
-        uint32_t val[U];
-        uint64_t key[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            val[u] = pend[u] ? v.pht_val[base + i[u]] : 0xffffffffu;
-            key[u] = pend[u] ? v.pht_key[base + i[u]] : 0;
-        }
-        bool more = false;
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            if (!pend[u]) continue;
-            if (val[u] == 0xffffffffu) {
-                pend[u] = false;
-            } else if (key[u] == h[u]) {
-                s[u] = (int32_t)val[u];
-                pend[u] = false;
-            } else {
-                i[u] = (i[u] + 1) & mask;
-                more = true;
-            }
-        }
-        if (!more) break;
-    }
-}
-
 constexpr int REFINE_WARPS = 8;
-constexpr int REFINE_U = 2;  // position chunks whose seeds are fetched together
+constexpr int REFINE_U = 2;   // position chunks whose seeds are fetched together (1 and 4: 1.06 to 1.3 times the stage's time)
+constexpr int REFINE_U2 = 4;  // and window starts whose differences are
+
+// The best window of a candidate, a lane's share of the starts at a time:
+// the first maximum of the score I / d (Containment: d = m; Jaccard: d = m +
+// window - I). Scores are compared as fractions, which orders them as their
+// rounded quotients: two different ones, at most 1, differ by at least
+// 1 / (d d'), which for d, d' < 2^26 is over 2^-52 and more than the spacing of
+// doubles there (larger windows compare the quotients), and equal ones round
+// alike. The division is done once, for the winner.
+// SMALL: m < 2^15, products in 32 bits.
+template <bool SMALL>
+struct BestWindow {
+    int32_t I = -1, l = -1, r = 0, d = 1;
+    __device__ __forceinline__ static bool above(int32_t Ia, int32_t da, int32_t Ib, int32_t db) {
+        if (SMALL) return Ia * db > Ib * da;
+        if (max(da, db) < (1 << 26)) return (int64_t)Ia * db > (int64_t)Ib * da;
+        return __ddiv_rn((double)Ia, (double)da) > __ddiv_rn((double)Ib, (double)db);
+    }
+    __device__ __forceinline__ void take(int32_t I_, int32_t d_, int32_t x, int32_t r_) {
+        if (!above(I_, d_, I, d)) return;  // (the first: I = -1)
+        I = I_;
+        d = d_;
+        l = x;
+        r = r_;
+    }
+    __device__ __forceinline__ void reduce() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            BestWindow b;
+            b.I = __shfl_xor_sync(0xffffffffu, I, o);
+            b.d = __shfl_xor_sync(0xffffffffu, d, o);
+            b.l = __shfl_xor_sync(0xffffffffu, l, o);
+            b.r = __shfl_xor_sync(0xffffffffu, r, o);
+            if (above(b.I, b.d, I, d) || (b.l >= 0 && b.l < l && !above(I, d, b.I, b.d))) *this = b;
+        }
+    }
+    __device__ __forceinline__ double score() const { return l < 0 ? -1.0 : __ddiv_rn((double)I, (double)d); }
+};
 
 // ------------------------------------------------------------------ bucket_LCS
 // Each seed's read positions in decreasing order (its pmatches,
@@ -1846,6 +1948,7 @@ __global__ void __launch_bounds__(256) k_lcs_occ(BatchView v, uint32_t* __restri
         const uint64_t kb = v.kcap_off[q];
         const int64_t len = v.roff[q + 1] - v.roff[q];
         const bool ranked = lcs_ranked(m, len, bm_words);
+        const PhtRef T = pht_of(v, q, (uint32_t)m, (uint32_t)n_u);
         if (ranked) {
             const int32_t nw = (int32_t)((len + 31) >> 5), per = (nw + 255) / 256;
             for (int32_t i = threadIdx.x; i < nw; i += 256) lo_bm[i] = 0;
@@ -1870,9 +1973,10 @@ __global__ void __launch_bounds__(256) k_lcs_occ(BatchView v, uint32_t* __restri
             const uint64_t h[1] = {v.km_h[kb + j]};
             const bool on[1] = {true};
             int32_t sx[1];
-            pht_lookup_u<1>(v, q, h, on, sx);
+            uint32_t os[1], ooff[1];
+            pht_find_u<1>(T, h, on, sx, os, ooff);
             if (sx[0] < 0) continue;  // every sketch hash is a seed's: not taken
-            const uint32_t at = v.sd[kb + sx[0]].ooff + atomicAdd(cnt + kb + sx[0], 1u);
+            const uint32_t at = ooff[0] + atomicAdd(cnt + kb + sx[0], 1u);
             const uint32_t r = v.km_rs[kb + j] >> 1;
             pos[kb + at] = ranked ? lo_pre[r >> 5] + __popc(lo_bm[r >> 5] & ((1u << (r & 31)) - 1u)) : r;
         }
@@ -1990,19 +2094,16 @@ __device__ __forceinline__ int32_t lcs_one(const BatchView& v, const BucketJob* 
     const int64_t end = min(((int64_t)J->bb + 2) * h, (int64_t)(Gend - G0));
     const int32_t W = (int32_t)max(end - from, (int64_t)0);
     if (lane == 0 && W > 0) atomicAdd(&v.mx->refine_kmers, (unsigned long long)W);
+    const PhtRef T = pht_of(v, q, (uint32_t)v.r_m[q], (uint32_t)v.r_nu[q]);
     int32_t li = 0, ld = 0;
     for (int32_t c0 = 0; c0 < W; c0 += 32) {
         const int32_t x = c0 + lane;
         const bool on[1] = {x < W};
         const uint64_t hx[1] = {on[0] ? __ldg(I.ref_h + G0 + (uint32_t)(from + x)) : 0};
         int32_t sx[1];
-        pht_lookup_u<1>(v, q, hx, on, sx);
-        uint32_t occ = 0, ooff = 0;
-        if (sx[0] >= 0) {
-            const SeedRec sr = v.sd[kb + sx[0]];
-            occ = sr.os >> 1;
-            ooff = sr.ooff;
-        }
+        uint32_t osx[1], oox[1];
+        pht_find_u<1>(T, hx, on, sx, osx, oox);
+        const uint32_t occ = osx[0] >> 1, ooff = oox[0];
         for (unsigned mk = __ballot_sync(0xffffffffu, occ > 0); mk; mk &= mk - 1) {
             const int src = __ffs(mk) - 1;
             const uint32_t o = __shfl_sync(0xffffffffu, occ, src), off = __shfl_sync(0xffffffffu, ooff, src);
@@ -2103,6 +2204,7 @@ __device__ __forceinline__ int32_t lcs_bits(const BatchView& v, const BucketJob*
     for (int w = 0; w < WPL; w++) A[w] = ~0u;
 #pragma unroll
     for (int w = 0; w < (HALF ? 1 : WPL); w++) B[w] = ~0u;
+    const PhtRef T = pht_of(v, q, m, (uint32_t)v.r_nu[q]);
     const uint32_t hl = HALF ? (uint32_t)lane & 15u : (uint32_t)lane;
     const bool rev_lane = HALF && lane >= 16;
     constexpr int NM = HALF ? 16 : 32 * WPL;  // mask words a direction, in shared memory: the read's, then the reversed
@@ -2111,14 +2213,9 @@ __device__ __forceinline__ int32_t lcs_bits(const BatchView& v, const BucketJob*
         const bool on[1] = {x < W};
         const uint64_t hx[1] = {on[0] ? __ldg(I.ref_h + G0 + (uint32_t)(from + x)) : 0};
         int32_t sx[1];
-        pht_lookup_u<1>(v, q, hx, on, sx);
-        uint32_t occ = 0, ooff = 0, rk = 0;
-        if (sx[0] >= 0) {
-            const SeedRec sr = v.sd[kb + sx[0]];
-            occ = sr.os >> 1;
-            ooff = sr.ooff;
-            rk = v.lcs_pos[kb + ooff];
-        }
+        uint32_t osx[1], oox[1];
+        pht_find_u<1>(T, hx, on, sx, osx, oox);
+        const uint32_t occ = osx[0] >> 1, ooff = oox[0], rk = sx[0] >= 0 ? v.lcs_pos[kb + ooff] : 0u;
         for (unsigned mk = __ballot_sync(0xffffffffu, occ > 0); mk; mk &= mk - 1) {
             const int src = __ffs(mk) - 1;
             const uint32_t o = __shfl_sync(0xffffffffu, occ, src);
@@ -2155,23 +2252,23 @@ __device__ __forceinline__ int32_t lcs_bits(const BatchView& v, const BucketJob*
             if (HALF) {
                 if (o > 1) {  // only the reversed read's row takes more positions of the k-mer
                     const uint32_t R[1] = {rev_lane ? MA[0] : 0u};
-                    uint32_t T[1] = {A[0]};
+                    uint32_t N[1] = {A[0]};
                     for (uint32_t t = 1; t < o; t++) {
-                        lcs_step<1, true>(T, R, lane);
-                        const bool same = T[0] == A[0];
-                        A[0] = T[0];
+                        lcs_step<1, true>(N, R, lane);
+                        const bool same = N[0] == A[0];
+                        A[0] = N[0];
                         if (__all_sync(0xffffffffu, same)) break;
                     }
                 }
             } else {
                 for (uint32_t t = 0; t < o; t++) {
                     bool same = true;
-                    uint32_t T[HALF ? 1 : WPL];
+                    uint32_t N[HALF ? 1 : WPL];
 #pragma unroll
-                    for (int w = 0; w < (HALF ? 1 : WPL); w++) T[w] = B[w];
+                    for (int w = 0; w < (HALF ? 1 : WPL); w++) N[w] = B[w];
                     lcs_step<HALF ? 1 : WPL, false>(B, MB, lane);
 #pragma unroll
-                    for (int w = 0; w < (HALF ? 1 : WPL); w++) same = same && T[w] == B[w];
+                    for (int w = 0; w < (HALF ? 1 : WPL); w++) same = same && N[w] == B[w];
                     if (t + 1 < o && __all_sync(0xffffffffu, same)) break;
                 }
             }
@@ -2204,7 +2301,6 @@ __device__ __forceinline__ void refine_one(const BatchView& v, BucketJob* J, int
     const DevIndex& I = v.I;
     const int32_t m = v.r_m[q], n_u = v.r_nu[q];
     const int64_t h = v.r_half[q];
-    const uint64_t kb = v.kcap_off[q];
     const int32_t seg = J->seg;
     const uint32_t G0 = __ldg(I.seg_off + seg), Gend = __ldg(I.seg_off + seg + 1);
     const int64_t seglen = (int64_t)(Gend - G0);
@@ -2217,31 +2313,34 @@ __device__ __forceinline__ void refine_one(const BatchView& v, BucketJob* J, int
     __syncwarp();
     // phase 1: seed of every position, its occurrence interval of windows,
     // and the prefix PC of strand agreement (+1 same strand, -1 opposite).
-    // REFINE_U chunks of 32 positions at a time: their reference k-mers,
-    // probe lookups and seed records are fetched together, then the chunks
-    // are folded in order.
+    // REFINE_U chunks of 32 positions at a time: their probes are issued
+    // together, then the chunks are folded in order; the next chunks' reference
+    // k-mers are loaded meanwhile.
+    const PhtRef T = pht_of(v, q, (uint32_t)m, (uint32_t)n_u);
     int32_t pc_carry = 0;
     if (lane == 0) PC[0] = 0;
+    const uint32_t g_from = G0 + (uint32_t)from;
+    uint64_t hx[REFINE_U];
+    uint32_t rsx[REFINE_U];
+#pragma unroll
+    for (int u = 0; u < REFINE_U; u++) {
+        const int32_t x = 32 * u + lane;
+        hx[u] = x < W ? __ldg(I.ref_h + g_from + x) : 0;
+        rsx[u] = x < W ? __ldg(I.ref_rs + g_from + x) : 0;
+    }
     for (int32_t c00 = 0; c00 < W; c00 += 32 * REFINE_U) {
-        uint64_t hx[REFINE_U];
-        uint32_t rsx[REFINE_U], osx[REFINE_U], ooffx[REFINE_U];
+        uint64_t hy[REFINE_U];
+        uint32_t ry[REFINE_U], osx[REFINE_U], ooffx[REFINE_U];
         bool on[REFINE_U];
         int32_t sx[REFINE_U];
 #pragma unroll
         for (int u = 0; u < REFINE_U; u++) {
-            const int32_t x = c00 + 32 * u + lane;
-            on[u] = x < W;
-            const uint32_t gid = G0 + (uint32_t)(from + (on[u] ? x : 0));
-            hx[u] = on[u] ? __ldg(I.ref_h + gid) : 0;
-            rsx[u] = on[u] ? __ldg(I.ref_rs + gid) : 0;
+            const int32_t y = c00 + 32 * (REFINE_U + u) + lane;
+            hy[u] = y < W ? __ldg(I.ref_h + g_from + y) : 0;
+            ry[u] = y < W ? __ldg(I.ref_rs + g_from + y) : 0;
+            on[u] = c00 + 32 * u + lane < W;
         }
-        pht_lookup_u<REFINE_U>(v, q, hx, on, sx);
-#pragma unroll
-        for (int u = 0; u < REFINE_U; u++) {
-            const SeedRec sr = sx[u] >= 0 ? v.sd[kb + sx[u]] : SeedRec{0u, 0u, 0u, 0u};
-            osx[u] = sr.os;
-            ooffx[u] = sr.ooff;
-        }
+        pht_find_u<REFINE_U>(T, hx, on, sx, osx, ooffx);
 #pragma unroll
         for (int u = 0; u < REFINE_U; u++) {
             const int32_t c0 = c00 + 32 * u;
@@ -2302,31 +2401,40 @@ __device__ __forceinline__ void refine_one(const BatchView& v, BucketJob* J, int
             }
             __syncwarp();
         }
+#pragma unroll
+        for (int u = 0; u < REFINE_U; u++) {
+            hx[u] = hy[u];
+            rsx[u] = ry[u];
+        }
     }
     __syncwarp();
-    // phase 2: intersection per window start, score, first maximum. Under
-    // Containment every score is I / m for the same m, and distinct I < 2^31
-    // give distinct quotients, so the first maximum of I is the first
-    // maximum of the score: the division is done once, for the winner.
+    // phase 2: intersection per window start, score, first maximum, REFINE_U2
+    // chunks of 32 starts loaded at once.
     const bool jac = v.P.metric == 1;
-    double best = -1.0;
-    int32_t bl = -1, bI = -1, bS = 0, br = 0;
+    BestWindow<false> best;
     int32_t icarry = 0;
-    for (int32_t c0 = 0; c0 < W; c0 += 32) {
-        const int32_t x = c0 + lane;
-        int32_t dv = x < W ? D[x] : 0;
-        int32_t inc = warp_inclusive_scan(dv) + icarry;
-        icarry = __shfl_sync(0xffffffffu, inc, 31);
-        if (x < W) {
+    for (int32_t c00 = 0; c00 < W; c00 += 32 * REFINE_U2) {
+        int32_t dv[REFINE_U2];
+#pragma unroll
+        for (int u = 0; u < REFINE_U2; u++) {
+            const int32_t x = c00 + 32 * u + lane;
+            dv[u] = x < W ? D[x] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < REFINE_U2; u++) {
+            const int32_t x = c00 + 32 * u + lane;
+            const int32_t inc = warp_inclusive_scan(dv[u]) + icarry;
+            icarry = __shfl_sync(0xffffffffu, inc, 31);
+            if (x >= W) continue;
             int32_t r;
             if (!ap) {
                 r = min(x + m, W);
             } else {
-                const int32_t lim = (int32_t)(__ldg(I.ref_rs + G0 + from + x) >> 1) + m;
+                const int32_t lim = (int32_t)(__ldg(I.ref_rs + g_from + x) >> 1) + m;
                 int32_t lo = x, len = W - x;
                 while (len > 0) {
                     int32_t half = len >> 1;
-                    if ((int32_t)(__ldg(I.ref_rs + G0 + from + lo + half) >> 1) < lim) {
+                    if ((int32_t)(__ldg(I.ref_rs + g_from + lo + half) >> 1) < lim) {
                         lo += half + 1;
                         len -= half + 1;
                     } else {
@@ -2335,50 +2443,19 @@ __device__ __forceinline__ void refine_one(const BatchView& v, BucketJob* J, int
                 }
                 r = lo;
             }
-            const int32_t I_ = inc, sk = r - x;
-            bool better;
-            if (jac) {
-                const double score = __ddiv_rn((double)I_, (double)(m + sk - I_));
-                better = score > best;
-                if (better) best = score;
-            } else {
-                better = I_ > bI;
-            }
-            if (better) {
-                bl = x;
-                bI = I_;
-                bS = (int32_t)PC[r] - (int32_t)PC[x];
-                br = r;
-            }
+            best.take(inc, jac ? m + (r - x) - inc : m, x, r);
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        int32_t obl = __shfl_xor_sync(0xffffffffu, bl, o);
-        int32_t obI = __shfl_xor_sync(0xffffffffu, bI, o);
-        int32_t obS = __shfl_xor_sync(0xffffffffu, bS, o);
-        int32_t obr = __shfl_xor_sync(0xffffffffu, br, o);
-        const bool take = jac ? (ob > best || (ob == best && obl >= 0 && (bl < 0 || obl < bl)))
-                              : (obI > bI || (obI == bI && obl >= 0 && (bl < 0 || obl < bl)));
-        if (take) {
-            best = ob;
-            bl = obl;
-            bI = obI;
-            bS = obS;
-            br = obr;
-        }
-    }
-    if (!jac && bl >= 0) best = __ddiv_rn((double)bI, (double)m);
+    best.reduce();
     if (lane == 0) {
-        J->score = best;
-        if (bl >= 0) {
-            const int32_t tl = (int32_t)(__ldg(I.ref_rs + G0 + from + bl) >> 1);
-            const int32_t tr = (int32_t)(__ldg(I.ref_rs + G0 + from + br - 1) >> 1);
+        J->score = best.score();
+        if (best.l >= 0) {
+            const int32_t tl = (int32_t)(__ldg(I.ref_rs + g_from + best.l) >> 1);
+            const int32_t tr = (int32_t)(__ldg(I.ref_rs + g_from + best.r - 1) >> 1);
             J->t_l = tl;
             J->t_r = tr;
-            J->inter = bI;
-            J->same = bS;
+            J->inter = best.I;
+            J->same = (int32_t)PC[best.r] - (int32_t)PC[best.l];
             J->s_sz = tr - tl + 1;
         }
     }
@@ -2523,6 +2600,7 @@ __device__ void refine_rarity_one(const BatchView& v, BucketJob* J, int32_t q, c
         R.nxt[i] = INT32_MAX;
     }
     __syncwarp();
+    const PhtRef T = pht_of(v, q, (uint32_t)m, (uint32_t)n_u);
     int32_t pc_carry = 0;
     if (lane == 0) R.PC[0] = 0;
     for (int32_t c0 = 0; c0 < W; c0 += 32) {
@@ -2533,7 +2611,8 @@ __device__ void refine_rarity_one(const BatchView& v, BucketJob* J, int32_t q, c
         const uint32_t rs = valid ? __ldg(I.ref_rs + gid) : 0;
         bool on[1] = {valid};
         int32_t sx[1];
-        pht_lookup_u<1>(v, q, hx, on, sx);
+        uint32_t osx[1], oox[1];
+        pht_find_u<1>(T, hx, on, sx, osx, oox);
         const int32_t s = sx[0];
         const SeedRec sr = s >= 0 ? v.sd[kb + s] : SeedRec{0u, 0u, 0u, 0u};
         {
@@ -2790,23 +2869,6 @@ __device__ __forceinline__ int32_t chip_lookup(const uint16_t* tslot, const uint
     }
 }
 
-// Inserts seed i (hash hs) into the table: a compare-and-swap on the word
-// that holds the slot.
-__device__ __forceinline__ void chip_insert(uint16_t* tslot, uint32_t T, uint64_t hs, uint32_t i) {
-    uint32_t sl = (uint32_t)hs & (T - 1);
-    for (;;) {
-        uint32_t* w = (uint32_t*)tslot + (sl >> 1);
-        const uint32_t sh = (sl & 1u) * 16u;
-        uint32_t old = *(volatile uint32_t*)w;
-        while (((old >> sh) & 0xffffu) == 0) {
-            const uint32_t got = atomicCAS(w, old, old | ((i + 1u) << sh));
-            if (got == old) return;
-            old = got;  // the other slot of the word changed: look again
-        }
-        sl = (sl + 1) & (T - 1);
-    }
-}
-
 // best_fixed_length (src/shmap/scoring.rs:189-291) for one candidate window,
 // the arithmetic of refine_one with every per-read array on chip; the strand
 // agreement of the winning window is counted from the ballots.
@@ -2905,8 +2967,7 @@ __device__ __forceinline__ void refine_chip_one(const BatchView& v, BucketJob* J
     __syncwarp();
     // intersection per window start, score, first maximum (as refine_one)
     const bool jac = v.P.metric == 1;
-    double best = -1.0;
-    int32_t bl = -1, bI = -1, br = 0;
+    BestWindow<true> best;
     int32_t icarry = 0;
     for (int32_t c0 = 0; c0 < W; c0 += 32) {
         const int32_t x = c0 + lane;
@@ -2915,38 +2976,11 @@ __device__ __forceinline__ void refine_chip_one(const BatchView& v, BucketJob* J
         icarry = __shfl_sync(0xffffffffu, inc, 31);
         if (x < W) {
             const int32_t r = min(x + m, W);
-            const int32_t I_ = inc, sk = r - x;
-            bool better;
-            if (jac) {
-                const double score = __ddiv_rn((double)I_, (double)(m + sk - I_));
-                better = score > best;
-                if (better) best = score;
-            } else {
-                better = I_ > bI;
-            }
-            if (better) {
-                bl = x;
-                bI = I_;
-                br = r;
-            }
+            best.take(inc, jac ? m + (r - x) - inc : m, x, r);
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        int32_t obl = __shfl_xor_sync(0xffffffffu, bl, o);
-        int32_t obI = __shfl_xor_sync(0xffffffffu, bI, o);
-        int32_t obr = __shfl_xor_sync(0xffffffffu, br, o);
-        const bool take = jac ? (ob > best || (ob == best && obl >= 0 && (bl < 0 || obl < bl)))
-                              : (obI > bI || (obI == bI && obl >= 0 && (bl < 0 || obl < bl)));
-        if (take) {
-            best = ob;
-            bl = obl;
-            bI = obI;
-            br = obr;
-        }
-    }
-    if (!jac && bl >= 0) best = __ddiv_rn((double)bI, (double)m);
+    best.reduce();
+    const int32_t bl = best.l, br = best.r;
     // every lane holds the winner: the strand agreement over [bl, br) from
     // the ballots, a lane per 32 positions
     int32_t same = 0;
@@ -2962,13 +2996,13 @@ __device__ __forceinline__ void refine_chip_one(const BatchView& v, BucketJob* J
         for (int o = 16; o > 0; o >>= 1) same += __shfl_xor_sync(0xffffffffu, same, o);
     }
     if (lane == 0) {
-        J->score = best;
+        J->score = best.score();
         if (bl >= 0) {
             const int32_t tl = (int32_t)(__ldg(I.ref_rs + G0 + from + bl) >> 1);
             const int32_t tr = (int32_t)(__ldg(I.ref_rs + G0 + from + br - 1) >> 1);
             J->t_l = tl;
             J->t_r = tr;
-            J->inter = bI;
+            J->inter = best.I;
             J->same = same;
             J->s_sz = tr - tl + 1;
         }
@@ -3033,7 +3067,7 @@ __global__ void __launch_bounds__(RCHIP_WARPS * 32, 4) k_refine_chip(BatchView v
                     sinfo[i] = sr.os | (sr.ooff << 16);
                 }
                 __syncwarp();
-                for (int32_t i = lane; i < n_u; i += 32) chip_insert(tslot, T, shash[i], (uint32_t)i);
+                for (int32_t i = lane; i < n_u; i += 32) slot_insert(tslot, T, shash[i], (uint32_t)i);
                 __syncwarp();
                 cur = q;
             }
@@ -3319,13 +3353,13 @@ struct MapScratch {
     DevBuf<int64_t> retry_list;
     DevBuf<int32_t> retry_idx;
     DevBuf<uint8_t> zero;  // the arrays a batch starts from zero (ZeroArena)
-    DevBuf<uint64_t> km_h, pht_key, hw_off, bt_off, scan_sums;
+    DevBuf<uint64_t> km_h, hw_off, bt_off, scan_sums;
+    DevBuf<ulonglong2> pht;
     DevBuf<SeedRec> sd;
     DevBuf<uint32_t> pk_codes[2], pk_mask[2];  // host-buffer batches, packed (host/pack.hpp)
     DevBuf<uint32_t> pk_list[2];               // their nonzero mask words as uploaded (index, word)
     DevBuf<uint32_t> dpk_codes, dpk_mask;      // device-resident batches, packed on the device
-    DevBuf<uint64_t> sd_h;
-    DevBuf<uint32_t> km_rs, sd_hpre, pht_val, coff, cidx, cfar, cfar_q, sort_scr;
+    DevBuf<uint32_t> km_rs, sd_hpre, coff, cidx, cfar, cfar_q, sort_scr;
     DevBuf<uint32_t> lcs_pos, lcs_cnt;  // bucket_LCS only
     DevBuf<uint32_t> r_lead;
     DevBuf<int32_t> ref_scr;
@@ -3710,10 +3744,8 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     S.km_h.reserve(kcap + 1);
     S.km_rs.reserve(kcap + 1);
     S.sd.reserve(kcap + 1);
-    S.sd_h.reserve(kcap + 1);
     S.sd_hpre.reserve(kcap + 1);
-    S.pht_key.reserve(phtn);
-    S.pht_val.reserve(phtn);
+    S.pht.reserve(phtn);
     S.r_smatch.reserve((size_t)n);
     S.hw_off.reserve((size_t)n + 1);
     S.bt_off.reserve((size_t)n + 1);
@@ -3779,11 +3811,10 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     v.km_h = S.km_h.p;
     v.km_rs = S.km_rs.p;
     v.sd = S.sd.p;
-    v.sd_h = S.sd_h.p;
+    v.sd_h = S.km_h.p;  // (a chip read's k-mers are read before its seeds are written, and not after)
     v.sd_hpre = S.sd_hpre.p;
     v.pht_off = dp.pht_off;
-    v.pht_key = S.pht_key.p;
-    v.pht_val = S.pht_val.p;
+    v.pht = S.pht.p;
     int32_t* ri = Z.r_i32;
     v.r_status = ri;
     v.r_m = ri + n;
