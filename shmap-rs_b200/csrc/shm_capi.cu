@@ -193,51 +193,81 @@ int shm_sketch(shm_ctx* ctx, const uint8_t* seq, int64_t len, int32_t k, double 
     *n_out = 0;
     if (len < k) return SHM_OK;
     const int64_t nw = len - k + 1;
-    const uint64_t n_chunks = (uint64_t)((nw + shm::SKETCH_WIN - 1) / shm::SKETCH_WIN);
-    shm::DevBuf<uint8_t> d_seq;
-    shm::DevBuf<int64_t> d_off;
-    shm::DevBuf<uint64_t> d_coff, d_h;
-    shm::DevBuf<uint32_t> d_cnt, d_out, d_rs;
-    d_seq.reserve((size_t)len + 32);
+    shm::TmpBuf<uint8_t> d_seq;
+    shm::TmpBuf<int64_t> d_off;
+    shm::TmpBuf<uint64_t> d_coff, d_h;
+    shm::TmpBuf<uint32_t> d_cnt, d_out, d_rs;
+    d_seq.reserve((size_t)len + 32, s);
     SHM_CUDA(cudaMemsetAsync(d_seq.p + len, 0, 32, s));
     SHM_CUDA(cudaMemcpyAsync(d_seq.p, seq, (size_t)len, cudaMemcpyHostToDevice, s));
-    int64_t off[2] = {0, len};
-    uint64_t coff[2] = {0, n_chunks};
-    d_off.reserve(2);
-    d_coff.reserve(2);
+    const int64_t off[2] = {0, len};
+    d_off.reserve(2, s);
     SHM_CUDA(cudaMemcpyAsync(d_off.p, off, sizeof off, cudaMemcpyHostToDevice, s));
-    SHM_CUDA(cudaMemcpyAsync(d_coff.p, coff, sizeof coff, cudaMemcpyHostToDevice, s));
-    d_cnt.reserve(n_chunks + 1);
-    d_out.reserve(n_chunks + 1);
-    shm::SketchLuts* L = shm::create_device_luts(k, s);
+    const shm::SketchLuts* L = shm::ctx_luts(ctx->m, k);
     shm::SketchArgs a{};
     a.seq = d_seq.p;
     a.seq_off = d_off.p;
-    a.chunk_off = d_coff.p;
     a.n_seq = 1;
-    a.n_chunks = n_chunks;
     a.k = k;
     a.thr = shm::h_thres(h_frac);
     a.r_offset = offset;
-    a.chunk_cnt = d_cnt.p;
-    shm::launch_sketch(shm::SK_COUNT, a, L, s);
-    shm::exclusive_scan_u32(d_cnt.p, d_out.p, n_chunks, s);
+    a.base0 = 0;
+    a.base1 = len;
+    // counted by parts (a warp's tiles, or a run of windows), scanned, written
+    // in order. Up to 2^22 windows nothing waits for the count: there is room
+    // for every window, and about the expected number comes back with it.
+    const bool bits = shm::sketch_bits_takes(k);
+    const uint64_t parts = bits ? shm::ordered_warps(a) : (uint64_t)((nw + shm::SKETCH_WIN - 1) / shm::SKETCH_WIN);
+    d_cnt.reserve(parts + 1, s);
+    d_out.reserve(parts + 1, s);
+    if (bits) {
+        shm::launch_sketch_ordered(a, L, d_cnt.p, nullptr, nullptr, 0, s);
+    } else {
+        const uint64_t coff[2] = {0, parts};
+        d_coff.reserve(2, s);
+        SHM_CUDA(cudaMemcpyAsync(d_coff.p, coff, sizeof coff, cudaMemcpyHostToDevice, s));
+        a.chunk_off = d_coff.p;
+        a.n_chunks = parts;
+        a.chunk_cnt = d_cnt.p;
+        shm::launch_sketch(shm::SK_COUNT, a, L, s);
+    }
+    shm::exclusive_scan_u32(d_cnt.p, d_out.p, parts, s);
     uint32_t total = 0;
-    SHM_CUDA(cudaMemcpyAsync(&total, d_out.p + n_chunks, sizeof total, cudaMemcpyDeviceToHost, s));
-    SHM_CUDA(cudaStreamSynchronize(s));
-    d_h.reserve((size_t)total + 1);
-    d_rs.reserve((size_t)total + 1);
-    a.chunk_out = d_out.p;
+    size_t room = (size_t)nw, first = std::min(room, (size_t)(1.25 * h_frac * (double)nw) + 512);
+    if (nw > (int64_t)1 << 22) {
+        SHM_CUDA(cudaMemcpyAsync(&total, d_out.p + parts, sizeof total, cudaMemcpyDeviceToHost, s));
+        SHM_CUDA(cudaStreamSynchronize(s));
+        room = first = total;
+    }
+    d_h.reserve(room + 1, s);
+    d_rs.reserve(room + 1, s);
     a.out_h = d_h.p;
     a.out_rs = d_rs.p;
-    shm::launch_sketch(shm::SK_WRITE, a, L, s);
+    if (bits) {
+        shm::launch_sketch_ordered(a, L, d_cnt.p, nullptr, d_out.p, 0, s);
+    } else {
+        a.chunk_out = d_out.p;
+        shm::launch_sketch(shm::SK_WRITE, a, L, s);
+    }
     ctx->m->launches += 3;
-    std::vector<uint64_t> hh(total);
-    std::vector<uint32_t> rs(total);
-    SHM_CUDA(cudaMemcpyAsync(hh.data(), d_h.p, sizeof(uint64_t) * total, cudaMemcpyDeviceToHost, s));
-    SHM_CUDA(cudaMemcpyAsync(rs.data(), d_rs.p, sizeof(uint32_t) * total, cudaMemcpyDeviceToHost, s));
+    uint8_t* pin = shm::pinned_stage(ctx->m, 16 + 12 * first);
+    uint64_t* hh = (uint64_t*)(pin + 16);
+    uint32_t* rs = (uint32_t*)(hh + first);
+    SHM_CUDA(cudaMemcpyAsync(pin, d_out.p + parts, sizeof total, cudaMemcpyDeviceToHost, s));
+    if (first) {
+        SHM_CUDA(cudaMemcpyAsync(hh, d_h.p, sizeof(uint64_t) * first, cudaMemcpyDeviceToHost, s));
+        SHM_CUDA(cudaMemcpyAsync(rs, d_rs.p, sizeof(uint32_t) * first, cudaMemcpyDeviceToHost, s));
+    }
     SHM_CUDA(cudaStreamSynchronize(s));
-    SHM_CUDA(cudaFree(L));
+    std::memcpy(&total, pin, sizeof total);
+    if (total > first) {  // more than expected (repeats): all of it again
+        pin = shm::pinned_stage(ctx->m, 12 * (size_t)total);
+        hh = (uint64_t*)pin;
+        rs = (uint32_t*)(hh + total);
+        SHM_CUDA(cudaMemcpyAsync(hh, d_h.p, sizeof(uint64_t) * total, cudaMemcpyDeviceToHost, s));
+        SHM_CUDA(cudaMemcpyAsync(rs, d_rs.p, sizeof(uint32_t) * total, cudaMemcpyDeviceToHost, s));
+        SHM_CUDA(cudaStreamSynchronize(s));
+    }
     *n_out = total;
     if ((int64_t)total > cap) return fail(SHM_ERR_CAPACITY, "output capacity too small");
     for (uint32_t i = 0; i < total; i++) {
@@ -259,7 +289,8 @@ int shm_index_build(shm_ctx* ctx, const uint8_t* seq, const int64_t* seg_off, in
     SHM_GUARD_BEGIN
     SHM_CUDA(cudaSetDevice(ctx->m->device));
     auto* ix = new shm_index();
-    ix->s = shm::build_index(seq, seg_off, n_seg, split_names(names, n_seg), k, h_frac, max_matches, ctx->m->stream);
+    ix->s = shm::build_index(seq, seg_off, n_seg, split_names(names, n_seg), k, h_frac, max_matches,
+                             shm::ctx_luts(ctx->m, k), ctx->m->stream);
     ctx->m->launches += 40;
     *out = ix;
     return SHM_OK;
@@ -334,7 +365,7 @@ int shm_index_build_fasta(shm_ctx* ctx, const shm_fasta* fa, int32_t k, double h
     SHM_CUDA(cudaSetDevice(ctx->m->device));
     auto* ix = new shm_index();
     ix->s = shm::build_index(nullptr, fa->f->offs.data(), fa->f->n, split_names(fa->f->names.c_str(), fa->f->n), k,
-                             h_frac, max_matches, ctx->m->stream, fa->f->seq.p);
+                             h_frac, max_matches, shm::ctx_luts(ctx->m, k), ctx->m->stream, fa->f->seq.p);
     ctx->m->launches += 40;
     *out = ix;
     return SHM_OK;
@@ -429,10 +460,10 @@ int shm_index_count(shm_ctx* ctx, const shm_index* idx, const uint64_t* h, int64
     SHM_CUDA(cudaSetDevice(ctx->m->device));
     if (n == 0) return SHM_OK;
     cudaStream_t s = ctx->m->stream;
-    shm::DevBuf<uint64_t> dh;
-    shm::DevBuf<int32_t> dout;
-    dh.reserve((size_t)n);
-    dout.reserve((size_t)n);
+    shm::TmpBuf<uint64_t> dh;
+    shm::TmpBuf<int32_t> dout;
+    dh.reserve((size_t)n, s);
+    dout.reserve((size_t)n, s);
     SHM_CUDA(cudaMemcpyAsync(dh.p, h, sizeof(uint64_t) * (size_t)n, cudaMemcpyHostToDevice, s));
     k_count<<<shm::grid_for((size_t)n, 256), 256, 0, s>>>(idx->s->dev, dh.p, n, dout.p);
     SHM_CUDA(cudaGetLastError());
@@ -450,8 +481,8 @@ int shm_index_hits(shm_ctx* ctx, const shm_index* idx, uint64_t h, int32_t* segm
     SHM_CUDA(cudaSetDevice(ctx->m->device));
     cudaStream_t s = ctx->m->stream;
     const shm::IndexStorage* ix = idx->s;
-    shm::DevBuf<uint32_t> ac;
-    ac.reserve(2);
+    shm::TmpBuf<uint32_t> ac;
+    ac.reserve(2, s);
     k_one_list<<<1, 1, 0, s>>>(ix->dev, h, ac.p);
     SHM_CUDA(cudaGetLastError());
     ctx->m->launches++;

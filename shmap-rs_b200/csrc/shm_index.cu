@@ -180,9 +180,9 @@ __global__ void k_btab_fill(const uint64_t* __restrict__ keys, const uint32_t* _
 // ref_rs, keys[n_kept], key_off[n_kept+1] and hits[n_hits] on the device.
 static void finish_index(IndexStorage* ix, uint64_t thr, uint32_t n_kept, uint32_t n_kmers, uint32_t n_hits,
                          uint32_t highest, cudaStream_t s) {
-    DevBuf<uint32_t> flag;
-    flag.reserve((size_t)n_hits + 1);
-    ix->hit_fw.reserve((size_t)n_hits + 1);
+    TmpBuf<uint32_t> flag;
+    flag.reserve((size_t)n_hits + 1, s);
+    ix->hit_fw.reserve((size_t)n_hits + 1, s);
     k_fw_flags<<<grid_for(n_hits, 256), 256, 0, s>>>(ix->hits.p, n_hits, ix->ref_rs.p, flag.p);
     SHM_CUDA(cudaGetLastError());
     exclusive_scan_u32(flag.p, ix->hit_fw.p, n_hits, s);
@@ -192,7 +192,7 @@ static void finish_index(IndexStorage* ix, uint64_t thr, uint32_t n_kept, uint32
     // mul = floor(2^64 * nb / (thr + 1)): h <= thr maps monotonically onto [0, nb)
     unsigned __int128 m128 = ((unsigned __int128)nb << 64) / ((unsigned __int128)thr + 1);
     const uint64_t mul = m128 > (unsigned __int128)UINT64_MAX ? UINT64_MAX : (uint64_t)m128;
-    ix->dir.reserve((size_t)nb + 1);
+    ix->dir.reserve((size_t)nb + 1, s);
     k_dir_fill<<<grid_for((size_t)std::max<int64_t>(nb, (int64_t)n_kept), 256), 256, 0, s>>>(ix->keys.p, n_kept,
                                                                                            ix->dir.p, nb, mul);
     SHM_CUDA(cudaGetLastError());
@@ -205,7 +205,7 @@ static void finish_index(IndexStorage* ix, uint64_t thr, uint32_t n_kept, uint32
         const int64_t nt = (int64_t)1 << tbits;
         unsigned __int128 t128 = ((unsigned __int128)nt << 64) / ((unsigned __int128)thr + 1);
         tmul = t128 > (unsigned __int128)UINT64_MAX ? UINT64_MAX : (uint64_t)t128;
-        ix->btab.reserve(2 * (size_t)nt);
+        ix->btab.reserve(2 * (size_t)nt, s);
         k_btab_clear<<<grid_for((size_t)nt, 256), 256, 0, s>>>(ix->btab.p, nt);
         SHM_CUDA(cudaGetLastError());
         k_btab_fill<<<grid_for((size_t)n_kept, 256), 256, 0, s>>>(ix->keys.p, ix->key_off.p, n_kept, ix->btab.p,
@@ -239,7 +239,7 @@ static void finish_index(IndexStorage* ix, uint64_t thr, uint32_t n_kept, uint32
 
 IndexStorage* build_index(const uint8_t* h_seq, const int64_t* seg_off_b, int32_t n_seg,
                           const std::vector<std::string>& names, int32_t k, double h_frac, int32_t max_matches,
-                          cudaStream_t s, const uint8_t* d_seq_in) {
+                          const SketchLuts* luts, cudaStream_t s, const uint8_t* d_seq_in) {
     auto* ix = new IndexStorage();
     try {
         SHM_CUDA(cudaGetDevice(&ix->device));
@@ -261,69 +261,89 @@ IndexStorage* build_index(const uint8_t* h_seq, const int64_t* seg_off_b, int32_
             uint64_t ch = nw > 0 ? (uint64_t)((nw + SKETCH_WIN - 1) / SKETCH_WIN) : 0;
             chunk_off[(size_t)i + 1] = chunk_off[(size_t)i] + ch;
         }
-        const uint64_t n_chunks = chunk_off[(size_t)n_seg];
-
-        DevBuf<uint8_t> d_seq;
-        DevBuf<int64_t> d_soff;
-        DevBuf<uint64_t> d_chunk_off;
-        DevBuf<uint32_t> d_ccnt, d_cout;
+        TmpBuf<uint8_t> d_seq;
+        TmpBuf<int64_t> d_soff;
+        TmpBuf<uint32_t> d_ccnt, d_cout;
         if (!d_seq_in) {
-            d_seq.reserve((size_t)total_bases + 32);
+            d_seq.reserve((size_t)total_bases + 32, s);
             SHM_CUDA(cudaMemsetAsync(d_seq.p + total_bases, 0, 32, s));
-            SHM_CUDA(cudaMemcpyAsync(d_seq.p, h_seq + seg_off_b[0], (size_t)total_bases, cudaMemcpyHostToDevice, s));
+            if (total_bases)
+                SHM_CUDA(cudaMemcpyAsync(d_seq.p, h_seq + seg_off_b[0], (size_t)total_bases, cudaMemcpyHostToDevice, s));
         }
-        d_soff.reserve((size_t)n_seg + 1);
+        d_soff.reserve((size_t)n_seg + 1, s);
         SHM_CUDA(cudaMemcpyAsync(d_soff.p, soff.data(), sizeof(int64_t) * ((size_t)n_seg + 1), cudaMemcpyHostToDevice, s));
-        d_chunk_off.reserve((size_t)n_seg + 1);
-        SHM_CUDA(cudaMemcpyAsync(d_chunk_off.p, chunk_off.data(), sizeof(uint64_t) * ((size_t)n_seg + 1),
-                                 cudaMemcpyHostToDevice, s));
-        d_ccnt.reserve(n_chunks + 1);
-        d_cout.reserve(n_chunks + 1);
 
-        SketchLuts* luts = create_device_luts(k, s);
         SketchArgs a{};
         a.seq = d_seq_in ? d_seq_in + seg_off_b[0] : d_seq.p;
         a.seq_off = d_soff.p;
-        a.chunk_off = d_chunk_off.p;
         a.n_seq = n_seg;
-        a.n_chunks = n_chunks;
         a.k = k;
         a.thr = thr;
         a.r_offset = 0;
-        a.chunk_cnt = d_ccnt.p;
-        launch_sketch(SK_COUNT, a, luts, s);
-        exclusive_scan_u32(d_ccnt.p, d_cout.p, n_chunks, s);
+        a.base0 = 0;
+        a.base1 = total_bases;
         uint32_t n_kmers = 0;
-        SHM_CUDA(cudaMemcpyAsync(&n_kmers, d_cout.p + n_chunks, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        SHM_CUDA(cudaStreamSynchronize(s));
-        ix->ref_h.reserve((size_t)n_kmers + 1);
-        ix->ref_rs.reserve((size_t)n_kmers + 1);
-        a.chunk_out = d_cout.p;
-        a.out_h = ix->ref_h.p;
-        a.out_rs = ix->ref_rs.p;
-        launch_sketch(SK_WRITE, a, luts, s);
-        ix->seg_off.reserve((size_t)n_seg + 1);
-        k_seg_offsets<<<grid_for((size_t)n_seg + 1, 128), 128, 0, s>>>(d_chunk_off.p, d_cout.p, n_seg, ix->seg_off.p);
-        SHM_CUDA(cudaGetLastError());
-        SHM_CUDA(cudaFree(luts));
+        ix->seg_off.reserve((size_t)n_seg + 1, s);
+        if (sketch_bits_takes(k) && total_bases > 0) {
+            // on bit planes: every warp's and segment's k-mers counted, then written at their places
+            const uint32_t nw = ordered_warps(a);
+            TmpBuf<uint32_t> seg_cnt;
+            d_ccnt.reserve(nw, s);
+            d_cout.reserve((size_t)nw + 1, s);
+            seg_cnt.reserve((size_t)n_seg, s);
+            SHM_CUDA(cudaMemsetAsync(seg_cnt.p, 0, sizeof(uint32_t) * (size_t)n_seg, s));
+            launch_sketch_ordered(a, luts, d_ccnt.p, seg_cnt.p, nullptr, 0, s);
+            exclusive_scan_u32(d_ccnt.p, d_cout.p, nw, s);
+            exclusive_scan_u32(seg_cnt.p, ix->seg_off.p, (size_t)n_seg, s);
+            SHM_CUDA(cudaMemcpyAsync(&n_kmers, d_cout.p + nw, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+            SHM_CUDA(cudaStreamSynchronize(s));
+            ix->ref_h.reserve((size_t)n_kmers + 1, s);
+            ix->ref_rs.reserve((size_t)n_kmers + 1, s);
+            a.out_h = ix->ref_h.p;
+            a.out_rs = ix->ref_rs.p;
+            launch_sketch_ordered(a, luts, d_ccnt.p, nullptr, d_cout.p, 0, s);
+        } else {
+            const uint64_t n_chunks = chunk_off[(size_t)n_seg];
+            TmpBuf<uint64_t> d_chunk_off;
+            d_chunk_off.reserve((size_t)n_seg + 1, s);
+            SHM_CUDA(cudaMemcpyAsync(d_chunk_off.p, chunk_off.data(), sizeof(uint64_t) * ((size_t)n_seg + 1),
+                                     cudaMemcpyHostToDevice, s));
+            d_ccnt.reserve(n_chunks + 1, s);
+            d_cout.reserve(n_chunks + 1, s);
+            a.chunk_off = d_chunk_off.p;
+            a.n_chunks = n_chunks;
+            a.chunk_cnt = d_ccnt.p;
+            launch_sketch(SK_COUNT, a, luts, s);
+            exclusive_scan_u32(d_ccnt.p, d_cout.p, n_chunks, s);
+            SHM_CUDA(cudaMemcpyAsync(&n_kmers, d_cout.p + n_chunks, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+            SHM_CUDA(cudaStreamSynchronize(s));
+            ix->ref_h.reserve((size_t)n_kmers + 1, s);
+            ix->ref_rs.reserve((size_t)n_kmers + 1, s);
+            a.chunk_out = d_cout.p;
+            a.out_h = ix->ref_h.p;
+            a.out_rs = ix->ref_rs.p;
+            launch_sketch(SK_WRITE, a, luts, s);
+            k_seg_offsets<<<grid_for((size_t)n_seg + 1, 128), 128, 0, s>>>(d_chunk_off.p, d_cout.p, n_seg, ix->seg_off.p);
+            SHM_CUDA(cudaGetLastError());
+        }
         d_seq.release();
         d_ccnt.release();
         d_cout.release();
         ix->h_seg_off.resize((size_t)n_seg + 1);
         SHM_CUDA(cudaMemcpyAsync(ix->h_seg_off.data(), ix->seg_off.p, sizeof(uint32_t) * ((size_t)n_seg + 1),
                                  cudaMemcpyDeviceToHost, s));
-        ix->seg_sz.reserve((size_t)n_seg + 1);
+        ix->seg_sz.reserve((size_t)n_seg + 1, s);
         SHM_CUDA(cudaMemcpyAsync(ix->seg_sz.p, ix->seg_len.data(), sizeof(int32_t) * (size_t)n_seg,
                                  cudaMemcpyHostToDevice, s));
 
         // 2. stable sort of (hash, gidx) by hash
         const size_t n = n_kmers;
-        DevBuf<uint64_t> k0, k1;
-        DevBuf<uint32_t> v0, v1;
-        k0.reserve(n + 1);
-        k1.reserve(n + 1);
-        v0.reserve(n + 1);
-        v1.reserve(n + 1);
+        TmpBuf<uint64_t> k0, k1;
+        TmpBuf<uint32_t> v0, v1;
+        k0.reserve(n + 1, s);
+        k1.reserve(n + 1, s);
+        v0.reserve(n + 1, s);
+        v1.reserve(n + 1, s);
         SHM_CUDA(cudaMemcpyAsync(k0.p, ix->ref_h.p, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, s));
         k_iota<<<grid_for(n, 256), 256, 0, s>>>(v0.p, n);
         SHM_CUDA(cudaGetLastError());
@@ -333,37 +353,36 @@ IndexStorage* build_index(const uint8_t* h_seq, const int64_t* seg_off_b, int32_
         uint32_t* vals = flipped ? v1.p : v0.p;
 
         // 3. CSR over runs of equal hashes
-        DevBuf<uint32_t> flag, fscan;
-        flag.reserve(n + 1);
-        fscan.reserve(n + 1);
+        TmpBuf<uint32_t> flag, fscan;
+        flag.reserve(n + 1, s);
+        fscan.reserve(n + 1, s);
         k_key_flags<<<grid_for(n, 256), 256, 0, s>>>(ks, n, flag.p);
         SHM_CUDA(cudaGetLastError());
         exclusive_scan_u32(flag.p, fscan.p, n, s);
         uint32_t n_keys = 0;
         SHM_CUDA(cudaMemcpyAsync(&n_keys, fscan.p + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         SHM_CUDA(cudaStreamSynchronize(s));
-        DevBuf<uint64_t> keys_all;
-        DevBuf<uint32_t> key_off_all;
-        keys_all.reserve((size_t)n_keys + 1);
-        key_off_all.reserve((size_t)n_keys + 1);
+        TmpBuf<uint64_t> keys_all;
+        TmpBuf<uint32_t> key_off_all;
+        keys_all.reserve((size_t)n_keys + 1, s);
+        key_off_all.reserve((size_t)n_keys + 1, s);
         k_key_emit<<<grid_for(n, 256), 256, 0, s>>>(ks, n, fscan.p, keys_all.p, key_off_all.p);
         SHM_CUDA(cudaGetLastError());
         uint32_t nn = (uint32_t)n;
         SHM_CUDA(cudaMemcpyAsync(key_off_all.p + n_keys, &nn, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
 
-        IdxStatsDev* dst = nullptr;
-        SHM_CUDA(cudaMallocAsync(&dst, sizeof(IdxStatsDev), s));
-        SHM_CUDA(cudaMemsetAsync(dst, 0, sizeof(IdxStatsDev), s));
-        DevBuf<uint32_t> keep, keep_hits, keep_scan, hits_scan;
-        keep.reserve((size_t)n_keys + 1);
-        keep_hits.reserve((size_t)n_keys + 1);
-        keep_scan.reserve((size_t)n_keys + 1);
-        hits_scan.reserve((size_t)n_keys + 1);
-        k_key_keep<<<grid_for(n_keys, 256), 256, 0, s>>>(key_off_all.p, n_keys, max_matches, keep.p, keep_hits.p, dst);
+        TmpBuf<IdxStatsDev> dst;
+        dst.reserve(1, s);
+        SHM_CUDA(cudaMemsetAsync(dst.p, 0, sizeof(IdxStatsDev), s));
+        TmpBuf<uint32_t> keep, keep_hits, keep_scan, hits_scan;
+        keep.reserve((size_t)n_keys + 1, s);
+        keep_hits.reserve((size_t)n_keys + 1, s);
+        keep_scan.reserve((size_t)n_keys + 1, s);
+        hits_scan.reserve((size_t)n_keys + 1, s);
+        k_key_keep<<<grid_for(n_keys, 256), 256, 0, s>>>(key_off_all.p, n_keys, max_matches, keep.p, keep_hits.p, dst.p);
         SHM_CUDA(cudaGetLastError());
         IdxStatsDev hst{};
-        SHM_CUDA(cudaMemcpyAsync(&hst, dst, sizeof hst, cudaMemcpyDeviceToHost, s));
-        SHM_CUDA(cudaFreeAsync(dst, s));
+        SHM_CUDA(cudaMemcpyAsync(&hst, dst.p, sizeof hst, cudaMemcpyDeviceToHost, s));
         exclusive_scan_u32(keep.p, keep_scan.p, n_keys, s);
         exclusive_scan_u32(keep_hits.p, hits_scan.p, n_keys, s);
         uint32_t n_kept = 0, n_hits = 0;
@@ -371,9 +390,9 @@ IndexStorage* build_index(const uint8_t* h_seq, const int64_t* seg_off_b, int32_
         SHM_CUDA(cudaMemcpyAsync(&n_hits, hits_scan.p + n_keys, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         SHM_CUDA(cudaStreamSynchronize(s));
 
-        ix->keys.reserve((size_t)n_kept + 1);
-        ix->key_off.reserve((size_t)n_kept + 1);
-        ix->hits.reserve((size_t)n_hits + 1);
+        ix->keys.reserve((size_t)n_kept + 1, s);
+        ix->key_off.reserve((size_t)n_kept + 1, s);
+        ix->hits.reserve((size_t)n_hits + 1, s);
         k_compact_keys<<<grid_for(n_keys, 256), 256, 0, s>>>(keys_all.p, key_off_all.p, n_keys, keep_scan.p,
                                                              hits_scan.p, ix->keys.p, ix->key_off.p);
         SHM_CUDA(cudaGetLastError());
@@ -518,13 +537,16 @@ struct FileR {
 // Where the checked sections go: device buffers on load, nowhere on a check.
 struct IdxUpload {
     IndexStorage* ix;  // null: check only
+    cudaStream_t s;
     template <class T>
-    void slice(DevBuf<T>* d, size_t at, const T* h, size_t c) {
+    void slice(PoolBuf<T>* d, size_t at, const T* h, size_t c) {
         if (ix && c) SHM_CUDA(cudaMemcpy(d->p + at, h, sizeof(T) * c, cudaMemcpyHostToDevice));
     }
     template <class T>
-    void reserve(DevBuf<T>* d, size_t n) {
-        if (ix) d->reserve(n);
+    void reserve(PoolBuf<T>* d, size_t n) {
+        if (!ix) return;
+        d->reserve(n, s);
+        SHM_CUDA(cudaStreamSynchronize(s));  // the slices are copied on the default stream
     }
 };
 
@@ -597,10 +619,10 @@ void read_index_file(const char* path, IndexStorage& hx, IdxUpload up) {
         }
         IndexStorage* ix = up.ix;
         if (ix) {
-            ix->seg_off.reserve((size_t)n_seg + 1);
+            up.reserve(&ix->seg_off, (size_t)n_seg + 1);
             SHM_CUDA(cudaMemcpy(ix->seg_off.p, hx.h_seg_off.data(), sizeof(uint32_t) * ((size_t)n_seg + 1),
                                 cudaMemcpyHostToDevice));
-            ix->seg_sz.reserve((size_t)n_seg + 1);
+            up.reserve(&ix->seg_sz, (size_t)n_seg + 1);
             if (n_seg)
                 SHM_CUDA(cudaMemcpy(ix->seg_sz.p, hx.seg_len.data(), sizeof(int32_t) * (size_t)n_seg,
                                     cudaMemcpyHostToDevice));
@@ -742,14 +764,14 @@ void save_index(const IndexStorage* ix, const char* path) {
 
 void check_index_file(const char* path) {
     IndexStorage hx;
-    read_index_file(path, hx, IdxUpload{nullptr});
+    read_index_file(path, hx, IdxUpload{nullptr, nullptr});
 }
 
 IndexStorage* load_index(const char* path, cudaStream_t s) {
     auto* ix = new IndexStorage();
     try {
         SHM_CUDA(cudaGetDevice(&ix->device));
-        read_index_file(path, *ix, IdxUpload{ix});
+        read_index_file(path, *ix, IdxUpload{ix, s});
         finish_index(ix, h_thres(ix->h_frac), ix->dev.n_keys, ix->dev.n_kmers, ix->dev.n_hits, ix->max_list, s);
         return ix;
     } catch (...) {

@@ -53,12 +53,69 @@ struct DevBuf {
     DevBuf& operator=(const DevBuf&) = delete;
 };
 
+// Memory of the current device, usable on stream s and, once s has been
+// synchronized, on any: from the device's pool (shm_prims.cu) up to POOL_MOST
+// bytes, above that from cudaMalloc (the pool keeps less than large builds need
+// and would map their memory again after every synchronize: an index of 3.1
+// Gbp took 0.61 s with its 3.1 GB of bases in the pool, 0.33 s without).
+// pool_put gives it back behind the work queued on s.
+constexpr size_t POOL_MOST = (size_t)1 << 28;
+void* pool_get(size_t bytes, cudaStream_t s);
+inline void pool_put(void* p, size_t bytes, cudaStream_t s) {
+    if (bytes > POOL_MOST) cudaFree(p);  // (waits for the device)
+    else cudaFreeAsync(p, s);
+}
+
+// A temporary of work queued on one stream: given back on that stream, behind
+// its last use.
+template <class T>
+struct TmpBuf {
+    T* p = nullptr;
+    size_t bytes = 0;
+    cudaStream_t s = nullptr;
+    void reserve(size_t n, cudaStream_t st) {
+        release();
+        s = st;
+        bytes = n * sizeof(T);
+        p = (T*)pool_get(bytes, st);
+    }
+    void release() {
+        if (p) pool_put(p, bytes, s);
+        p = nullptr;
+    }
+    ~TmpBuf() { release(); }
+    TmpBuf() = default;
+    TmpBuf(const TmpBuf&) = delete;
+    TmpBuf& operator=(const TmpBuf&) = delete;
+};
+
+// An array of an object that outlives the call that made it and is read on any
+// stream: given back when the device is idle (as cudaFree would wait for).
+template <class T>
+struct PoolBuf {
+    T* p = nullptr;
+    size_t bytes = 0;
+    void reserve(size_t n, cudaStream_t s) {
+        if (p) throw shm_cuda_error(cudaErrorInvalidValue);  // made once
+        bytes = n * sizeof(T);
+        p = (T*)pool_get(bytes, s);
+    }
+    ~PoolBuf() {
+        if (!p) return;
+        cudaDeviceSynchronize();
+        pool_put(p, bytes, nullptr);
+    }
+    PoolBuf() = default;
+    PoolBuf(const PoolBuf&) = delete;
+    PoolBuf& operator=(const PoolBuf&) = delete;
+};
+
 struct IndexStorage {
     DevIndex dev{};
-    DevBuf<uint32_t> seg_off, key_off, hits, hit_fw, dir, ref_rs;
-    DevBuf<int32_t> seg_sz;
-    DevBuf<uint64_t> ref_h, keys;
-    DevBuf<uint4> btab;
+    PoolBuf<uint32_t> seg_off, key_off, hits, hit_fw, dir, ref_rs;
+    PoolBuf<int32_t> seg_sz;
+    PoolBuf<uint64_t> ref_h, keys;
+    PoolBuf<uint4> btab;
     std::vector<std::string> names;
     std::vector<int32_t> seg_len;        // bases
     std::vector<uint32_t> h_seg_off;     // k-mer offsets (n_seg+1)
@@ -82,9 +139,10 @@ void check_index_file(const char* path);
 
 // The segments' bases are read from h_seq (host) or, when d_seq is given,
 // from device memory (d_seq + seg_off[i], 32 readable bytes past the end).
+// luts: the tables of k (create_device_luts).
 IndexStorage* build_index(const uint8_t* h_seq, const int64_t* seg_off, int32_t n_seg,
                           const std::vector<std::string>& names, int32_t k, double h_frac, int32_t max_matches,
-                          cudaStream_t s, const uint8_t* d_seq = nullptr);
+                          const SketchLuts* luts, cudaStream_t s, const uint8_t* d_seq = nullptr);
 
 }  // namespace shm
 

@@ -3483,8 +3483,19 @@ struct BatchPlan {
     }
 };
 
+const SketchLuts* ctx_luts(MapCtx* c, int32_t k) {
+    MapScratch& S = *c->scr;
+    if (!S.luts || S.luts_k != k) {
+        if (S.luts) SHM_CUDA(cudaFree(S.luts));
+        S.luts = nullptr;
+        S.luts = create_device_luts(k, c->stream);
+        S.luts_k = k;
+    }
+    return S.luts;
+}
+
 // Grow-only pinned host staging of a context (the plan of the batch in flight).
-static uint8_t* pinned_stage(MapCtx* c, size_t bytes) {
+uint8_t* pinned_stage(MapCtx* c, size_t bytes) {
     if (bytes > c->h_pinned_cap) {
         if (c->h_pinned) SHM_CUDA(cudaFreeHost(c->h_pinned));
         c->h_pinned = nullptr;
@@ -3711,11 +3722,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     // / pk_mask, and pk_words code words are readable there (0: the batch's own)
     plan_batch(h_plan, h_offs, n, p.k, p.h_frac, caps, bp, pk_codes ? pk_base : 0);
     H.mark("plan");
-    if (!S.luts || S.luts_k != p.k) {
-        if (S.luts) SHM_CUDA(cudaFree(S.luts));
-        S.luts = create_device_luts(p.k, s);
-        S.luts_k = p.k;
-    }
+    const SketchLuts* luts = ctx_luts(c, p.k);
     const uint64_t kcap = bp.kcap_off[(size_t)n], phtn = bp.pht_off[(size_t)n];
     // the plan goes up in one copy from its own pinned block, by the copy
     // engine, or (plan_mapped) by a kernel reading the block through its
@@ -3875,7 +3882,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     a.pk_mask = pk_mask;
     a.pk_words = pk_codes ? (pk_words ? pk_words : packed_code_words(batch_bytes)) : 0;
     T.begin(STG_SKETCH, false);
-    launch_sketch(SK_APPEND, a, S.luts, s);
+    launch_sketch(SK_APPEND, a, luts, s);
     T.end();
     if (c->sketch_done) SHM_CUDA(cudaEventRecord(c->sketch_done, s));  // the batch's bytes are free again
 

@@ -117,6 +117,11 @@ struct MapCtx {
 MapCtx* mapctx_create(int device, size_t hbm_budget);
 void mapctx_destroy(MapCtx* c);
 
+// The sketch tables of k on the context's device (kept until another k is asked for).
+const SketchLuts* ctx_luts(MapCtx* c, int32_t k);
+// The context's pinned staging block, grown to at least `bytes` (its contents are the last user's).
+uint8_t* pinned_stage(MapCtx* c, size_t bytes);
+
 // Maps reads [0, n) whose bytes are at d_seq (device) with host offsets
 // h_offs[0..n] (h_offs[0] may be nonzero: bytes are relative to d_seq - h_offs[0]).
 // Writes n records to d_out (device). plain = one read per launch sequence.

@@ -5,15 +5,19 @@
 #include <cstdio>
 
 #include "shm_common.cuh"
+#include "shm_internal.hpp"
 #include "shm_prims.cuh"
 
 #include <mutex>
 
 namespace shm {
 
-// Temporaries of the primitives come from one stream-ordered pool per device
-// that keeps its memory (release threshold: never), so that a call after a
-// synchronize does not map the pool's memory again.
+// Temporaries and indexes come from one stream-ordered pool per device that
+// keeps up to POOL_KEEP bytes of freed memory, so that a call after a
+// synchronize does not map memory again (an index of 155 Mbp took 16 ms to
+// build, most of it in some forty cudaMalloc and cudaFree calls; what is freed
+// beyond that goes back to the device at the next synchronize).
+constexpr uint64_t POOL_KEEP = (uint64_t)1 << 30;
 static cudaMemPool_t prim_pool() {
     static std::mutex mu;
     static cudaMemPool_t pools[64] = {};
@@ -27,15 +31,22 @@ static cudaMemPool_t prim_pool() {
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
         SHM_CUDA(cudaMemPoolCreate(&pools[dev], &props));
-        uint64_t keep = UINT64_MAX;
+        uint64_t keep = POOL_KEEP;
         SHM_CUDA(cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep));
     }
     return pools[dev];
 }
 
+void* pool_get(size_t bytes, cudaStream_t s) {
+    void* p = nullptr;
+    if (bytes > POOL_MOST) SHM_CUDA(cudaMalloc(&p, bytes));
+    else SHM_CUDA(cudaMallocFromPoolAsync(&p, bytes < 16 ? 16 : bytes, prim_pool(), s));
+    return p;
+}
+
 template <class T>
 static void pool_alloc(T** p, size_t bytes, cudaStream_t s) {
-    SHM_CUDA(cudaMallocFromPoolAsync((void**)p, bytes, prim_pool(), s));
+    *p = (T*)pool_get(bytes, s);
 }
 
 
@@ -141,7 +152,7 @@ static void exclusive_scan_impl(const T* in, T* out, size_t n, cudaStream_t s) {
     k_scan_apply<T><<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, n, sums, out, true);
     SHM_CUDA(cudaGetLastError());
     count_launch(2);
-    SHM_CUDA(cudaFreeAsync(sums, s));
+    pool_put(sums, sizeof(T) * (nb + 1), s);
 }
 
 // Two arrays at once (blockIdx.y), two launches at any size: a block of the
@@ -315,8 +326,8 @@ bool radix_sort_pairs(uint64_t* k0, uint32_t* v0, uint64_t* k1, uint32_t* v1, si
         count_launch(2);
         flipped = !flipped;
     }
-    SHM_CUDA(cudaFreeAsync(hist, s));
-    SHM_CUDA(cudaFreeAsync(off, s));
+    pool_put(hist, sizeof(uint32_t) * (size_t)RS_BINS * nb, s);
+    pool_put(off, sizeof(uint32_t) * ((size_t)RS_BINS * nb + 1), s);
     return flipped;
 }
 

@@ -1,6 +1,7 @@
 // Device-wide primitives written for this path: an exclusive scan and a
-// stable LSD radix sort of (u64 key, u32 value) pairs. Temporaries come from
-// a stream-ordered pool per device that keeps its memory.
+// stable LSD radix sort of (u64 key, u32 value) pairs, and the stream-ordered
+// memory pool per device that temporaries and indexes come from (it keeps a
+// bounded amount of freed memory).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -835,15 +835,32 @@ SketchLuts* create_device_luts(int32_t k, cudaStream_t s) {
 // 0.48 / 0.93, 2.32 / 5.54).
 constexpr int SKB_KMIN = 15, SKB_KMAX = 32;
 template <int K>
-void launch_sketch_bits_k(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s);
+int launch_sketch_bits_k(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s);
 template <int... I>
-static void launch_bits_of(int k, const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s,
-                           std::integer_sequence<int, I...>) {
-    (void)((k == SKB_KMIN + I ? (launch_sketch_bits_k<SKB_KMIN + I>(a, tabs, s), true) : false) || ...);
+static int launch_bits_of(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s,
+                          std::integer_sequence<int, I...>) {
+    int r = 0;
+    (void)((a.k == SKB_KMIN + I ? (r = launch_sketch_bits_k<SKB_KMIN + I>(a, tabs, s), true) : false) || ...);
+    return r;
+}
+static int launch_bits(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s) {
+    return launch_bits_of(a, tabs, s, std::make_integer_sequence<int, SKB_KMAX - SKB_KMIN + 1>{});
 }
 bool sketch_bits_takes(int32_t k) { return k >= SKB_KMIN && k <= SKB_KMAX; }
-void launch_sketch_bits(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s) {
-    launch_bits_of(a.k, a, tabs, s, std::make_integer_sequence<int, SKB_KMAX - SKB_KMIN + 1>{});
+void launch_sketch_bits(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s) { launch_bits(a, tabs, s); }
+uint32_t ordered_warps(const SketchArgs& a) {
+    uint32_t any;  // (asks for the grid only: no tables, nothing is launched)
+    SketchArgs b = a;
+    b.ord_cnt = &any;
+    return (uint32_t)launch_bits(b, nullptr, nullptr);
+}
+void launch_sketch_ordered(SketchArgs a, const SketchLuts* luts, uint32_t* cnt, uint32_t* seq_cnt, const uint32_t* off,
+                           uint32_t stride, cudaStream_t s) {
+    a.ord_cnt = cnt;
+    a.ord_seq_cnt = seq_cnt;
+    a.ord_off = off;
+    a.ord_stride = stride;
+    launch_bits(a, (const SketchTabs*)luts, s);
 }
 
 void launch_sketch(int mode, const SketchArgs& a, const SketchLuts* L, cudaStream_t s) {

@@ -42,6 +42,10 @@ struct SketchArgs {
     // SK_APPEND only: seq_off[0] and seq_off[n_seq] on the host, when the caller has
     // them and `luts` is of create_device_luts (the bit-plane kernels take the call then)
     int64_t base0, base1;
+    // launch_sketch_ordered only (set by it)
+    uint32_t *ord_cnt, *ord_seq_cnt;
+    const uint32_t* ord_off;
+    uint32_t ord_stride;
 };
 
 // The five lookup tables of src/sketch.rs:50-97 for one k, in device memory
@@ -52,6 +56,16 @@ SketchLuts* create_device_luts(int32_t k, cudaStream_t s);
 bool sketch_bits_takes(int32_t k);
 struct SketchTabs;
 void launch_sketch_bits(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s);
+// The selected windows of all sequences of a (seq, seq_off, n_seq, k, thr,
+// r_offset, base0, base1; a k that sketch_bits_takes) in sequence order, by
+// warps that each take a contiguous part: warp w's number goes to cnt[w], and
+// from off[w] to off[w + 1] of a.out_h and a.out_rs (off null: from w * stride,
+// at most stride) as many of them as there is room for; seq_cnt (may be null,
+// n_seq zeroed words) counts each sequence's. ordered_warps: the number of
+// warps, cnt's length (the same for the same a).
+uint32_t ordered_warps(const SketchArgs& a);
+void launch_sketch_ordered(SketchArgs a, const SketchLuts* luts, uint32_t* cnt, uint32_t* seq_cnt, const uint32_t* off,
+                           uint32_t stride, cudaStream_t s);
 void launch_sketch(int mode, const SketchArgs& a, const SketchLuts* luts, cudaStream_t s);
 
 // Builds the tables on the device into caller-provided device memory of

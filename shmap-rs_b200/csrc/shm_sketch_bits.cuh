@@ -1,4 +1,5 @@
-// The read sketch on bit planes (SK_APPEND for SKB_KMIN <= k <= SKB_KMAX).
+// The sketch on bit planes (SKB_KMIN <= k <= SKB_KMAX): reads' k-mers in any
+// order (SK_APPEND), or all sequences' in sequence order (launch_sketch_ordered).
 //
 // Selection needs only the top bits of a window's hash h = F ^ R to reject
 // all but about r of the windows, and each bit of F and R is an XOR of one
@@ -254,6 +255,18 @@ struct SkbSource {
     }
 };
 
+// Bit b of lane a's word to bit a of lane b's.
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1) {
+        const uint32_t m = j == 16 ? 0x0000ffffu : j == 8 ? 0x00ff00ffu : j == 4 ? 0x0f0f0f0fu : j == 2 ? 0x33333333u
+                                                                                                 : 0x55555555u;
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = lane & j ? (x & ~m) | ((y & ~m) >> j) : (x & m) | ((y & m) << j);
+    }
+    return x;
+}
+
 template <int K, bool PK>
 struct SkbShared {
     uint4 wt[(K + 3) / 4][256];
@@ -269,7 +282,13 @@ constexpr int skb_ctas() {
     return 3 * (sizeof(SkbShared<K, PK>) + 1024) <= 228 * 1024 ? 3 : 2;
 }
 
-template <int K, bool PK>
+// ORD: the k-mers of a warp's tiles in sequence order, counted in
+// a.ord_cnt[warp] and written (as many as there is room for) from
+// a.ord_off[warp] to a.ord_off[warp + 1], or with no ord_off from warp *
+// a.ord_stride; a.ord_seq_cnt[q] (unless null) counts those of sequence q. The
+// candidate masks are transposed first, so that lane i holds sub-run i's and
+// the queue fills in order.
+template <int K, bool PK, bool ORD>
 __global__ void __launch_bounds__(SKB_WARPS * 32, skb_ctas<K, PK>()) k_sketch_bits(SketchArgs a,
                                                                           const SketchTabs* __restrict__ tabs) {
     constexpr int NG = (K + 3) / 4;
@@ -302,7 +321,17 @@ __global__ void __launch_bounds__(SKB_WARPS * 32, skb_ctas<K, PK>()) k_sketch_bi
     int32_t q_tile = warp_last_le((const uint64_t*)a.seq_off, a.n_seq, (uint64_t)min(max(base, lo), hi), lane);
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (!any) return;
+    if (!any) {
+        if (ORD && lane == 0) a.ord_cnt[gw] = 0;
+        return;
+    }
+    // ORD: where the warp's k-mers go, and how many there were so far
+    uint64_t ord_base = 0;
+    uint32_t ord_cap = 0, ord_n = 0;
+    if (ORD) {
+        ord_base = a.ord_off ? (uint64_t)a.ord_off[gw] : (uint64_t)gw * a.ord_stride;
+        ord_cap = a.ord_off ? a.ord_off[gw + 1] - a.ord_off[gw] : a.ord_stride;
+    }
     int32_t q_queue = q_tile;  // no queued candidate's read comes before it
     uint32_t qn = 0;
 
@@ -343,6 +372,17 @@ __global__ void __launch_bounds__(SKB_WARPS * 32, skb_ctas<K, PK>()) k_sketch_bi
         }
         const unsigned peers = __match_any_sync(FULL, sel ? q : -1);
         const int leader = __ffs(peers) - 1;
+        if (ORD) {
+            const unsigned bal = __ballot_sync(FULL, sel);
+            const uint32_t slot = ord_n + __popc(bal & ((1u << lane) - 1u));
+            if (sel && slot < ord_cap) {
+                a.out_h[ord_base + slot] = h;
+                a.out_rs[ord_base + slot] = rs;
+            }
+            if (sel && lane == leader && a.ord_seq_cnt) atomicAdd(a.ord_seq_cnt + q, (uint32_t)__popc(peers));
+            ord_n += __popc(bal);
+            return;
+        }
         uint32_t at = 0;
         if (sel && lane == leader) at = atomicAdd(a.kmer_cnt + q, (uint32_t)__popc(peers));
         at = __shfl_sync(FULL, at, leader) + __popc(peers & ((1u << lane) - 1u));
@@ -431,35 +471,63 @@ __global__ void __launch_bounds__(SKB_WARPS * 32, skb_ctas<K, PK>()) k_sketch_bi
         if (tl + 1 < t_end) src.fetch(buf, t0 + SKB_TILE - SKB_LEAD, lane);
         uint32_t le[4] = {0u, 0u, 0u, 0u};
         if (__any_sync(FULL, bad != 0)) {
-            // a lane rolls sub-run `lane` through the byte tables
-            const int64_t s0 = t0 + SKB_S * lane;
-            uint64_t f = 0, r = 0;
-            for (int i = 0; i < K; i++) {
-                const uint32_t c = src.letter(s0 + i);
-                f = rotl64(f, 1) ^ __ldg(&tabs->luts.fw[c]);
-                r = rotr64(r, 1) ^ __ldg(&tabs->luts.rc_k1[c]);
-            }
-            int32_t q = q_tile;
-            for (int t = 0; t < SKB_S; t++) {
-                const int64_t p = s0 + t;
-                const uint64_t h = f ^ r;
-                if (h <= thr && p >= lo && p < hi) {
-                    while (__ldg(a.seq_off + q + 1) <= p) q++;  // ends: p < hi = seq_off[n_seq]
-                    if (p + K <= __ldg(a.seq_off + q + 1)) {
-                        const uint64_t o = __ldg(a.kmer_off + q);
-                        const uint32_t at = atomicAdd(a.kmer_cnt + q, 1u);
-                        if (at < (uint32_t)(__ldg(a.kmer_off + q + 1) - o)) {
-                            a.out_h[o + at] = h;
-                            a.out_rs[o + at] =
-                                ((uint32_t)((int32_t)(p - __ldg(a.seq_off + q)) + K - 1 + a.r_offset) << 1) |
-                                (f > r ? 1u : 0u);
-                        }
-                    }
+            // a lane rolls sub-run `lane` through the byte tables; take_one gets
+            // each selected window's sequence, hash and r << 1 | strand
+            auto roll = [&](auto&& take_one) {
+                const int64_t s0 = t0 + SKB_S * lane;
+                uint64_t f = 0, r = 0;
+                for (int i = 0; i < K; i++) {
+                    const uint32_t c = src.letter(s0 + i);
+                    f = rotl64(f, 1) ^ __ldg(&tabs->luts.fw[c]);
+                    r = rotr64(r, 1) ^ __ldg(&tabs->luts.rc_k1[c]);
                 }
-                const uint32_t ci = src.letter(p + K), co = src.letter(p);
-                f = rotl64(f, 1) ^ __ldg(&tabs->luts.fw_k[co]) ^ __ldg(&tabs->luts.fw[ci]);
-                r = rotr64(r, 1) ^ __ldg(&tabs->luts.rc_r1[co]) ^ __ldg(&tabs->luts.rc_k1[ci]);
+                int32_t q = q_tile;
+                for (int t = 0; t < SKB_S; t++) {
+                    const int64_t p = s0 + t;
+                    const uint64_t h = f ^ r;
+                    if (h <= thr && p >= lo && p < hi) {
+                        while (__ldg(a.seq_off + q + 1) <= p) q++;  // ends: p < hi = seq_off[n_seq]
+                        if (p + K <= __ldg(a.seq_off + q + 1))
+                            take_one(q, h, ((uint32_t)((int32_t)(p - __ldg(a.seq_off + q)) + K - 1 + a.r_offset) << 1) |
+                                               (f > r ? 1u : 0u));
+                    }
+                    const uint32_t ci = src.letter(p + K), co = src.letter(p);
+                    f = rotl64(f, 1) ^ __ldg(&tabs->luts.fw_k[co]) ^ __ldg(&tabs->luts.fw[ci]);
+                    r = rotr64(r, 1) ^ __ldg(&tabs->luts.rc_r1[co]) ^ __ldg(&tabs->luts.rc_k1[ci]);
+                }
+            };
+            if (ORD) {
+                if (qn) take(0, qn);  // the tiles before come first
+                qn = 0;
+                __syncwarp();
+                uint32_t mine = 0;
+                roll([&](int32_t q, uint64_t, uint32_t) {
+                    mine++;
+                    if (a.ord_seq_cnt) atomicAdd(a.ord_seq_cnt + q, 1u);
+                });
+                __syncwarp();
+                const uint32_t inc = warp_inclusive_scan(mine);
+                uint32_t slot = ord_n + inc - mine;
+                ord_n += __shfl_sync(FULL, inc, 31);
+                if (ord_cap)
+                    roll([&](int32_t, uint64_t h, uint32_t rs) {
+                        if (slot < ord_cap) {
+                            a.out_h[ord_base + slot] = h;
+                            a.out_rs[ord_base + slot] = rs;
+                        }
+                        slot++;
+                    });
+            } else {
+                roll([&](int32_t q, uint64_t h, uint32_t rs) {
+                    const uint64_t o = __ldg(a.kmer_off + q);
+                    const uint32_t at = atomicAdd(a.kmer_cnt + q, 1u);
+                    if (at < (uint32_t)(__ldg(a.kmer_off + q + 1) - o)) {
+                        a.out_h[o + at] = h;
+                        a.out_rs[o + at] = rs;
+                    }
+                });
             }
+            __syncwarp();
         } else {
             uint32_t o0[4], o1[4];
             transpose4(y0, o0);
@@ -483,17 +551,35 @@ __global__ void __launch_bounds__(SKB_WARPS * 32, skb_ctas<K, PK>()) k_sketch_bi
         }
         // the candidates to the queue; full rounds of 32 are taken at once, the
         // rest with the next tile's (or now, after the last tile)
-        const uint32_t rel0 = (uint32_t)(t0 - base) + 4u * (uint32_t)lane - (uint32_t)SKB_LEAD;
+        const uint32_t rel0 =
+            (uint32_t)(t0 - base) - (uint32_t)SKB_LEAD + (ORD ? (uint32_t)SKB_S : 4u) * (uint32_t)lane;
+        if (ORD) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) le[q] = transpose32(le[q], lane);
+        }
         for (bool more = true; more;) {
             const uint32_t cnt = __popc(le[0]) + __popc(le[1]) + __popc(le[2]) + __popc(le[3]);
             const uint32_t inc = warp_inclusive_scan(cnt), total = __shfl_sync(FULL, inc, 31);
             uint32_t at = qn + inc - cnt;
+            if (ORD) {
+                for (uint32_t l; (l = le[0] | le[1] | le[2] | le[3]) != 0 && at < (uint32_t)SKB_Q;) {
+                    const uint32_t bit = l & (0u - l);
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                while (le[q] != 0 && at < (uint32_t)SKB_Q) {
-                    queue[at++] = rel0 + (uint32_t)q + (uint32_t)SKB_S * (uint32_t)(__ffs(le[q]) - 1);
-                    le[q] &= le[q] - 1;
+                    for (int q = 0; q < 4; q++)
+                        if ((le[q] & bit) && at < (uint32_t)SKB_Q) {
+                            queue[at++] = rel0 + 4u * (uint32_t)(__ffs(bit) - 1) + (uint32_t)q;
+                            le[q] &= ~bit;
+                        }
                 }
+            }
+            if (!ORD) {
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    while (le[q] != 0 && at < (uint32_t)SKB_Q) {
+                        queue[at++] = rel0 + (uint32_t)q + (uint32_t)SKB_S * (uint32_t)(__ffs(le[q]) - 1);
+                        le[q] &= le[q] - 1;
+                    }
+            }
             more = qn + total > (uint32_t)SKB_Q;
             const uint32_t have = min(qn + total, (uint32_t)SKB_Q);
             const uint32_t upto = !more && tl + 1 == t_end ? have : have & ~31u;
@@ -510,6 +596,7 @@ __global__ void __launch_bounds__(SKB_WARPS * 32, skb_ctas<K, PK>()) k_sketch_bi
             __syncwarp();
         }
     }
+    if (ORD && lane == 0) a.ord_cnt[gw] = ord_n;
 }
 
 }  // namespace shm

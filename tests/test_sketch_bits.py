@@ -70,3 +70,31 @@ def test_any_first_base(gpu_ctx, lead):
         got = _at_offset(reads, lead, 25, 0.05, packed)
         for i, x in enumerate(reads):
             assert all(np.array_equal(a, b) for a, b in zip(got[i], O.sketch(x, 25, 0.05))), (packed, i)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [14, 15, 25, 28, 32, 33])
+@pytest.mark.parametrize("r", [1.0, 0.1, 0.01])
+def test_ordered_edges(gpu_ctx, k, r):
+    """One sequence's sketch and an index's segments, in order: at tile edges,
+    with masked bases, with segments shorter than k, and with far more k-mers
+    than a random sequence of the length would have."""
+    rng = np.random.default_rng(k)
+
+    def dna(n):
+        return np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, n)].tobytes()
+
+    masked = bytearray(dna(4 * TILE))
+    masked[TILE + 119] = ord("N")
+    masked[2 * TILE - 1:2 * TILE + 1] = b"nR"
+    masked[3 * TILE:] = b"N" * TILE
+    rich = next(u for u in (dna(40) for _ in range(400)) if len(O.sketch(u * 3, k, 0.01)[0]) > 3)  # selected once a copy
+    seqs = [dna(n) for n in (k, 120 + k - 1, TILE, TILE + k, 7 * TILE + 5)] + [bytes(masked), (rich * 2000)[:70001]]
+    for x in seqs:
+        got, want = gpu_ctx.sketch(x, k, r, 7), O.sketch(x, k, r, 7)
+        assert all(np.array_equal(a, b) for a, b in zip(got, want)), len(x)
+    recs = [(f"s{i}", x) for i, x in enumerate([dna(3), *seqs, b"", dna(k - 1), dna(2 * TILE + 1)])]
+    idx = sb.SketchIndex.from_records(gpu_ctx, recs, k, r)
+    for i, (_, x) in enumerate(recs):
+        assert all(np.array_equal(a, b) for a, b in zip(idx.segment(i)[:3], O.sketch(x, k, r))), i
+    idx.close()
