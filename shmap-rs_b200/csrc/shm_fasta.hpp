@@ -15,7 +15,7 @@ namespace shm {
 struct FastaDev {
     int device = 0;
     int32_t n = 0;
-    DevBuf<uint8_t> seq;         // every record's bases back to back, 32 zero bytes past the end
+    PoolBuf<uint8_t> seq;        // every record's bases back to back, 32 zero bytes past the end
     std::vector<int64_t> offs;   // n+1: record i is seq[offs[i], offs[i+1])
     std::string names;           // '\n'-joined record names
     DevBuf<shm_map_record> rec;  // records of the reads mapped from it

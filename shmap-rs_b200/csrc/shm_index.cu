@@ -88,9 +88,19 @@ __global__ void k_key_keep(const uint32_t* __restrict__ key_off, uint32_t n_keys
         keep[j] = kept ? 1u : 0u;
         keep_hits[j] = kept ? len : 0u;
     }
+    // a warp's sums first: every thread of the grid on the same four words took
+    // 0.6 ms for 1.5 million keys
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ih += __shfl_xor_sync(0xffffffffu, ih, o);
+        bk += __shfl_xor_sync(0xffffffffu, bk, o);
+        bh += __shfl_xor_sync(0xffffffffu, bh, o);
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if ((threadIdx.x & 31) != 0 || ih == 0) return;
     atomicAdd(&st->indexed_hits, ih);
-    atomicAdd(&st->blacklisted_kmers, bk);
-    atomicAdd(&st->blacklisted_hits, bh);
+    if (bk) atomicAdd(&st->blacklisted_kmers, bk);
+    if (bh) atomicAdd(&st->blacklisted_hits, bh);
     atomicMax(&st->highest, hi);
 }
 
