@@ -199,7 +199,7 @@ int shm_sketch(shm_ctx* ctx, const uint8_t* seq, int64_t len, int32_t k, double 
     shm::TmpBuf<uint32_t> d_cnt, d_out, d_rs;
     d_seq.reserve((size_t)len + 32, s);
     SHM_CUDA(cudaMemsetAsync(d_seq.p + len, 0, 32, s));
-    SHM_CUDA(cudaMemcpyAsync(d_seq.p, seq, (size_t)len, cudaMemcpyHostToDevice, s));
+    shm::upload(ctx->m->up, ctx->m->device, d_seq.p, seq, (size_t)len, s);
     const int64_t off[2] = {0, len};
     d_off.reserve(2, s);
     SHM_CUDA(cudaMemcpyAsync(d_off.p, off, sizeof off, cudaMemcpyHostToDevice, s));
@@ -290,7 +290,7 @@ int shm_index_build(shm_ctx* ctx, const uint8_t* seq, const int64_t* seg_off, in
     SHM_CUDA(cudaSetDevice(ctx->m->device));
     auto* ix = new shm_index();
     ix->s = shm::build_index(seq, seg_off, n_seg, split_names(names, n_seg), k, h_frac, max_matches,
-                             shm::ctx_luts(ctx->m, k), ctx->m->stream);
+                             shm::ctx_luts(ctx->m, k), ctx->m->up, ctx->m->stream);
     ctx->m->launches += 40;
     *out = ix;
     return SHM_OK;
@@ -320,7 +320,7 @@ int shm_fasta_parse_device(shm_ctx* ctx, const uint8_t* file, int64_t len, shm_f
     *out = nullptr;
     SHM_GUARD_BEGIN
     std::string why;
-    shm::FastaDev* f = shm::fasta_parse_device(ctx->m->device, ctx->m->stream, file, len, &why);
+    shm::FastaDev* f = shm::fasta_parse_device(ctx->m->device, ctx->m->stream, ctx->m->up, file, len, &why);
     if (!f) return fail(SHM_ERR_INVALID, "not parsed on the device: " + why);
     auto* h = new shm_fasta();
     h->f = f;
@@ -365,7 +365,8 @@ int shm_index_build_fasta(shm_ctx* ctx, const shm_fasta* fa, int32_t k, double h
     SHM_CUDA(cudaSetDevice(ctx->m->device));
     auto* ix = new shm_index();
     ix->s = shm::build_index(nullptr, fa->f->offs.data(), fa->f->n, split_names(fa->f->names.c_str(), fa->f->n), k,
-                             h_frac, max_matches, shm::ctx_luts(ctx->m, k), ctx->m->stream, fa->f->seq.p);
+                             h_frac, max_matches, shm::ctx_luts(ctx->m, k), ctx->m->up, ctx->m->stream,
+                             fa->f->seq.p);
     ctx->m->launches += 40;
     *out = ix;
     return SHM_OK;

@@ -480,7 +480,8 @@ __global__ void k_fa_name_write(FaView v, const int64_t* __restrict__ hdr_pos, i
 
 }  // namespace
 
-FastaDev* fasta_parse_device(int device, cudaStream_t s, const uint8_t* file, int64_t len, std::string* why) {
+FastaDev* fasta_parse_device(int device, cudaStream_t s, UploadStage* up, const uint8_t* file, int64_t len,
+                             std::string* why) {
     SHM_CUDA(cudaSetDevice(device));
     auto* F = new FastaDev();
     try {
@@ -492,7 +493,7 @@ FastaDev* fasta_parse_device(int device, cudaStream_t s, const uint8_t* file, in
             while (len > 0 && (file[len - 1] == '\n' || file[len - 1] == '\r')) len--;
         TmpBuf<uint8_t> raw;
         raw.reserve(((size_t)len + 64) / 64 * 64 + 64, s);
-        if (len) SHM_CUDA(cudaMemcpyAsync(raw.p, file, (size_t)len, cudaMemcpyHostToDevice, s));
+        upload(up, device, raw.p, file, (size_t)len, s);
         v.d = raw.p;
         v.len = len;
         v.n_chunks = (len + CHUNK - 1) / CHUNK;

@@ -25,6 +25,6 @@ struct FastaDev {
 // the first byte is '@'. Returns null, with the reason in *why, for files the
 // host reader handles instead: a FASTA file with a line starting with '@' or
 // text before the first header, a FASTQ file not made of four-line records.
-FastaDev* fasta_parse_device(int device, cudaStream_t s, const uint8_t* file, int64_t len, std::string* why);
+FastaDev* fasta_parse_device(int device, cudaStream_t s, UploadStage* up, const uint8_t* file, int64_t len, std::string* why);
 
 }  // namespace shm

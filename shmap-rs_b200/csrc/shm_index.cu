@@ -249,7 +249,7 @@ static void finish_index(IndexStorage* ix, uint64_t thr, uint32_t n_kept, uint32
 
 IndexStorage* build_index(const uint8_t* h_seq, const int64_t* seg_off_b, int32_t n_seg,
                           const std::vector<std::string>& names, int32_t k, double h_frac, int32_t max_matches,
-                          const SketchLuts* luts, cudaStream_t s, const uint8_t* d_seq_in) {
+                          const SketchLuts* luts, UploadStage* up, cudaStream_t s, const uint8_t* d_seq_in) {
     auto* ix = new IndexStorage();
     try {
         SHM_CUDA(cudaGetDevice(&ix->device));
@@ -277,8 +277,7 @@ IndexStorage* build_index(const uint8_t* h_seq, const int64_t* seg_off_b, int32_
         if (!d_seq_in) {
             d_seq.reserve((size_t)total_bases + 32, s);
             SHM_CUDA(cudaMemsetAsync(d_seq.p + total_bases, 0, 32, s));
-            if (total_bases)
-                SHM_CUDA(cudaMemcpyAsync(d_seq.p, h_seq + seg_off_b[0], (size_t)total_bases, cudaMemcpyHostToDevice, s));
+            if (total_bases) upload(up, ix->device, d_seq.p, h_seq + seg_off_b[0], (size_t)total_bases, s);
         }
         d_soff.reserve((size_t)n_seg + 1, s);
         SHM_CUDA(cudaMemcpyAsync(d_soff.p, soff.data(), sizeof(int64_t) * ((size_t)n_seg + 1), cudaMemcpyHostToDevice, s));

@@ -3399,6 +3399,7 @@ MapCtx* mapctx_create(int device, size_t hbm_budget) {
     for (auto& e : c->raw_copied) SHM_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (auto& e : c->raw_sketched) SHM_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     c->scr = new MapScratch();
+    c->up = upload_stage_create();
     return c;
 }
 
@@ -3413,6 +3414,7 @@ void mapctx_destroy(MapCtx* c) {
     paf_scratch_free(c->paf);
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
     if (c->h_slots) cudaFreeHost(c->h_slots);
+    upload_stage_destroy(c->up);
     if (c->h_pack) cudaFreeHost(c->h_pack);
     if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
     for (auto& e : c->copied)

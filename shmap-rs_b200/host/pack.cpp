@@ -392,6 +392,12 @@ void pack_reads_host(const uint8_t* seq, int64_t nb, uint32_t* codes, uint32_t* 
     if (own) g_pack_mu.unlock();
 }
 
+void host_tasks(int n, std::function<void(int)> f) {
+    std::unique_lock<std::mutex> g(g_pack_mu, std::defer_lock);
+    if (!t_pack_held) g.lock();
+    pool().run(n, std::move(f));
+}
+
 void pack_reads_host_start(const uint8_t* seq, int64_t nb, uint32_t* codes, int64_t task_groups) {
     if (!t_pack_held) {
         g_pack_mu.lock();

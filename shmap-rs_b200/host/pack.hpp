@@ -2,6 +2,7 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
+#include <functional>
 
 namespace shm {
 
@@ -34,6 +35,9 @@ struct PackSink {
     virtual bool piece_raw(int worker, const uint8_t* src, size_t first_group, size_t groups) { return false; }
     virtual ~PackSink() = default;
 };
+// Calls f(task) for the tasks 0 .. n - 1 on the packing threads and the
+// caller's (f must not throw), taking its turn among the packings.
+void host_tasks(int n, std::function<void(int)> f);
 // The number of packing threads (the pool's and the one holding the packing).
 int pack_workers();
 

@@ -408,16 +408,16 @@ class SketchIndex:
         cp = params.c()
         need = ctypes.c_int64()
         cap = 640 * n + len(joined) + 1  # a line is about 480 bytes plus its names
-        buf = ctypes.create_string_buffer(cap)
+        buf = np.empty(cap, np.uint8)
         rc = lib().shm_map_paf(self.ctx.h, self.h, ctypes.byref(cp), _ptr(seq), _ptr(offs), n, joined,
-                               0 if out is None else _ptr(out), buf, cap, ctypes.byref(need))
+                               0 if out is None else _ptr(out), _ptr(buf), cap, ctypes.byref(need))
         if rc == SHM_ERR_CAPACITY:
             cap = need.value + 1
-            buf = ctypes.create_string_buffer(cap)
+            buf = np.empty(cap, np.uint8)
             rc = lib().shm_map_paf(self.ctx.h, self.h, ctypes.byref(cp), _ptr(seq), _ptr(offs), n, joined,
-                                   0 if out is None else _ptr(out), buf, cap, ctypes.byref(need))
+                                   0 if out is None else _ptr(out), _ptr(buf), cap, ctypes.byref(need))
         _check(rc)
-        return ctypes.string_at(buf, need.value).decode(), out
+        return str(memoryview(buf)[:need.value], "utf-8"), out
 
     def format_paf(self, params: Params, records: np.ndarray, names: Sequence[str],
                    map_time: Optional[np.ndarray] = None) -> str:
