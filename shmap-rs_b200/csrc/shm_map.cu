@@ -1652,51 +1652,86 @@ __global__ void __launch_bounds__(256) k_bt_second(BatchView v) {
 }
 
 // ------------------------------------------------------------------ K4 distinct buckets
-__global__ void __launch_bounds__(256) k_bscan(BatchView v) {
-    const int lane = threadIdx.x & 31;
-    const int32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int32_t q = wid; q < v.n; q += nwarps) {
-        const uint32_t nb = v.r_seeded[q];
-        if (v.r_flags[q]) {  // its capped bucket table filled up, or lay past the pool: mapped again
-            if (lane == 0) v.r_status[q] = ST_OVERFLOW;
-            continue;
-        }
-        if (nb == 0) continue;
-        const uint64_t base = v.bt_tab[q].x;
-        if (lane == 0) atomicAdd(&v.mx->buckets, (unsigned long long)nb);
-        for (uint32_t j = lane; j < nb; j += 32) {
-            const BSlot s = v.bt[base + v.bt_list[base + j]];
-            BucketJob jb;
-            jb.read = q;
-            jb.seg = (int32_t)(s.key >> 32);
-            jb.bb = (int32_t)(s.key & 0xffffffffu);
-            int32_t s_matches, s_codir;
-            bt_unpack(s.mc, s_matches, s_codir);
-            jb.m0 = s_matches;
-            jb.matches = s_matches;
-            jb.codir = s_codir;
-            jb.rmin = s.rmin;
-            jb.rmax = s.rmax;
-            jb.pad0 = jb.pad1 = 0;
-            jb.score = -1.0;
-            jb.support = 0.0;
-            jb.t_l = jb.t_r = jb.inter = jb.same = jb.s_sz = -1;
-            if (v.P.nbp) {
-                jb.sh = 1.0;  // seed_heuristic_pass does nothing under NBP (pruning.rs:351)
-                jb.is_cand = 1;
-            } else {
-                const double sh0 = hseed(v.r_m[q], v.r_S0[q], s_matches);
-                if (sh0 < v.P.theta_low) continue;
-                jb.sh = sh0;
-                jb.is_cand = 0;
+// A warp a read, a CTA's reads in step: the jobs of their first 32 buckets
+// are counted in shared memory and numbered by one counter update a CTA. With
+// an update a read every warp waited for its turn at the counter's cache
+// line: 0.42 ms for 150,000 reads, 0.21 so.
+constexpr int BSCAN_WARPS = 8;
+__global__ void __launch_bounds__(BSCAN_WARPS * 32) k_bscan(BatchView v) {
+    __shared__ uint32_t s_cnt[2][BSCAN_WARPS], s_base[2];
+    __shared__ unsigned long long s_buckets;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_buckets = 0;
+    __syncthreads();
+    int par = 0;
+    for (int32_t q0 = (int32_t)blockIdx.x * BSCAN_WARPS; q0 < v.n; q0 += (int32_t)gridDim.x * BSCAN_WARPS, par ^= 1) {
+        const int32_t q = q0 + wib;
+        uint32_t nb = 0;
+        uint64_t base = 0;
+        if (q < v.n) {
+            nb = v.r_seeded[q];
+            if (v.r_flags[q]) {  // its capped bucket table filled up, or lay past the pool: mapped again
+                if (lane == 0) v.r_status[q] = ST_OVERFLOW;
+                nb = 0;
             }
-            uint32_t ji = atomicAdd(v.n_jobs, 1u);
-            if (ji < v.job_cap) {
+            if (nb) {
+                base = v.bt_tab[q].x;
+                if (lane == 0) atomicAdd(&s_buckets, (unsigned long long)nb);
+            }
+        }
+        for (uint32_t j0 = 0; j0 == 0 || j0 < nb; j0 += 32) {
+            const uint32_t j = j0 + (uint32_t)lane;
+            bool pass = false;
+            BSlot s{};
+            double sh0 = 1.0;  // seed_heuristic_pass does nothing under NBP (pruning.rs:351)
+            int32_t s_matches = 0, s_codir = 0;
+            if (j < nb) {
+                s = v.bt[base + v.bt_list[base + j]];
+                bt_unpack(s.mc, s_matches, s_codir);
+                if (!v.P.nbp) sh0 = hseed(v.r_m[q], v.r_S0[q], s_matches);
+                pass = v.P.nbp || !(sh0 < v.P.theta_low);
+            }
+            const unsigned mask = __ballot_sync(0xffffffffu, pass);
+            uint32_t first = 0;
+            if (j0 == 0) {
+                if (lane == 0) s_cnt[par][wib] = (uint32_t)__popc(mask);
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    uint32_t t = 0;
+                    for (int w = 0; w < BSCAN_WARPS; w++) t += s_cnt[par][w];
+                    s_base[par] = t ? atomicAdd(v.n_jobs, t) : 0u;
+                }
+                __syncthreads();
+                first = s_base[par];
+                for (int w = 0; w < wib; w++) first += s_cnt[par][w];
+            } else if (mask) {
+                if (lane == 0) first = atomicAdd(v.n_jobs, (uint32_t)__popc(mask));
+                first = __shfl_sync(0xffffffffu, first, 0);
+            }
+            const uint32_t ji = first + (uint32_t)__popc(mask & ((1u << lane) - 1u));
+            if (pass && ji < v.job_cap) {
+                BucketJob jb;
+                jb.read = q;
+                jb.seg = (int32_t)(s.key >> 32);
+                jb.bb = (int32_t)(s.key & 0xffffffffu);
+                jb.m0 = s_matches;
+                jb.matches = s_matches;
+                jb.codir = s_codir;
+                jb.rmin = s.rmin;
+                jb.rmax = s.rmax;
+                jb.pad0 = jb.pad1 = 0;
+                jb.score = -1.0;
+                jb.support = 0.0;
+                jb.t_l = jb.t_r = jb.inter = jb.same = jb.s_sz = -1;
+                jb.sh = sh0;
+                jb.is_cand = v.P.nbp ? 1 : 0;
                 v.jobs[ji] = jb;
                 if (jb.is_cand) atomicAdd(v.ccnt + q, 1u);
             }
         }
     }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_buckets) atomicAdd(&v.mx->buckets, s_buckets);
 }
 
 // ------------------------------------------------------------------ K5 extension
