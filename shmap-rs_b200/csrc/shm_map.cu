@@ -1367,35 +1367,65 @@ __device__ __forceinline__ void bt_unpack(unsigned long long mc, int32_t& matche
     matches = (int32_t)((mc - (unsigned long long)(long long)codir) >> 32);
 }
 
-__device__ __forceinline__ void bt_add(const BatchView& v, int32_t q, int32_t seg, int64_t bb, int32_t matches,
-                                       int32_t codir, int32_t rmin, int32_t rmax) {
-    if (v.r_flags[q]) return;  // the read is mapped again, or given a second table first
-    const ulonglong2 tb = v.bt_tab[q];
-    const uint64_t base = tb.x, mask = tb.y;
-    const unsigned long long key = ((unsigned long long)(uint32_t)seg << 32) | (uint32_t)bb;
-    uint64_t i = mix64(key) & mask;
-    BSlot* s;
-    for (uint64_t probe = 0;; probe++) {
-        if (probe > mask) {  // every slot taken by other buckets
+struct BtTab {  // a read's bucket table
+    uint64_t base, mask;
+};
+
+// A slot's key as this SM last saw it. A key is written once, in place of
+// EMPTY_KEY, so one that was seen stays right; EMPTY_KEY may be out of date.
+__device__ __forceinline__ unsigned long long bt_key(const BSlot* s) {
+    unsigned long long k;
+    asm volatile("ld.global.ca.u64 %0, [%1];" : "=l"(k) : "l"(&s->key));
+    return k;
+}
+// Neighbouring buckets of a segment start at different slots.
+__device__ __forceinline__ uint64_t bt_hash(int32_t seg, uint32_t bb, uint64_t mask) {
+    const uint32_t x = bb * 0x9E3779B1u + (uint32_t)seg * 0x85EBCA6Bu;
+    return (uint64_t)(x ^ (x >> 16)) & mask;
+}
+
+// Adds to bucket (seg, bb) from slot i on, whose key was seen as k. Only a
+// new bucket costs a compare-and-swap: its round trip to the L2 for every
+// addition was what the contributions waited for (150,000 hifi reads: 1.79 ms
+// so, 1.36 with the key read first and the next hit loaded ahead).
+__device__ __forceinline__ void bt_add(const BatchView& v, int32_t q, const BtTab& tb, int32_t seg, uint32_t bb,
+                                       uint64_t i, unsigned long long k, int32_t matches, int32_t codir,
+                                       int32_t rmin, int32_t rmax) {
+    const unsigned long long key = ((unsigned long long)(uint32_t)seg << 32) | bb;
+    BSlot* s = v.bt + tb.base + i;
+    for (uint64_t probe = 1; k != key; probe++) {
+        if (k == EMPTY_KEY) {
+            k = atomicCAS(&s->key, EMPTY_KEY, key);
+            if (k == EMPTY_KEY) {  // a new bucket: list it for k_bscan (seeded_buckets, mod.rs:794)
+                const uint32_t at = atomicAdd(v.r_seeded + q, 1u);  // < slots: every listed bucket holds a slot
+                v.bt_list[tb.base + at] = (uint32_t)i;
+                if ((uint64_t)at + 1 > ((tb.mask + 1) >> 1) + ((tb.mask + 1) >> 2))
+                    atomicOr(v.r_flags + q, 1u);  // load > 3/4
+                break;
+            }
+            if (k == key) break;
+        }
+        if (probe > tb.mask) {  // every slot taken by other buckets
             atomicOr(v.r_flags + q, 1u);
             return;
         }
-        s = v.bt + base + i;
-        unsigned long long prev = atomicCAS(&s->key, EMPTY_KEY, key);
-        if (prev == EMPTY_KEY) {  // a new bucket: list it for k_bscan (seeded_buckets, mod.rs:794)
-            const uint32_t at = atomicAdd(v.r_seeded + q, 1u);  // < slots: every listed bucket holds a slot
-            v.bt_list[base + at] = (uint32_t)i;
-            if ((uint64_t)at + 1 > ((mask + 1) >> 1) + ((mask + 1) >> 2)) atomicOr(v.r_flags + q, 1u);  // load > 3/4
-            break;
-        }
-        if (prev == key) break;
-        i = (i + 1) & mask;
+        // a table that fills up is given up: the read is mapped again, or given a second one
+        if ((probe & 3) == 0 && __ldcg(v.r_flags + q)) return;
+        i = (i + 1) & tb.mask;
+        s = v.bt + tb.base + i;
+        k = bt_key(s);
     }
     atomicAdd(&s->mc, bt_pack(matches, codir));
     if (bucket_metric(v.P)) {  // the position range is read by the bucket metrics only
         atomicMin(&s->rmin, rmin);
         atomicMax(&s->rmax, rmax);
     }
+}
+
+// floor(x / h) with inv = 0xffffffff / h: the product falls short by one at most.
+__device__ __forceinline__ uint32_t div_by(uint32_t x, uint32_t h, uint32_t inv) {
+    const uint32_t d = __umulhi(x, inv);
+    return d + (x - d * h >= h ? 1u : 0u);
 }
 
 __device__ __forceinline__ uint32_t ub_u64(const uint64_t* a, uint32_t n, uint64_t x) {  // first index with a[i] > x
@@ -1429,11 +1459,17 @@ __device__ __forceinline__ uint32_t ub_u32(const uint32_t* a, uint32_t n, uint32
 // and seed come from two binary searches, the rest by stepping through the
 // seed's hit list (sorted by gidx) and on to the next seed or read. The
 // previous hit's bucket and the current segment's bounds are carried along.
-// A run is CONTRIB_RUN words, fewer while there is not a run for every thread
-// of the grid (a run's hits are one dependent chain after the other).
+// A run is CONTRIB_RUN words where seeds have several hits each, so that the
+// searches at its start are shared by more of them, and half as many else,
+// where each word is a seed's own chain of loads (12,500 reads of repeats, 8.7
+// hits a seed: 4.83 ms with runs of 8, 5.14 of 4; 30,000 ONT-like reads, 1.0
+// hits a seed: 0.57 and 0.52). Fewer while there is not a run for every thread
+// of the grid. Bound by the latency of those loads at the 32 warps an SM that
+// the registers allow (40 warps with 48 registers take as long).
 constexpr int CONTRIB_RUN = 8;
-__device__ __forceinline__ uint32_t contrib_run(uint64_t total) {
-    return (uint32_t)min((uint64_t)CONTRIB_RUN, max((uint64_t)1, total / ((uint64_t)gridDim.x * blockDim.x)));
+__device__ __forceinline__ uint32_t contrib_run(const BatchView& v, uint64_t total) {
+    const uint32_t most = total >= 4 * v.mx->proc_seeds ? CONTRIB_RUN : CONTRIB_RUN / 2;
+    return (uint32_t)min((uint64_t)most, max((uint64_t)1, total / ((uint64_t)gridDim.x * blockDim.x)));
 }
 
 __device__ __forceinline__ int32_t seg_step(const DevIndex& I, uint32_t g, int32_t seg, uint32_t& s_lo,
@@ -1453,11 +1489,15 @@ __device__ __forceinline__ void contrib_span(const BatchView& v, uint64_t w, con
     const DevIndex& I = v.I;
     uint64_t kb = v.kcap_off[q];
     uint32_t np = (uint32_t)v.r_nproc[q];
-    uint32_t h = (uint32_t)v.r_half[q];
+    uint32_t h = (uint32_t)v.r_half[q], inv = 0xffffffffu / h;
+    bool dead = v.r_flags[q] != 0;  // the read is mapped again, or given a second table first
+    BtTab tb{v.bt_tab[q].x, v.bt_tab[q].y};
     uint32_t j = ub_u32(v.sd_hpre + kb, np, (uint32_t)(w - v.hw_off[q])) - 1;
     uint32_t t = (uint32_t)(w - v.hw_off[q]) - v.sd_hpre[kb + j];
     SeedRec sr = v.sd[kb + j];
     uint32_t a = sr.a, cnt = sr.cnt, os = sr.os;
+    uint32_t g_t = __ldg(I.hits + a + t);
+    SeedRec nx = v.sd[kb + min(j + 1, np - 1)];  // the seed after it
     int32_t seg = -1;
     uint32_t s_lo = 0, s_hi = 0;
     int32_t seg_p = -1;  // bucket of the seed's previous hit (seg_p < 0: none)
@@ -1465,91 +1505,112 @@ __device__ __forceinline__ void contrib_span(const BatchView& v, uint64_t w, con
     if (t > 0) {
         const uint32_t g_p = __ldg(I.hits + a + t - 1);
         seg_p = seg = seg_step(I, g_p, seg, s_lo, s_hi);
-        b_p = (ap ? (__ldg(I.ref_rs + g_p) >> 1) : g_p - s_lo) / h;
+        b_p = div_by(ap ? (__ldg(I.ref_rs + g_p) >> 1) : g_p - s_lo, h, inv);
     }
     for (;;) {
+        // the next hit is on its way while this one's buckets are updated (the
+        // processed seeds after one with hits all have some)
+        const bool in_seed = t + 1 < cnt, in_read = in_seed || j + 1 < np;
+        uint32_t g_n = 0;
+        if (in_read && w + 1 < wend) g_n = __ldg(I.hits + (in_seed ? a + t + 1 : nx.a));
         const uint32_t occs = os >> 1, sstr = os & 1u;
-        const uint32_t g_t = __ldg(I.hits + a + t);
         seg = seg_step(I, g_t, seg, s_lo, s_hi);
-        const uint32_t b_t = (ap ? (__ldg(I.ref_rs + g_t) >> 1) : g_t - s_lo) / h;
+        const uint32_t b_t = div_by(ap ? (__ldg(I.ref_rs + g_t) >> 1) : g_t - s_lo, h, inv);
         const bool first = !(seg_p == seg && b_p == b_t);
         const bool prev_is_bm1 = seg_p == seg && b_p + 1 == b_t;
-        if (first) {
+        if (first && !dead) {
+            // the hit's two buckets, b_t and b_t - 1 (add_to_pos,
+            // buckets.rs:642-662; the latter unless the seed's previous hit is in it)
+            const bool lower = b_t > 0 && !prev_is_bm1;
+            const uint64_t i1 = bt_hash(seg, b_t, tb.mask), i0 = bt_hash(seg, b_t - 1, tb.mask);
+            const unsigned long long k1 = bt_key(v.bt + tb.base + i1);
+            const unsigned long long k0 = lower ? bt_key(v.bt + tb.base + i0) : 0;
+            int32_t m1 = 1, m0 = 1, c1 = 0, c0 = 0, lo1 = 0, hi1 = 0, lo0 = 0, hi0 = 0;
             if (cnt == 1) {
-                const uint32_t rs = sh_out ? __ldg(I.ref_rs + g_t) : 0u;
-                const int32_t cd = ((rs & 1u) == sstr) ? 1 : -1, r = (int32_t)(rs >> 1);
-                bt_add(v, q, seg, b_t, 1, cd, r, r);  // add_to_pos (buckets.rs:642-662)
-                if (b_t > 0) bt_add(v, q, seg, (int64_t)b_t - 1, 1, cd, r, r);
+                if (sh_out) {
+                    const uint32_t rs = __ldg(I.ref_rs + g_t);
+                    c1 = c0 = ((rs & 1u) == sstr) ? 1 : -1;
+                    lo1 = hi1 = lo0 = hi0 = (int32_t)(rs >> 1);
+                }
             } else if (!ap) {
                 // streamed multi-hit seed: one clamped contribution per bucket
-                // (seeding.rs:113-205). Both of this hit's ranges, buckets b_t
-                // and b_t - 1 (the latter unless the previous hit is in it),
-                // start at this hit: the previous hit lies in a lower bucket
-                // (below b_t - 1 when b_t - 1 is added) or an earlier segment.
-                // Their ends are found by galloping forward.
+                // (seeding.rs:113-205). Both of this hit's ranges start at this
+                // hit: the previous hit lies in a lower bucket (below b_t - 1
+                // when b_t - 1 is added) or an earlier segment. Their ends are
+                // found by galloping forward.
                 const uint32_t A = a + t, E = a + cnt;
                 const uint64_t up1 = (uint64_t)s_lo + (uint64_t)(b_t + 1) * h, up0 = up1 + h;
                 const uint32_t B1 = hits_gallop(I.hits, A + 1, E, (uint32_t)min(up1, (uint64_t)s_hi));
                 const uint32_t B0 = hits_gallop(I.hits, B1, E, (uint32_t)min(up0, (uint64_t)s_hi));
-                if (!sh_out) {  // matches only
-                    bt_add(v, q, seg, b_t, min((int32_t)(B0 - A), (int32_t)occs), 0, 0, 0);
-                    if (b_t > 0 && !prev_is_bm1)
-                        bt_add(v, q, seg, (int64_t)b_t - 1, min((int32_t)(B1 - A), (int32_t)occs), 0, 0, 0);
-                } else {
-                    const int32_t r0 = (int32_t)(__ldg(I.ref_rs + g_t) >> 1);
+                m1 = (int32_t)(B0 - A);
+                m0 = (int32_t)(B1 - A);
+                if (sh_out) {
+                    lo1 = lo0 = (int32_t)(__ldg(I.ref_rs + g_t) >> 1);
                     const uint32_t fwA = __ldg(I.hit_fw + A);
-                    {
-                        const int32_t c = (int32_t)(B0 - A), fw = (int32_t)(__ldg(I.hit_fw + B0) - fwA);
-                        const int32_t same = sstr ? c - fw : fw;
-                        const int32_t r1 = (int32_t)(__ldg(I.ref_rs + __ldg(I.hits + B0 - 1)) >> 1);
-                        bt_add(v, q, seg, b_t, min(c, (int32_t)occs), 2 * same - c, r0, r1);
-                    }
-                    if (b_t > 0 && !prev_is_bm1) {
-                        const int32_t c = (int32_t)(B1 - A), fw = (int32_t)(__ldg(I.hit_fw + B1) - fwA);
-                        const int32_t same = sstr ? c - fw : fw;
-                        const int32_t r1 = (int32_t)(__ldg(I.ref_rs + __ldg(I.hits + B1 - 1)) >> 1);
-                        bt_add(v, q, seg, (int64_t)b_t - 1, min(c, (int32_t)occs), 2 * same - c, r0, r1);
-                    }
+                    const int32_t f1 = (int32_t)(__ldg(I.hit_fw + B0) - fwA), f0 = (int32_t)(__ldg(I.hit_fw + B1) - fwA);
+                    c1 = 2 * (sstr ? m1 - f1 : f1) - m1;
+                    c0 = 2 * (sstr ? m0 - f0 : f0) - m0;
+                    hi1 = (int32_t)(__ldg(I.ref_rs + __ldg(I.hits + B0 - 1)) >> 1);
+                    hi0 = (int32_t)(__ldg(I.ref_rs + __ldg(I.hits + B1 - 1)) >> 1);
                 }
+                m1 = min(m1, (int32_t)occs);
+                m0 = min(m0, (int32_t)occs);
             } else {
                 // streamed multi-hit seed, absolute positions: the ranges by search
-                for (int e = 0; e < 2; e++) {
+                for (int e = 0; e < (lower ? 2 : 1); e++) {
                     const int64_t bb = (int64_t)b_t - e;
-                    if (bb < 0) break;
-                    if (e == 1 && prev_is_bm1) break;
                     uint32_t A, B;
                     seed_range(I, a, cnt, seg, bb * (int64_t)h, (bb + 2) * (int64_t)h, ap, A, B);
-                    Agg g = range_agg(I, A, B, sstr, sh_out);
-                    bt_add(v, q, seg, bb, min(g.count, (int32_t)occs), g.codir, g.rmin, g.rmax);
+                    const Agg g = range_agg(I, A, B, sstr, sh_out);
+                    (e ? m0 : m1) = min(g.count, (int32_t)occs);
+                    (e ? c0 : c1) = g.codir;
+                    (e ? lo0 : lo1) = g.rmin;
+                    (e ? hi0 : hi1) = g.rmax;
                 }
             }
+            bt_add(v, q, tb, seg, b_t, i1, k1, m1, c1, lo1, hi1);
+            if (lower) bt_add(v, q, tb, seg, b_t - 1, i0, k0, m0, c0, lo0, hi0);
         }
         if (++w >= wend) break;
         seg_p = seg;
         b_p = b_t;
-        if (++t == cnt) {  // next seed of the read, or the next read with hits
-            t = 0;
-            seg_p = -1;
-            if (++j == np) {
-                do {
-                    q++;
-                } while (v.hw_off[q + 1] <= w);
-                kb = v.kcap_off[q];
-                np = (uint32_t)v.r_nproc[q];
-                h = (uint32_t)v.r_half[q];
-                j = ub_u32(v.sd_hpre + kb, np, 0u) - 1;  // past the seeds without hits
-            }
+        g_t = g_n;
+        if (in_seed) {
+            t++;
+            continue;
+        }
+        // the next seed of the read, or the next read with hits
+        t = 0;
+        seg_p = -1;
+        if (in_read) {
+            j++;
+            a = nx.a;
+            cnt = nx.cnt;
+            os = nx.os;
+        } else {
+            do {
+                q++;
+            } while (v.hw_off[q + 1] <= w);
+            kb = v.kcap_off[q];
+            np = (uint32_t)v.r_nproc[q];
+            h = (uint32_t)v.r_half[q];
+            inv = 0xffffffffu / h;
+            dead = v.r_flags[q] != 0;
+            tb = BtTab{v.bt_tab[q].x, v.bt_tab[q].y};
+            j = ub_u32(v.sd_hpre + kb, np, 0u) - 1;  // past the seeds without hits
             sr = v.sd[kb + j];
             a = sr.a;
             cnt = sr.cnt;
             os = sr.os;
+            g_t = __ldg(I.hits + a);
         }
+        nx = v.sd[kb + min(j + 1, np - 1)];
     }
 }
 
-__global__ void __launch_bounds__(256) k_contrib(BatchView v) {
+__global__ void __launch_bounds__(256, 4) k_contrib(BatchView v) {
     const uint64_t total = v.hw_off[v.n];
-    const uint32_t run = contrib_run(total);
+    const uint32_t run = contrib_run(v, total);
     const uint64_t nrun = (total + run - 1) / run;
     const int lane = threadIdx.x & 31;
     // a warp takes 32 consecutive runs: the read of its first by a 32-way
@@ -1568,7 +1629,7 @@ __global__ void __launch_bounds__(256) k_contrib(BatchView v) {
 
 // The hits of the reads given a second bucket table (k_bt_second), again: the
 // runs of all of them over the whole grid, each run's read by its first run.
-__global__ void __launch_bounds__(256) k_contrib2(BatchView v) {
+__global__ void __launch_bounds__(256, 4) k_contrib2(BatchView v) {
     const unsigned long long pack = v.mx->bt2_pack;
     const uint32_t nl = (uint32_t)(pack >> BT2_RUN_BITS);
     const uint64_t nrun = pack & (((uint64_t)1 << BT2_RUN_BITS) - 1);
