@@ -1296,9 +1296,11 @@ __device__ __forceinline__ uint32_t hits_gallop(const uint32_t* __restrict__ hit
     return hits_lower_bound(hits, lo, end - lo, v);
 }
 
-// Hits of one seed's list [a, a+cnt) in segment g with pos in [lo, hi): returns [A, B).
+// Hits of one seed's list [a, a+cnt) in segment g with pos in [lo, hi): returns
+// [A, B), or a B with at least `most` hits before it where there are more.
 __device__ __forceinline__ void seed_range(const DevIndex& I, uint32_t a, uint32_t cnt, int32_t g, int64_t lo,
-                                           int64_t hi, bool ap, uint32_t& A, uint32_t& B) {
+                                           int64_t hi, bool ap, uint32_t& A, uint32_t& B,
+                                           uint32_t most = UINT32_MAX) {
     const uint32_t s_lo = __ldg(I.seg_off + g), s_hi = __ldg(I.seg_off + g + 1);
     if (!ap) {
         uint64_t glo = (uint64_t)s_lo + (uint64_t)max(lo, (int64_t)0);
@@ -1307,7 +1309,7 @@ __device__ __forceinline__ void seed_range(const DevIndex& I, uint32_t a, uint32
         A = hits_lower_bound(I.hits, a, cnt, (uint32_t)glo);
         // the range spans two half-lengths, which few hits of a list fall in:
         // its end is galloped to from A rather than searched for from a
-        B = ghi > glo ? hits_gallop(I.hits, A, a + cnt, (uint32_t)ghi) : A;
+        B = ghi > glo ? hits_gallop(I.hits, A, A + min(a + cnt - A, most), (uint32_t)ghi) : A;
         return;
     }
     uint32_t sA = hits_lower_bound(I.hits, a, cnt, s_lo), sB = hits_lower_bound(I.hits, a, cnt, s_hi);
@@ -1537,8 +1539,9 @@ __device__ __forceinline__ void contrib_span(const BatchView& v, uint64_t w, con
                 // (seeding.rs:113-205). Both of this hit's ranges start at this
                 // hit: the previous hit lies in a lower bucket (below b_t - 1
                 // when b_t - 1 is added) or an earlier segment. Their ends are
-                // found by galloping forward.
-                const uint32_t A = a + t, E = a + cnt;
+                // found by galloping forward, no further than the clamp
+                // unless the bucket's content is reported.
+                const uint32_t A = a + t, E = A + min(cnt - t, sh_out ? UINT32_MAX : occs);
                 const uint64_t up1 = (uint64_t)s_lo + (uint64_t)(b_t + 1) * h, up0 = up1 + h;
                 const uint32_t B1 = hits_gallop(I.hits, A + 1, E, (uint32_t)min(up1, (uint64_t)s_hi));
                 const uint32_t B0 = hits_gallop(I.hits, B1, E, (uint32_t)min(up0, (uint64_t)s_hi));
@@ -1824,8 +1827,11 @@ __global__ void __launch_bounds__(256) k_extend(BatchView v) {
                 ds = (int32_t)(os >> 1);
                 if (cnt > 0) {
                     uint32_t A, B;
-                    seed_range(v.I, sr.a, cnt, seg, (int64_t)bb * h, ((int64_t)bb + 2) * h, ap, A, B);
-                    Agg g = range_agg(v.I, A, B, os & 1u, bucket_metric(v.P));
+                    // only the bucket metrics ask for more hits than the seed has occurrences
+                    const bool full = bucket_metric(v.P);
+                    seed_range(v.I, sr.a, cnt, seg, (int64_t)bb * h, ((int64_t)bb + 2) * h, ap, A, B,
+                               full ? UINT32_MAX : (uint32_t)ds);
+                    Agg g = range_agg(v.I, A, B, os & 1u, full);
                     dm = min(g.count, ds);
                     dc = g.codir;
                     rmn = g.rmin;
