@@ -1802,12 +1802,24 @@ __global__ void __launch_bounds__(BSCAN_WARPS * 32) k_bscan(BatchView v) {
 // One warp per bucket; 32 remaining seeds per step, matches_in_bucket for each
 // (pruning.rs:18-80), then an inclusive scan of (seeds, matches) finds the
 // first prefix whose sh drops below theta_low.
-__global__ void __launch_bounds__(256) k_extend(BatchView v) {
+//
+// A warp a job. Bound by the searches' loads: every lane follows its own list.
+// Where a read has many jobs, which are consecutive, the warps of a CTA go
+// through the seeds in step, so that the same 32 lists serve all of them from
+// L1 (12,500 dense reads, 31 jobs a read: 2.6 ms, 5.0 with warps on their own,
+// which drift apart; 17.7 a read 0.71 and 1.18, 9.0 a read 0.49 and 0.57). With
+// fewer jobs a read the lists are not shared and the barriers cost more
+// (150,000 hifi reads, 5.8 a read: 1.6 and 0.94 ms). Two CTAs an SM: three
+// leave 40 registers, hifi 1.08 ms.
+constexpr int EXT_THREADS = 512, EXT_CTAS = 2, EXT_STEP_JOBS = 8;
+__global__ void __launch_bounds__(EXT_THREADS, EXT_CTAS) k_extend(BatchView v) {
     const int lane = threadIdx.x & 31;
     const uint32_t njobs = min(*v.n_jobs, v.job_cap);
-    const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    const bool ap = v.P.ap != 0;
-    for (uint32_t ji = wid; ji < njobs; ji += nwarps) {
+    const uint32_t w0 = blockIdx.x * (EXT_THREADS / 32), wib = threadIdx.x >> 5, nwarps = gridDim.x * (EXT_THREADS / 32);
+    const bool ap = v.P.ap != 0, in_step = njobs / EXT_STEP_JOBS >= (uint32_t)v.n;
+    for (uint32_t j0 = w0; j0 < njobs; j0 += nwarps) {
+        const uint32_t ji = min(j0 + wib, njobs - 1);
+        const bool mine = j0 + wib < njobs;
         BucketJob* J = v.jobs + ji;
         const int32_t q = J->read, seg = J->seg, bb = J->bb;
         const int32_t m = v.r_m[q], n_u = v.r_nu[q], np = v.r_nproc[q];
@@ -1816,7 +1828,9 @@ __global__ void __launch_bounds__(256) k_extend(BatchView v) {
         int32_t seeds = v.r_S0[q], matches = J->matches, codir = J->codir, rmin = J->rmin, rmax = J->rmax;
         bool stopped = false;
         int32_t examined = 0;
-        for (int32_t i0 = np; i0 < n_u; i0 += 32) {
+        int32_t i0 = np;
+        for (bool more = mine && i0 < n_u; in_step ? __syncthreads_or(more) : more; more = more && i0 < n_u) {
+            if (!more) continue;
             examined += min(32, n_u - i0);
             const int32_t i = i0 + lane;
             const bool valid = i < n_u;
@@ -1842,8 +1856,10 @@ __global__ void __launch_bounds__(256) k_extend(BatchView v) {
             const bool low = valid && hseed(m, seeds + ps, matches + pm) < v.P.theta_low;
             if (__any_sync(0xffffffffu, low)) {
                 stopped = true;
-                break;
+                i0 = n_u;
+                continue;
             }
+            i0 += 32;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 dc += __shfl_xor_sync(0xffffffffu, dc, o);
@@ -1856,8 +1872,8 @@ __global__ void __launch_bounds__(256) k_extend(BatchView v) {
             rmin = min(rmin, rmn);
             rmax = max(rmax, rmx);
         }
-        if (lane == 0) atomicAdd(&v.mx->ext_seeds, (unsigned long long)examined);
-        if (lane == 0 && !stopped) {
+        if (lane == 0 && mine) atomicAdd(&v.mx->ext_seeds, (unsigned long long)examined);
+        if (lane == 0 && mine && !stopped) {
             J->sh = hseed(m, seeds, matches);
             J->matches = matches;
             J->codir = codir;
@@ -4175,7 +4191,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     T.end();
     if (!p.no_bucket_pruning) {
         T.begin(STG_EXTEND);
-        k_extend<<<wide, 256, 0, s>>>(v);
+        k_extend<<<grid_for((size_t)job_cap * 32, EXT_THREADS, EXT_CTAS), EXT_THREADS, 0, s>>>(v);
         SHM_CUDA(cudaGetLastError());
         T.end();
     }
