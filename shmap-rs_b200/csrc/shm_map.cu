@@ -81,6 +81,7 @@ struct BatchMax {
     unsigned int far_bin[FAR_BINS];  // those candidates by cost bin (their read's bucket half-length)
     unsigned int far_next[2];        // next candidate of the refinement queue a warp takes, per pass
     unsigned int n_jobs, n_cands;    // bucket jobs, candidates
+    unsigned int bt_pre, pad;        // reads put down for a second table before their contributions
     unsigned long long refined;      // candidates refined (the reads' leads and those that can still score)
     unsigned long long bt2_next;     // spare bucket-table slots handed out (second tables)
     // reads given a second table (listed in bt2_list) << BT2_RUN_BITS, plus the
@@ -1489,10 +1490,21 @@ __device__ __forceinline__ void contrib_span(const BatchView& v, uint64_t w, con
     const bool ap = v.P.ap != 0;
     const bool sh_out = bucket_metric(v.P);  // codirection and positions are reported (bucket metrics)
     const DevIndex& I = v.I;
+    // past the reads that are mapped again, or given a second table first
+    auto live = [&]() -> bool {
+        while (__ldcg(v.r_flags + q)) {
+            w = v.hw_off[q + 1];
+            if (w >= wend) return false;
+            do {
+                q++;
+            } while (v.hw_off[q + 1] <= w);
+        }
+        return true;
+    };
+    if (!live()) return;
     uint64_t kb = v.kcap_off[q];
     uint32_t np = (uint32_t)v.r_nproc[q];
     uint32_t h = (uint32_t)v.r_half[q], inv = 0xffffffffu / h;
-    bool dead = v.r_flags[q] != 0;  // the read is mapped again, or given a second table first
     BtTab tb{v.bt_tab[q].x, v.bt_tab[q].y};
     uint32_t j = ub_u32(v.sd_hpre + kb, np, (uint32_t)(w - v.hw_off[q])) - 1;
     uint32_t t = (uint32_t)(w - v.hw_off[q]) - v.sd_hpre[kb + j];
@@ -1520,7 +1532,7 @@ __device__ __forceinline__ void contrib_span(const BatchView& v, uint64_t w, con
         const uint32_t b_t = div_by(ap ? (__ldg(I.ref_rs + g_t) >> 1) : g_t - s_lo, h, inv);
         const bool first = !(seg_p == seg && b_p == b_t);
         const bool prev_is_bm1 = seg_p == seg && b_p + 1 == b_t;
-        if (first && !dead) {
+        if (first) {
             // the hit's two buckets, b_t and b_t - 1 (add_to_pos,
             // buckets.rs:642-662; the latter unless the seed's previous hit is in it)
             const bool lower = b_t > 0 && !prev_is_bm1;
@@ -1594,11 +1606,11 @@ __device__ __forceinline__ void contrib_span(const BatchView& v, uint64_t w, con
             do {
                 q++;
             } while (v.hw_off[q + 1] <= w);
+            if (!live()) return;
             kb = v.kcap_off[q];
             np = (uint32_t)v.r_nproc[q];
             h = (uint32_t)v.r_half[q];
             inv = 0xffffffffu / h;
-            dead = v.r_flags[q] != 0;
             tb = BtTab{v.bt_tab[q].x, v.bt_tab[q].y};
             j = ub_u32(v.sd_hpre + kb, np, 0u) - 1;  // past the seeds without hits
             sr = v.sd[kb + j];
@@ -1654,13 +1666,26 @@ __global__ void __launch_bounds__(256, 4) k_contrib2(BatchView v) {
 // Clears the batch's bucket tables, the first `pool` slots at most: a read
 // whose table would end past the pool is flagged (mapped again) before any
 // kernel touches it.
+// A read with a capped table, at least a processed seed and BT_PRE hits for each
+// of its slots is put down for a second table at once: it would fill the first
+// and have its contributions made twice (12,500 dense reads, a fifth of them
+// in satellites: 4.25 ms, 3.2 so). By hits alone the rule also takes reads of
+// few seeds, whose hits share buckets and whose first table does (150,000 hifi
+// reads: 1.59 ms against 1.28). No more than pre_most reads, which leaves spare
+// slots for others.
+constexpr uint64_t BT_PRE = 16;
 __global__ void k_bt_init(BSlot* bt, const uint64_t* __restrict__ bt_off, int32_t n_reads, uint64_t pool,
-                          uint32_t* __restrict__ r_flags, ulonglong2* __restrict__ bt_tab) {
+                          uint32_t* __restrict__ r_flags, ulonglong2* __restrict__ bt_tab,
+                          const uint64_t* __restrict__ hw_off, const int32_t* __restrict__ r_nproc, uint64_t cap,
+                          uint32_t pre_most, unsigned int* pre) {
     const uint64_t n = min(bt_off[n_reads], pool);
     for (int32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n_reads; q += gridDim.x * blockDim.x) {
         const uint64_t b = bt_off[q], e = bt_off[q + 1];
         bt_tab[q] = make_ulonglong2(b, e - b - 1);
         if (e > pool) r_flags[q] = 1u;
+        else if (pre_most && e - b == cap && (uint64_t)r_nproc[q] >= cap && hw_off[q + 1] - hw_off[q] >= BT_PRE * cap &&
+                 atomicAdd(pre, 1u) < pre_most)
+            r_flags[q] = 1u;
     }
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         BSlot s;
@@ -4155,7 +4180,8 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     v.bt_pool = bt_slots_alloc;
     v.bt2_spare = spare;
     T.begin(STG_AUX);
-    k_bt_init<<<wide, 256, 0, s>>>(S.bt.p, S.bt_off.p, n, bt_slots_alloc, Z.r_flags, S.bt_tab.p);
+    k_bt_init<<<wide, 256, 0, s>>>(S.bt.p, S.bt_off.p, n, bt_slots_alloc, Z.r_flags, S.bt_tab.p, v.hw_off, v.r_nproc,
+                                   v.bt_cap, (uint32_t)std::min<uint64_t>(spare / BT2_MAX * 3 / 4, (uint64_t)n), &Z.mx->bt_pre);
     SHM_CUDA(cudaGetLastError());
     T.end();
     T.begin(STG_CONTRIB);
