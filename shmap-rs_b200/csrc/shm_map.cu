@@ -3272,11 +3272,13 @@ __global__ void __launch_bounds__(SWEEP_WARPS * 32) k_sweep(BatchView v, SweepCa
         const SweepCand* L;
         // Without a tie-break band both sweeps look only at candidates whose
         // score is above a threshold of at least theta_low (pass 2's is best *
-        // (1 - d) with best > theta), so the others, candidates never refined
-        // among them, are left out: a read from a repeat has hundreds of
-        // candidates and a few that pass (150,000 hifi reads: 0.53 ms, one lane
-        // walking every candidate, against 0.13).
-        const bool cut = v.P.tiebreak == 0.0;
+        // (1 - d) with best > theta, while 1 - d is not negative), so the
+        // others, candidates never refined among them, are left out: a read from
+        // a repeat has hundreds of candidates and a few that pass (150,000 hifi
+        // reads: 0.53 ms, one lane walking every candidate, against 0.13).
+        // Above d = 1 pass 2's threshold falls below theta_low, and it looks at
+        // scores of zero and at the -1 of empty windows too.
+        const bool cut = v.P.tiebreak == 0.0 && v.P.min_diff <= 1.0;
         uint32_t kept = 0;
         for (uint32_t i0 = 0; i0 < nc && kept <= SWEEP_CAP; i0 += 32) {
             const uint32_t i = i0 + lane;
