@@ -4277,7 +4277,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
         v.lcs_pos = S.lcs_pos.p;
         bm_words = (int32_t)std::min<int64_t>((bp.max_len + 31) / 32, LCS_BITS_WORDS) + 1 & ~1;
         const int bm_bytes = 6 * bm_words;
-        if (bm_bytes > 48 * 1024 && !c->lcs_smem_set) {
+        if (!c->lcs_smem_set) {  // (with the kernel's static arrays, 48 KiB are passed below 8,192 words)
             SHM_CUDA(cudaFuncSetAttribute(k_lcs_occ, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * LCS_BITS_WORDS));
             c->lcs_smem_set = 1;
         }
