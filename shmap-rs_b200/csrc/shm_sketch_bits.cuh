@@ -27,7 +27,8 @@
 // K is a template parameter because the tables are immediates.
 //
 // A tile with any byte that is no letter (or a masked base) rolls its
-// sub-runs through the byte tables instead, a lane each.
+// sub-runs instead, a lane each, eight bases of it in registers at a time and
+// the letters' words from five shared entries.
 //
 // Bound by integer issue, as the rolling kernels were, with a third of their
 // instructions: 0.36 warp instructions a base against 1.09 (half of them the
@@ -52,8 +53,10 @@ constexpr int SKB_WARPS = 8;
 constexpr int SKB_LEAD = 8;                // words before the sub-runs (lanes 0 and 1)
 constexpr int SKB_WORDS = 4 + 4 * 32 + 36; // a plane of a tile in shared memory: a pad, the lanes' words, the next sub-run's
 constexpr int SKB_Q = 128;                 // queued candidates of a warp
+constexpr uint32_t SKB_WAIT = 96;          // rolled windows selected and not yet listed
 constexpr int SKB_SPAN = SKB_TILE + 128;   // bases a tile loads: the lead, 32 sub-runs, 120 past them
 static_assert(SKB_S == 4 * 32 - SKB_LEAD && SKB_LEAD >= SKB_PL - 1, "lanes cover the lead and the sub-run");
+static_assert(SKB_WAIT * 12 <= 2 * SKB_WORDS * 4, "they wait in the planes' place");
 
 // Letter words by code, and their reverse complements' (the constants of src/sketch.rs:60-75).
 __host__ __device__ constexpr uint64_t skb_fw(int code) {
@@ -216,12 +219,40 @@ struct SkbSource {
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    // Byte of the read's letters at p: 0 outside [lo, hi), 'N' for a masked base.
-    __device__ __forceinline__ uint32_t letter(int64_t p) const {
-        if (p < lo || p >= hi) return 0u;
-        if (!PK) return __ldg(seq + p);
-        if ((__ldg(mask + (p >> 5)) >> (p & 31)) & 1u) return 0x4eu;
-        return (uint32_t)"ACTG"[(__ldg(codes + (p >> 4)) >> (2 * (p & 15))) & 3u];
+    // Eight bases from p, which is a multiple of 8 from the fetched bytes' start
+    // (so they share a word), as indices of the roll entries, four bits each:
+    // the code, or 4 for a base that is no letter, masked or outside [lo, hi).
+    // Reads only words that hold a base of [lo, hi).
+    __device__ __forceinline__ uint32_t eight(int64_t p) const {
+        if (p + 8 <= lo || p >= hi) return 0x44444444u;
+        const uint32_t out = (p < lo ? 0xffu >> (8 - (int)(lo - p)) : 0u) | (p + 8 > hi ? 0xffu << (int)(hi - p) : 0u);
+        uint32_t c, bad;  // two bits a base, one bit a base
+        if (PK) {
+            c = __ldg(codes + (p >> 4)) >> (2 * (p & 15)) & 0xffffu;
+            bad = __ldg(mask + (p >> 5)) >> (p & 31);
+        } else {
+            uint2 w = make_uint2(0u, 0u);
+            if (out == 0) {
+                w = __ldg((const uint2*)(seq + p));
+            } else {
+#pragma unroll 1
+                for (int i = (int)max(lo - p, (int64_t)0); i < (int)min(hi - p, (int64_t)8); i++) {
+                    const uint32_t x = (uint32_t)__ldg(seq + p + i) << (8 * (i & 3));
+                    if (i < 4) w.x |= x;
+                    else w.y |= x;
+                }
+            }
+            c = codes4(w.x) | codes4(w.y) << 8;
+            bad = bad4(w.x) | bad4(w.y) << 4;
+        }
+        bad = (bad | out) & 0xffu;
+        c = (c | c << 8) & 0x00ff00ffu;  // spread to four bits a base
+        c = (c | c << 4) & 0x0f0f0f0fu;
+        c = (c | c << 2) & 0x33333333u;
+        bad = (bad | bad << 12) & 0x000f000fu;
+        bad = (bad | bad << 6) & 0x03030303u;
+        bad = (bad | bad << 3) & 0x11111111u;
+        return (c & ~(3u * bad)) | bad << 2;
     }
     // Code byte (four bases, the earliest in bits 0-1) of bases p + 4g .. of a
     // window of K bases at p; bases past the window are any (their table
@@ -255,6 +286,17 @@ struct SkbSource {
     }
 };
 
+// What a base contributes to a rolled window's hashes (F low, high, R low,
+// high) as it enters (side 0) and as it leaves (side 1): entries by code, then
+// the one of a base that hashes to 0.
+template <int K>
+__device__ __forceinline__ uint4 skb_roll_entry(int side, int code) {
+    if (code > 3) return make_uint4(0u, 0u, 0u, 0u);
+    const uint64_t f = rotl64(skb_fw(code), side ? K : 0), c = skb_fw(code ^ 2);
+    const uint64_t r = side ? rotr64(c, 1) : rotl64(c, K - 1);
+    return make_uint4((uint32_t)f, (uint32_t)(f >> 32), (uint32_t)r, (uint32_t)(r >> 32));
+}
+
 // Bit b of lane a's word to bit a of lane b's.
 __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
 #pragma unroll
@@ -270,6 +312,7 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
 template <int K, bool PK>
 struct SkbShared {
     uint4 wt[(K + 3) / 4][256];
+    uint4 roll[2][5];  // skb_roll_entry
     uint32_t pl[SKB_WARPS][2][SKB_WORDS];
     uint32_t q[SKB_WARPS][SKB_Q];
     uint8_t tile[SKB_WARPS][PK ? SKB_SPAN / 4 : SKB_SPAN];
@@ -282,6 +325,143 @@ constexpr int skb_ctas() {
     return 3 * (sizeof(SkbShared<K, PK>) + 1024) <= 228 * 1024 ? 3 : 2;
 }
 
+// A tile whose bases are not all letters, by one warp: a lane rolls its
+// sub-run of windows from t0 + SKB_S * lane, its bases read once, eight at a
+// time as indices into the roll entries (skb_roll_entry, entering then
+// leaving); those of the last K bases wait in registers, and the selected
+// windows until the warp lists 32 at once. Out of line: its registers are not
+// the other tiles'. Bound by integer issue, some 30 instructions a base and
+// lane. 60 Mbases of letters with an N every 500, where every tile comes here:
+// the sketch 0.19 ms (0.60 with a base read as it entered and again as it
+// left, its words looked up in the byte tables, and a list counter's round
+// trip for every selected window), 0.054 without the Ns.
+// `wait`: the warp's planes, SKB_WAIT selected windows (not ORD). Returns
+// ord_n and the tile's selected windows.
+template <int K, bool PK, bool ORD>
+__device__ __noinline__ uint32_t skb_roll_tile(const SketchArgs& a, SkbSource<PK> src, const uint4* entries,
+                                               uint32_t* wait, int64_t t0, int64_t base, int32_t q_tile,
+                                               uint64_t ord_base, uint32_t ord_cap, uint32_t ord_n) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const uint64_t thr = a.thr;
+    const uint32_t thr_hi = (uint32_t)(thr >> 32);
+    const int64_t s0 = t0 + SKB_S * lane;
+    const int w0 = (int)min(max(src.lo - s0, (int64_t)0), (int64_t)SKB_S);
+    const int w1 = (int)min(max(src.hi - s0, (int64_t)0), (int64_t)SKB_S);
+    auto rs_of = [&](int64_t p, int32_t q, bool strand) {
+        return ((uint32_t)((int32_t)(p - __ldg(a.seq_off + q)) + K - 1 + a.r_offset) << 1) | (strand ? 1u : 0u);
+    };
+    // each(window, selected, F, R) is called by all lanes together, for every
+    // window of the sub-run that is selected in some lane
+    auto roll = [&](auto&& each) {
+        constexpr int BACK = (K + 7) / 8;  // words of eight bases to the first that leaves with this one's
+        uint32_t W[BACK + 1];
+#pragma unroll
+        for (int x = 0; x <= BACK; x++) W[x] = 0x44444444u;  // (before the first base: none)
+        uint32_t flo = 0, fhi = 0, rlo = 0, rhi = 0;
+#pragma unroll 1
+        for (int b0 = 0; b0 < SKB_S + K - 1; b0 += 8) {
+#pragma unroll
+            for (int x = 0; x < BACK; x++) W[x] = W[x + 1];
+            W[BACK] = src.eight(s0 + b0);
+            uint32_t in = W[BACK], out = K % 8 ? __funnelshift_r(W[0], W[1], 4 * (8 - K % 8)) : W[0];
+#pragma unroll 1
+            for (int b = b0; b < b0 + 8; b++) {
+                const uint4 e = entries[in & 7u], l = entries[5 + (out & 7u)];
+                in >>= 4;
+                out >>= 4;
+                const uint32_t f0 = __funnelshift_l(fhi, flo, 1), r0 = __funnelshift_r(rlo, rhi, 1);
+                fhi = __funnelshift_l(flo, fhi, 1) ^ e.y ^ l.y;
+                flo = f0 ^ e.x ^ l.x;
+                rhi = __funnelshift_r(rhi, rlo, 1) ^ e.w ^ l.w;
+                rlo = r0 ^ e.z ^ l.z;
+                if (__ballot_sync(FULL, (fhi ^ rhi) <= thr_hi) == 0) continue;
+                const uint64_t f = u64_of(flo, fhi), r = u64_of(rlo, rhi);
+                const int w = b - (K - 1);
+                each(w, (f ^ r) <= thr && w >= w0 && w < w1, f, r);
+            }
+        }
+    };
+    if (ORD) {
+        // counted first, for the lanes' places, then written (a lane's windows ascend)
+        int32_t q = q_tile;
+        auto whole = [&](int w) {  // window w of the lane's sub-run lies in one sequence, q
+            const int64_t p = s0 + w;
+            while (__ldg(a.seq_off + q + 1) <= p) q++;  // ends: p < hi = seq_off[n_seq]
+            return p + K <= __ldg(a.seq_off + q + 1);
+        };
+        uint32_t mine = 0;
+        roll([&](int w, bool sel, uint64_t, uint64_t) {
+            if (sel && whole(w)) {
+                mine++;
+                if (a.ord_seq_cnt) atomicAdd(a.ord_seq_cnt + q, 1u);
+            }
+        });
+        __syncwarp();
+        const uint32_t inc = warp_inclusive_scan(mine);
+        uint32_t slot = ord_n + inc - mine;
+        q = q_tile;
+        if (ord_cap)
+            roll([&](int w, bool sel, uint64_t f, uint64_t r) {
+                if (sel && whole(w)) {
+                    if (slot < ord_cap) {
+                        a.out_h[ord_base + slot] = f ^ r;
+                        a.out_rs[ord_base + slot] = rs_of(s0 + w, q, f > r);
+                    }
+                    slot++;
+                }
+            });
+        return ord_n + __shfl_sync(FULL, inc, 31);
+    }
+    // the selected windows wait until there are enough for the whole warp
+    // (their positions relative to base | strand << 31)
+    uint64_t* const wh = (uint64_t*)wait;
+    uint32_t* const wp = (uint32_t*)(wh + SKB_WAIT);
+    uint32_t nw = 0;
+    auto list = [&](uint32_t b, uint32_t n) {  // (as take of k_sketch_bits, from q_tile on, the hashes known)
+        const bool act = (uint32_t)lane < n;
+        const uint32_t e = act ? wp[b + lane] : 0u, rel = e & 0x7fffffffu;
+        const int64_t p = base + rel, pmax = base + __reduce_max_sync(FULL, rel);
+        int32_t q = q_tile;
+        for (int32_t q1 = q_tile + 1;; q1 += 32) {
+            const int64_t s = q1 + lane <= a.n_seq ? __ldg(a.seq_off + q1 + lane) : INT64_MAX;
+            const int nle = __popc(__ballot_sync(FULL, s <= pmax));
+            for (int x = 0; x < nle; x++) q += __shfl_sync(FULL, s, x) <= p ? 1 : 0;
+            if (nle < 32) break;
+        }
+        const bool sel = act && p + K <= __ldg(a.seq_off + min(q, a.n_seq - 1) + 1);
+        const unsigned peers = __match_any_sync(FULL, sel ? q : -1);
+        const int leader = __ffs(peers) - 1;
+        uint32_t at = 0;
+        if (sel && lane == leader) at = atomicAdd(a.kmer_cnt + q, (uint32_t)__popc(peers));
+        at = __shfl_sync(FULL, at, leader) + __popc(peers & ((1u << lane) - 1u));
+        if (sel) {
+            const uint64_t o = __ldg(a.kmer_off + q);
+            if (at < (uint32_t)(__ldg(a.kmer_off + q + 1) - o)) {
+                a.out_h[o + at] = wh[b + lane];
+                a.out_rs[o + at] = rs_of(p, q, e >> 31);
+            }
+        }
+    };
+    roll([&](int w, bool sel, uint64_t f, uint64_t r) {
+        const unsigned bal = __ballot_sync(FULL, sel);
+        if (sel) {
+            const uint32_t at = nw + __popc(bal & ((1u << lane) - 1u));
+            wh[at] = f ^ r;
+            wp[at] = (uint32_t)(s0 + w - base) + (f > r ? 1u << 31 : 0u);
+        }
+        nw += __popc(bal);
+        if (nw > SKB_WAIT - 32) {
+            __syncwarp();
+            while (nw >= 32) list(nw -= 32, 32);
+            __syncwarp();
+        }
+    });
+    __syncwarp();
+    for (uint32_t b = 0; b < nw; b += 32) list(b, min(32u, nw - b));
+    return ord_n;
+}
+
 // ORD: the k-mers of a warp's tiles in sequence order, counted in
 // a.ord_cnt[warp] and written (as many as there is room for) from
 // a.ord_off[warp] to a.ord_off[warp + 1], or with no ord_off from warp *
@@ -289,7 +469,7 @@ constexpr int skb_ctas() {
 // candidate masks are transposed first, so that lane i holds sub-run i's and
 // the queue fills in order.
 template <int K, bool PK, bool ORD>
-__global__ void __launch_bounds__(SKB_WARPS * 32, skb_ctas<K, PK>()) k_sketch_bits(SketchArgs a,
+__global__ void __launch_bounds__(SKB_WARPS * 32, skb_ctas<K, PK>()) k_sketch_bits(const __grid_constant__ SketchArgs a,
                                                                           const SketchTabs* __restrict__ tabs) {
     constexpr int NG = (K + 3) / 4;
     extern __shared__ __align__(16) uint8_t skb_smem[];
@@ -317,6 +497,7 @@ __global__ void __launch_bounds__(SKB_WARPS * 32, skb_ctas<K, PK>()) k_sketch_bi
         asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&s_wt[0][0] + i)),
                      "l"(&tabs->wt[0][0] + i)
                      : "memory");
+    if (threadIdx.x < 10) sm.roll[threadIdx.x / 5][threadIdx.x % 5] = skb_roll_entry<K>(threadIdx.x / 5, threadIdx.x % 5);
     if (any) src.fetch(buf, base - SKB_LEAD, lane);
     int32_t q_tile = warp_last_le((const uint64_t*)a.seq_off, a.n_seq, (uint64_t)min(max(base, lo), hi), lane);
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -471,62 +652,12 @@ __global__ void __launch_bounds__(SKB_WARPS * 32, skb_ctas<K, PK>()) k_sketch_bi
         if (tl + 1 < t_end) src.fetch(buf, t0 + SKB_TILE - SKB_LEAD, lane);
         uint32_t le[4] = {0u, 0u, 0u, 0u};
         if (__any_sync(FULL, bad != 0)) {
-            // a lane rolls sub-run `lane` through the byte tables; take_one gets
-            // each selected window's sequence, hash and r << 1 | strand
-            auto roll = [&](auto&& take_one) {
-                const int64_t s0 = t0 + SKB_S * lane;
-                uint64_t f = 0, r = 0;
-                for (int i = 0; i < K; i++) {
-                    const uint32_t c = src.letter(s0 + i);
-                    f = rotl64(f, 1) ^ __ldg(&tabs->luts.fw[c]);
-                    r = rotr64(r, 1) ^ __ldg(&tabs->luts.rc_k1[c]);
-                }
-                int32_t q = q_tile;
-                for (int t = 0; t < SKB_S; t++) {
-                    const int64_t p = s0 + t;
-                    const uint64_t h = f ^ r;
-                    if (h <= thr && p >= lo && p < hi) {
-                        while (__ldg(a.seq_off + q + 1) <= p) q++;  // ends: p < hi = seq_off[n_seq]
-                        if (p + K <= __ldg(a.seq_off + q + 1))
-                            take_one(q, h, ((uint32_t)((int32_t)(p - __ldg(a.seq_off + q)) + K - 1 + a.r_offset) << 1) |
-                                               (f > r ? 1u : 0u));
-                    }
-                    const uint32_t ci = src.letter(p + K), co = src.letter(p);
-                    f = rotl64(f, 1) ^ __ldg(&tabs->luts.fw_k[co]) ^ __ldg(&tabs->luts.fw[ci]);
-                    r = rotr64(r, 1) ^ __ldg(&tabs->luts.rc_r1[co]) ^ __ldg(&tabs->luts.rc_k1[ci]);
-                }
-            };
             if (ORD) {
                 if (qn) take(0, qn);  // the tiles before come first
                 qn = 0;
-                __syncwarp();
-                uint32_t mine = 0;
-                roll([&](int32_t q, uint64_t, uint32_t) {
-                    mine++;
-                    if (a.ord_seq_cnt) atomicAdd(a.ord_seq_cnt + q, 1u);
-                });
-                __syncwarp();
-                const uint32_t inc = warp_inclusive_scan(mine);
-                uint32_t slot = ord_n + inc - mine;
-                ord_n += __shfl_sync(FULL, inc, 31);
-                if (ord_cap)
-                    roll([&](int32_t, uint64_t h, uint32_t rs) {
-                        if (slot < ord_cap) {
-                            a.out_h[ord_base + slot] = h;
-                            a.out_rs[ord_base + slot] = rs;
-                        }
-                        slot++;
-                    });
-            } else {
-                roll([&](int32_t q, uint64_t h, uint32_t rs) {
-                    const uint64_t o = __ldg(a.kmer_off + q);
-                    const uint32_t at = atomicAdd(a.kmer_cnt + q, 1u);
-                    if (at < (uint32_t)(__ldg(a.kmer_off + q + 1) - o)) {
-                        a.out_h[o + at] = h;
-                        a.out_rs[o + at] = rs;
-                    }
-                });
             }
+            __syncwarp();
+            ord_n = skb_roll_tile<K, PK, ORD>(a, src, sm.roll[0], pl0, t0, base, q_tile, ord_base, ord_cap, ord_n);
             __syncwarp();
         } else {
             uint32_t o0[4], o1[4];
