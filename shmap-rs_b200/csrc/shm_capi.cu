@@ -216,7 +216,7 @@ int shm_sketch(shm_ctx* ctx, const uint8_t* seq, int64_t len, int32_t k, double 
     // counted by parts (a warp's tiles, or a run of windows), scanned, written
     // in order. Up to 2^22 windows nothing waits for the count: there is room
     // for every window, and about the expected number comes back with it.
-    const bool bits = shm::sketch_bits_takes(k);
+    const bool bits = shm::sketch_bits_takes(k, a.thr);
     const uint64_t parts = bits ? shm::ordered_warps(a) : (uint64_t)((nw + shm::SKETCH_WIN - 1) / shm::SKETCH_WIN);
     d_cnt.reserve(parts + 1, s);
     d_out.reserve(parts + 1, s);

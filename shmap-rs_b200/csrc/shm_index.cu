@@ -293,7 +293,7 @@ IndexStorage* build_index(const uint8_t* h_seq, const int64_t* seg_off_b, int32_
         a.base1 = total_bases;
         uint32_t n_kmers = 0;
         ix->seg_off.reserve((size_t)n_seg + 1, s);
-        if (sketch_bits_takes(k) && total_bases > 0) {
+        if (sketch_bits_takes(k, thr) && total_bases > 0) {
             // on bit planes: every warp's and segment's k-mers counted, then written at their places
             const uint32_t nw = ordered_warps(a);
             TmpBuf<uint32_t> seg_cnt;

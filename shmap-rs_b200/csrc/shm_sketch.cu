@@ -829,10 +829,7 @@ SketchLuts* create_device_luts(int32_t k, cudaStream_t s) {
 // The instances of the bit-plane kernels (an object each: shm_sketch_bits.cu).
 // They hold two words of bases a window (k <= 33) and tables of eight groups
 // of four bases (k <= 32); below 15 a k-mer says little about a genome's
-// place and the rolling kernels stay. At every hash ratio the bit planes are
-// the faster (0.092 Gbases, k = 25, ms on bit planes / rolled: letters 0.07 /
-// 0.16 at r = 0.01, 0.55 / 1.57 at 0.25, 2.65 / 7.49 at 1; packed 0.07 / 0.16,
-// 0.48 / 0.93, 2.32 / 5.54).
+// place and the rolling kernels stay.
 constexpr int SKB_KMIN = 15, SKB_KMAX = 32;
 template <int K>
 int launch_sketch_bits_k(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s);
@@ -846,7 +843,32 @@ static int launch_bits_of(const SketchArgs& a, const SketchTabs* tabs, cudaStrea
 static int launch_bits(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s) {
     return launch_bits_of(a, tabs, s, std::make_integer_sequence<int, SKB_KMAX - SKB_KMIN + 1>{});
 }
-bool sketch_bits_takes(int32_t k) { return k >= SKB_KMIN && k <= SKB_KMAX; }
+// A window whose top hash bits pass costs the bit planes its full hash, one by
+// one, and the rolling kernels nothing more: above a hash ratio of 1/4 these
+// take every sequence in order (k = 25, an index of 3,000 bases at r = 1:
+// planes 0.63 ms, rolled 0.41; 100 Mbases 62 and 60; one sequence of 3,000 at
+// 0.2: 0.10 and 0.09, at 0.1: 0.08 and 0.09) ...
+bool sketch_bits_takes(int32_t k, uint64_t thr) { return k >= SKB_KMIN && k <= SKB_KMAX && thr <= (uint64_t)1 << 62; }
+// ... and of the reads those where a warp's tile of windows is all there is to
+// do (few bases, short reads, whose lists' counters the rolling kernels do not
+// wait for). Sketch stage in ms, planes / rolled:
+//   bases / read length   r = 0.25      0.3           0.4           0.5           0.7           1
+//     150 / 150           0.01 / 0.03   0.01 / 0.03   0.01 / 0.03   0.01 / 0.03   0.19 / 0.04   0.21 / 0.05
+//     9 k / 9 k           0.05 / 0.06   0.06 / 0.07   0.08 / 0.05   0.10 / 0.05   0.19 / 0.06   0.23 / 0.06
+//     300 k / 150         0.09 / 0.10   0.11 / 0.08   0.14 / 0.08   0.17 / 0.09   0.25 / 0.09   0.38 / 0.10
+//     300 k / 10 k        0.06 / 0.11   0.07 / 0.11   0.10 / 0.12   0.12 / 0.14   0.23 / 0.20   0.28 / 0.30
+//     3 M / 1.5 k         -             0.09 / 0.12   0.11 / 0.11   0.14 / 0.12   0.24 / 0.13   0.31 / 0.13
+//     3 M / 10 k          0.08 / 0.15   0.08 / 0.19   0.11 / 0.25   0.13 / 0.33   0.23 / 0.48   0.29 / 0.67
+//     30 M / 150          -             0.54 / 0.41   0.71 / 0.46   0.89 / 0.52   1.27 / 0.64   1.82 / 0.78
+//     30 M / 1.5 k        -             0.28 / 0.45   0.38 / 0.49   0.48 / 0.54   0.71 / 0.64   1.09 / 0.48
+//     30 M / 10 k         0.23 / 0.50   0.27 / 0.62   0.36 / 0.82   0.46 / 1.05   0.67 / 1.50   1.05 / 1.92
+bool sketch_bits_reads(int32_t k, uint64_t thr, int64_t bases, int32_t n) {
+    if (k < SKB_KMIN || k > SKB_KMAX) return false;
+    if (thr <= (uint64_t)1 << 62) return true;
+    if (thr > (uint64_t)1 << 63) return bases > 300000 && bases > 2000 * (int64_t)n;
+    // (a tile has 3,840 windows)
+    return bases <= 3840 || (bases > 500 * (int64_t)n && (thr <= UINT64_MAX / 3 || bases > 100000));
+}
 void launch_sketch_bits(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s) { launch_bits(a, tabs, s); }
 uint32_t ordered_warps(const SketchArgs& a) {
     uint32_t any;  // (asks for the grid only: no tables, nothing is launched)
@@ -867,11 +889,12 @@ void launch_sketch(int mode, const SketchArgs& a, const SketchLuts* L, cudaStrea
     if (a.n_chunks == 0) return;
     const bool pk = a.pk_codes != nullptr;
     if (pk && mode != SK_APPEND) throw shm_cuda_error(cudaErrorInvalidValue);
-    // reads go through the bit planes where their k has an instance; other
+    // reads go through the bit planes where sketch_bits_reads says so; other
     // packed reads roll in the rotated frame (k_sketch_pk); SHMAP_SKETCH_LETTERS=1
     // rolls all of them from their letters instead (the same selections)
     static const bool letters = std::getenv("SHMAP_SKETCH_LETTERS") != nullptr;
-    if (mode == SK_APPEND && !letters && a.base1 > a.base0 && sketch_bits_takes(a.k)) {
+    if (mode == SK_APPEND && !letters && a.base1 > a.base0 &&
+        sketch_bits_reads(a.k, a.thr, a.base1 - a.base0, a.n_seq)) {
         launch_sketch_bits(a, (const SketchTabs*)L, s);
         return;
     }

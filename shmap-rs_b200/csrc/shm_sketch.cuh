@@ -52,12 +52,15 @@ struct SketchArgs {
 // (owned by the caller, released with cudaFree).
 struct SketchLuts;
 SketchLuts* create_device_luts(int32_t k, cudaStream_t s);
-// The bit-plane kernels (shm_sketch_bits.cuh) take an SK_APPEND call of this k.
-bool sketch_bits_takes(int32_t k);
+// The bit-plane kernels (shm_sketch_bits.cuh) take sequences in order
+// (launch_sketch_ordered) at this k and threshold, and n reads of `bases` bases
+// in all (SK_APPEND).
+bool sketch_bits_takes(int32_t k, uint64_t thr);
+bool sketch_bits_reads(int32_t k, uint64_t thr, int64_t bases, int32_t n);
 struct SketchTabs;
 void launch_sketch_bits(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s);
 // The selected windows of all sequences of a (seq, seq_off, n_seq, k, thr,
-// r_offset, base0, base1; a k that sketch_bits_takes) in sequence order, by
+// r_offset, base0, base1; where sketch_bits_takes) in sequence order, by
 // warps that each take a contiguous part: warp w's number goes to cnt[w], and
 // from off[w] to off[w + 1] of a.out_h and a.out_rs (off null: from w * stride,
 // at most stride) as many of them as there is room for; seq_cnt (may be null,
