@@ -2227,8 +2227,8 @@ __device__ __forceinline__ int32_t warp_inclusive_max(int32_t x) {
 //  * in Td the group's values increase, and value t's place is the first
 //    one past value t-1's: p_t = max(q_t, p_(t-1) + 1) with q_t its place
 //    among the tails before it, a running maximum of q_j - j.
-__device__ __forceinline__ int32_t lcs_one(const BatchView& v, const BucketJob* J, int32_t q, int32_t* Ti, int32_t* Td,
-                                           int lane) {
+__device__ __noinline__ int32_t lcs_one(const BatchView& v, const BucketJob* J, int32_t q, int32_t* Ti, int32_t* Td,
+                                        int lane) {
     const DevIndex& I = v.I;
     const int64_t h = v.r_half[q];
     const uint64_t kb = v.kcap_off[q];
@@ -2940,9 +2940,13 @@ __global__ void __launch_bounds__(REFINE_WARPS * 32, 4) k_refine_rarity(BatchVie
 
 // bucket_LCS over the refinement queue, a warp a candidate: by bit vectors
 // for reads with ranked positions, a vector word or more a lane by the read's
-// k-mers, else with the two tail arrays in the warp's global scratch. The
-// record takes the bucket's own content, as bucket_SH's does.
+// k-mers, else (TAILS: the batch may have such reads) with the two tail arrays
+// in the warp's global scratch. The record takes the bucket's own content, as
+// bucket_SH's does. (The tails out of line and only where they can be needed:
+// 20 reads of 0.9 Mb take 6.2 ms with them inline, 5.8 so, 2,000 hifi reads 1.38
+// without them, 1.57 with them out of line.)
 constexpr int LCS_WARPS = 8;
+template <bool TAILS>
 __global__ void __launch_bounds__(LCS_WARPS * 32, 5) k_refine_lcs(BatchView v, RefScratch rsc, int pass,
                                                                   int32_t bm_words) {
     __shared__ uint32_t s_mask[LCS_WARPS][2 * LCS_BITS_M / 32];
@@ -2956,7 +2960,7 @@ __global__ void __launch_bounds__(LCS_WARPS * 32, 5) k_refine_lcs(BatchView v, R
         if (lane == 0) atomicAdd(&v.mx->refined, 1ULL);
         const int32_t q = J->read, m = v.r_m[q];
         int32_t len;
-        if (!lcs_ranked(m, v.roff[q + 1] - v.roff[q], bm_words)) len = lcs_one(v, J, q, D, D + m, lane);
+        if (TAILS && !lcs_ranked(m, v.roff[q + 1] - v.roff[q], bm_words)) len = lcs_one(v, J, q, D, D + m, lane);
         else if (m <= 512) len = lcs_bits<1, true>(v, J, q, mask, lane);
         else if (m <= 1024) len = lcs_bits<1, false>(v, J, q, mask, lane);
         else if (m <= 2048) len = lcs_bits<2, false>(v, J, q, mask, lane);
@@ -4294,9 +4298,11 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
         c->rchip_smem_set = 1;
     }
     if (p.metric == SHM_BUCKET_LCS) {  // no read is refined on chip under the bucket metrics
+        const bool tails = bp.max_cap > (uint64_t)LCS_BITS_M || bp.max_len > 32 * (int64_t)bm_words;  // (lcs_ranked)
         for (int pass = 0; pass < (v.lead_on ? 2 : 1); pass++) {
-            k_refine_lcs<<<(unsigned)std::max<size_t>(1, warps / LCS_WARPS), LCS_WARPS * 32, 0, s>>>(v, rsc, pass,
-                                                                                                          bm_words);
+            const unsigned grid = (unsigned)std::max<size_t>(1, warps / LCS_WARPS);
+            if (tails) k_refine_lcs<true><<<grid, LCS_WARPS * 32, 0, s>>>(v, rsc, pass, bm_words);
+            else k_refine_lcs<false><<<grid, LCS_WARPS * 32, 0, s>>>(v, rsc, pass, bm_words);
             SHM_CUDA(cudaGetLastError());
             if (pass == 0 && v.lead_on) count_launch();  // the last launch is counted by the stage timer
         }
