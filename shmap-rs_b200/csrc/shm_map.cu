@@ -587,7 +587,11 @@ __device__ void seedprep_one(const BatchView& v, int32_t q, uint32_t P, const Se
     if (tid == 0) seed_epilogue(v, q, m, n_u, n_proc, S, S0, smatch, mxs, halflen, ebound);
 }
 
-constexpr int SEEDP_THREADS = 512;
+// A read's CTA is as wide as it can be: its sort is stages of barriers over
+// arrays in global memory. Stage in ms with 256 / 512 / 1,024 threads: one read
+// of 9,000 k-mers 0.78 / 0.63 / 0.61, of 18,000 4.1 / 2.2 / 1.5; 300 of 9,000 3.2
+// / 2.0 / 1.9; 1,200 12.1 / 8.5 / 7.8.
+constexpr int SEEDP_THREADS = 1024;
 __global__ void __launch_bounds__(SEEDP_THREADS) k_seedprep(BatchView v, const int32_t* __restrict__ list,
                                                             const uint32_t* __restrict__ n_list_d, uint32_t P,
                                                             uint8_t* gscr, size_t gscr_per_cta) {
@@ -4058,7 +4062,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
         const size_t bytes = SEED_BYTES_PER_ELEM * bp.P_g;
         const int grid = (int)std::min<size_t>(bp.n_cap_8192, 296);
         S.seed_gscr.reserve(bytes * (size_t)grid);
-        k_seedprep<<<grid, 256, 0, s2>>>(v, LB + 6 * (size_t)n, NB + 6, bp.P_g, S.seed_gscr.p, bytes);
+        k_seedprep<<<grid, SEEDP_THREADS, 0, s2>>>(v, LB + 6 * (size_t)n, NB + 6, bp.P_g, S.seed_gscr.p, bytes);
         SHM_CUDA(cudaGetLastError());
         count_launch();
     }
