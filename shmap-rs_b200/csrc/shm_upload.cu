@@ -1,21 +1,27 @@
 // Host bytes in ordinary (pageable) memory on their way to the device. The
 // driver's own copy from such memory goes through its staging buffers on the
-// calling thread; here the packing threads fill a context's pinned slots and
-// queue each slot's copy, so the bytes go up as fast as several cores read
+// calling thread; here several threads fill a context's pinned slots, one each,
+// and queue each slot's copy, so the bytes go up as fast as several cores read
 // them. Bytes that are pinned already are copied from where they lie.
+//
+// The threads are the upload's own: on the packing threads it would hold up
+// every context's host mapping, and wait for whole mapping calls itself. While
+// a packing is in flight, in any context, they rest, and the driver's copy on
+// the calling thread goes on by itself: the cores are the packing's.
 //
 // The copy takes this way from 64 MiB on, where both take the same time when
 // the bytes are in the cores' caches (4.9 and 4.7 ms on 16 cores); for more
 // bytes than those hold the threads are faster (240 MiB 24.7 and 11.0 ms), for
-// fewer the driver is (16 MiB 1.1 and 1.7 ms: the threads have to wake, and a
+// fewer the driver is (16 MiB 1.1 and 1.7 ms: the threads have to start, and a
 // slot's copy costs a call). Slots of 256 KiB took 17 ms for 256 MiB, of 1 MiB
 // 12: the queueing calls of all threads take turns.
 #include <algorithm>
 #include <atomic>
-#include <condition_variable>
+#include <chrono>
 #include <cstring>
-#include <deque>
 #include <mutex>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "shm_internal.hpp"
@@ -24,17 +30,13 @@
 namespace shm {
 
 constexpr size_t UPLOAD_SLOT = (size_t)2 << 20;  // bytes
-constexpr size_t UPLOAD_SLOTS = 8;               // 16 MiB a context, made when first needed
+constexpr size_t UPLOAD_SLOTS = 8;               // 16 MiB a context, made when first needed; a thread each
 constexpr size_t UPLOAD_LEAST = (size_t)64 << 20;
 
 struct UploadStage {
     std::mutex use;  // one upload at a time
     uint8_t* pinned = nullptr;
     std::vector<cudaEvent_t> ev;  // slot's last copy
-    // the slots no thread is filling, the longest queued first
-    std::mutex mu;
-    std::condition_variable cv;
-    std::deque<int> idle;
     ~UploadStage() {
         for (cudaEvent_t e : ev)
             if (e) cudaEventDestroy(e);
@@ -53,7 +55,6 @@ struct UploadStage {
                 cudaGetLastError();
                 return false;
             }
-            idle.push_back((int)ev.size());
             ev.push_back(e);
         }
         return true;
@@ -80,31 +81,43 @@ void upload(UploadStage* u, int device, void* dst, const void* src, size_t bytes
         SHM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
         return;
     }
+    std::atomic<size_t> next{0};  // bytes taken
     std::atomic<int> err{(int)cudaSuccess};
-    host_tasks((int)((bytes + UPLOAD_SLOT - 1) / UPLOAD_SLOT), [&](int t) {
-        const size_t at = (size_t)t * UPLOAD_SLOT, n = std::min(UPLOAD_SLOT, bytes - at);
-        int i;
-        {
-            std::unique_lock<std::mutex> g(u->mu);
-            u->cv.wait(g, [&] { return !u->idle.empty(); });  // one comes back when its thread has queued its copy
-            i = u->idle.front();
-            u->idle.pop_front();
-        }
+    // thread i: the next part through slot i, until all are taken or one failed
+    auto work = [&](size_t i) {
         cudaError_t e = cudaSetDevice(device);
-        if (e == cudaSuccess) e = cudaEventSynchronize(u->ev[(size_t)i]);
-        if (e == cudaSuccess) {
-            uint8_t* p = u->pinned + (size_t)i * UPLOAD_SLOT;
+        uint8_t* const p = u->pinned + i * UPLOAD_SLOT;
+        while (e == cudaSuccess && err.load() == (int)cudaSuccess && next.load() < bytes) {
+            const bool rest = packing_now();
+            if (rest && i) {
+                std::this_thread::sleep_for(std::chrono::microseconds(200));
+                continue;
+            }
+            const size_t take = rest ? UPLOAD_SLOT * UPLOAD_SLOTS : UPLOAD_SLOT, at = next.fetch_add(take);
+            if (at >= bytes) break;
+            const size_t n = std::min(take, bytes - at);
+            if (rest) {  // (the caller's)
+                e = cudaMemcpyAsync((uint8_t*)dst + at, (const uint8_t*)src + at, n, cudaMemcpyHostToDevice, s);
+                continue;
+            }
+            if ((e = cudaEventSynchronize(u->ev[i])) != cudaSuccess) break;
             std::memcpy(p, (const uint8_t*)src + at, n);
             e = cudaMemcpyAsync((uint8_t*)dst + at, p, n, cudaMemcpyHostToDevice, s);
-            if (e == cudaSuccess) e = cudaEventRecord(u->ev[(size_t)i], s);
+            const cudaError_t r = cudaEventRecord(u->ev[i], s);
+            if (e == cudaSuccess) e = r;
         }
         if (e != cudaSuccess) err.store((int)e);
-        {
-            std::lock_guard<std::mutex> g(u->mu);
-            u->idle.push_back(i);
-        }
-        u->cv.notify_one();
-    });
+    };
+    std::vector<std::thread> th;
+    try {
+        th.reserve(UPLOAD_SLOTS);
+        const size_t most = std::max(1u, std::thread::hardware_concurrency());
+        for (size_t i = 1; i < std::min(UPLOAD_SLOTS, most); i++) th.emplace_back(work, i);
+    } catch (const std::system_error&) {  // no more threads: those there are do it
+    } catch (const std::bad_alloc&) {
+    }
+    work(0);
+    for (std::thread& t : th) t.join();
     if (err.load() != (int)cudaSuccess) throw shm_cuda_error((cudaError_t)err.load());
 }
 

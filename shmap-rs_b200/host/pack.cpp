@@ -381,26 +381,31 @@ Stream g_stream;
 // from several host threads (one per device, say) take turns.
 static std::mutex g_pack_mu;
 static thread_local bool t_pack_held = false;
+static std::atomic<int> g_packers{0};  // threads that hold the lock or wait for it
+
+static void pack_lock() {
+    g_packers.fetch_add(1);
+    g_pack_mu.lock();
+}
+static void pack_unlock() {
+    g_pack_mu.unlock();
+    g_packers.fetch_sub(1);
+}
+bool packing_now() { return g_packers.load() > 0; }
 
 void pack_reads_host(const uint8_t* seq, int64_t nb, uint32_t* codes, uint32_t* mask) {
     const bool own = !t_pack_held;
-    if (own) g_pack_mu.lock();
+    if (own) pack_lock();
     int tasks = 0;
     auto f = pack_tasks<false>(seq, nb, codes, mask, tasks, 0);
     if (tasks > 0) pool().run(tasks, std::move(f));
     pack_tail<false>(seq, nb, codes + 2 * (nb / 32), mask + nb / 32, nullptr);
-    if (own) g_pack_mu.unlock();
-}
-
-void host_tasks(int n, std::function<void(int)> f) {
-    std::unique_lock<std::mutex> g(g_pack_mu, std::defer_lock);
-    if (!t_pack_held) g.lock();
-    pool().run(n, std::move(f));
+    if (own) pack_unlock();
 }
 
 void pack_reads_host_start(const uint8_t* seq, int64_t nb, uint32_t* codes, int64_t task_groups) {
     if (!t_pack_held) {
-        g_pack_mu.lock();
+        pack_lock();
         t_pack_held = true;
     }
     pool().finish();
@@ -414,7 +419,7 @@ void pack_reads_host_start(const uint8_t* seq, int64_t nb, uint32_t* codes, int6
 int pack_stream_start(const uint8_t* seq, int64_t nb, uint32_t* codes, int64_t task_groups, int chunk_tasks,
                       PackSink* sink, int raw_pct) {
     if (!t_pack_held) {
-        g_pack_mu.lock();
+        pack_lock();
         t_pack_held = true;
     }
     pool().finish();
@@ -470,7 +475,7 @@ void pack_stream_finish() {
     g_stream.chunks = 0;
     if (t_pack_held) {
         t_pack_held = false;
-        g_pack_mu.unlock();
+        pack_unlock();
     }
 }
 
@@ -487,7 +492,7 @@ size_t pack_reads_host_wait(uint32_t* pairs, size_t cap) {
         }
     if (t_pack_held) {
         t_pack_held = false;
-        g_pack_mu.unlock();
+        pack_unlock();
     }
     return n;
 }
@@ -496,7 +501,7 @@ void pack_reads_host_release() {
     if (!t_pack_held) return;
     pool().finish();
     t_pack_held = false;
-    g_pack_mu.unlock();
+    pack_unlock();
 }
 
 size_t packed_code_words(int64_t nb) { return 2 * (size_t)(nb / 32 + 3); }
@@ -521,6 +526,18 @@ extern "C" int shm_internal_pack_reads(const uint8_t* seq, int64_t nb, uint32_t*
     }
     shm::pack_reads_host(seq, nb, codes, mask);
     return 0;
+}
+
+// Test hook (not part of the C ABI of include/shmap_gpu.h): takes the packing,
+// as a call that maps host reads does, or (on = 0) gives it back, both on the
+// same thread.
+extern "C" void shm_internal_pack_hold(int on) {
+    if (on && !shm::t_pack_held) {
+        shm::pack_lock();
+        shm::t_pack_held = true;
+    } else if (!on) {
+        shm::pack_reads_host_release();
+    }
 }
 
 // Test hook (not part of the C ABI of include/shmap_gpu.h): the streamed

@@ -2,7 +2,6 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
-#include <functional>
 
 namespace shm {
 
@@ -35,9 +34,8 @@ struct PackSink {
     virtual bool piece_raw(int worker, const uint8_t* src, size_t first_group, size_t groups) { return false; }
     virtual ~PackSink() = default;
 };
-// Calls f(task) for the tasks 0 .. n - 1 on the packing threads and the
-// caller's (f must not throw), taking its turn among the packings.
-void host_tasks(int n, std::function<void(int)> f);
+// Whether a packing is in flight or waited for, in this process.
+bool packing_now();
 // The number of packing threads (the pool's and the one holding the packing).
 int pack_workers();
 
