@@ -735,6 +735,14 @@ int shm_server_destroy(shm_server* srv) {
     SHM_GUARD_END
 }
 
+// Test hook: what a context has done or holds that no result shows. 0: sketch
+// tables made, 1: bytes of its pinned staging block, 2: reads given a second
+// bucket table before their contributions.
+int64_t shm_internal_ctx_state(const shm_ctx* ctx, int32_t what) {
+    if (!ctx) return -1;
+    return what == 0 ? ctx->m->luts_made : what == 1 ? (int64_t)ctx->m->h_pinned_cap : what == 2 ? ctx->m->tables_ahead : -1;
+}
+
 // Test hook: the admission rule of a server slot (how many of the queued
 // requests one batch takes whole, and how many reads of the front request
 // when it alone is too large), with no device involved.

@@ -3644,6 +3644,7 @@ const SketchLuts* ctx_luts(MapCtx* c, int32_t k) {
         if (S.luts) SHM_CUDA(cudaFree(S.luts));
         S.luts = nullptr;
         S.luts = create_device_luts(k, c->stream);
+        c->luts_made++;
         S.luts_k = k;
     }
     return S.luts;
@@ -3753,6 +3754,7 @@ struct BatchSlot {
     int32_t i0, n;
     int64_t bases;
     uint32_t job_cap;  // set by run_batch: more jobs than this and the batch is mapped again
+    uint32_t pre_most;  // and the most reads put down for a second table ahead (k_bt_init)
 };
 
 // The bucket tables of a batch mapped without waiting for its sizes get at
@@ -3847,6 +3849,7 @@ static void collect_batch(MapCtx* c, const BatchSlot& sl, std::vector<Overflow>&
     c->work[W_REFINE_KMERS] += (int64_t)fin.refine_kmers;
     c->work[W_REFINED] += (int64_t)fin.refined;
     c->work[W_BT2_READS] += (int64_t)(fin.bt2_pack >> BT2_RUN_BITS);
+    c->tables_ahead += std::min(fin.bt_pre, sl.pre_most);  // (the counter goes on past the limit)
     const size_t at = ovf.size();
     for (uint32_t i = 0; i < fin.n_overflow && i < (uint32_t)sl.n; i++)
         ovf.push_back(Overflow{sl.i0 + (int32_t)sl.ovf[4 * i], sl.ovf[4 * i + 1],
@@ -4189,9 +4192,10 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     v.bt2_off = S.bt2_off.p;
     v.bt_pool = bt_slots_alloc;
     v.bt2_spare = spare;
+    sl.pre_most = (uint32_t)std::min<uint64_t>(spare / BT2_MAX * 3 / 4, (uint64_t)n);
     T.begin(STG_AUX);
     k_bt_init<<<wide, 256, 0, s>>>(S.bt.p, S.bt_off.p, n, bt_slots_alloc, Z.r_flags, S.bt_tab.p, v.hw_off, v.r_nproc,
-                                   v.bt_cap, (uint32_t)std::min<uint64_t>(spare / BT2_MAX * 3 / 4, (uint64_t)n), &Z.mx->bt_pre);
+                                   v.bt_cap, sl.pre_most, &Z.mx->bt_pre);
     SHM_CUDA(cudaGetLastError());
     T.end();
     T.begin(STG_CONTRIB);

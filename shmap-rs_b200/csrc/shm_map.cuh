@@ -103,6 +103,8 @@ struct MapCtx {
     size_t h_pack_cap = 0;
     // work counters (always on): see WORK_NAMES
     int64_t work[16] = {};
+    int64_t luts_made = 0;    // sketch tables made
+    int64_t tables_ahead = 0; // reads given a second bucket table before their contributions
     int seed_cta_set = 0;    // k_seedprep_cta's dynamic shared memory allowed
     int rchip_smem_set = 0;  // k_refine_chip's dynamic shared memory allowed
     int refine_smem_set = 0; // k_refine's
