@@ -203,7 +203,7 @@ int shm_sketch(shm_ctx* ctx, const uint8_t* seq, int64_t len, int32_t k, double 
     const int64_t off[2] = {0, len};
     d_off.reserve(2, s);
     SHM_CUDA(cudaMemcpyAsync(d_off.p, off, sizeof off, cudaMemcpyHostToDevice, s));
-    const shm::SketchLuts* L = shm::ctx_luts(ctx->m, k);
+    const shm::SketchLuts* L = shm::ctx_luts(ctx->m, k, false);
     shm::SketchArgs a{};
     a.seq = d_seq.p;
     a.seq_off = d_off.p;
@@ -290,7 +290,7 @@ int shm_index_build(shm_ctx* ctx, const uint8_t* seq, const int64_t* seg_off, in
     SHM_CUDA(cudaSetDevice(ctx->m->device));
     auto* ix = new shm_index();
     ix->s = shm::build_index(seq, seg_off, n_seg, split_names(names, n_seg), k, h_frac, max_matches,
-                             shm::ctx_luts(ctx->m, k), ctx->m->up, ctx->m->stream);
+                             shm::ctx_luts(ctx->m, k, false), ctx->m->up, ctx->m->stream);
     ctx->m->launches += 40;
     *out = ix;
     return SHM_OK;
@@ -365,7 +365,7 @@ int shm_index_build_fasta(shm_ctx* ctx, const shm_fasta* fa, int32_t k, double h
     SHM_CUDA(cudaSetDevice(ctx->m->device));
     auto* ix = new shm_index();
     ix->s = shm::build_index(nullptr, fa->f->offs.data(), fa->f->n, split_names(fa->f->names.c_str(), fa->f->n), k,
-                             h_frac, max_matches, shm::ctx_luts(ctx->m, k), ctx->m->up, ctx->m->stream,
+                             h_frac, max_matches, shm::ctx_luts(ctx->m, k, false), ctx->m->up, ctx->m->stream,
                              fa->f->seq.p);
     ctx->m->launches += 40;
     *out = ix;

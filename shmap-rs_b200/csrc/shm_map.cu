@@ -3525,8 +3525,8 @@ struct MapScratch {
     DevBuf<SweepCand> sweep_scr;
     DevBuf<uint8_t> seed_gscr;
     DevBuf<shm_map_record> out;
-    SketchLuts* luts = nullptr;
-    int32_t luts_k = -1;
+    SketchLuts* luts[2] = {};  // ctx_luts: mapping's, the others'
+    int32_t luts_k[2] = {-1, -1};
     // rarity weights max(c, 1)^-alpha for one (index, alpha), and per-read m_weight
     DevBuf<double> wtab, r_mw;
     double wtab_alpha = 0.0;
@@ -3561,7 +3561,8 @@ void mapctx_destroy(MapCtx* c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->scr) {
-        if (c->scr->luts) cudaFree(c->scr->luts);
+        for (SketchLuts* l : c->scr->luts)
+            if (l) cudaFree(l);
         delete c->scr;
     }
     paf_scratch_free(c->paf);
@@ -3638,16 +3639,17 @@ struct BatchPlan {
     }
 };
 
-const SketchLuts* ctx_luts(MapCtx* c, int32_t k) {
+const SketchLuts* ctx_luts(MapCtx* c, int32_t k, bool mapping) {
     MapScratch& S = *c->scr;
-    if (!S.luts || S.luts_k != k) {
-        if (S.luts) SHM_CUDA(cudaFree(S.luts));
-        S.luts = nullptr;
-        S.luts = create_device_luts(k, c->stream);
-        c->luts_made++;
-        S.luts_k = k;
-    }
-    return S.luts;
+    const int own = mapping ? 0 : 1;
+    for (int i : {own, 1 - own})
+        if (S.luts[i] && S.luts_k[i] == k) return S.luts[i];
+    if (S.luts[own]) SHM_CUDA(cudaFree(S.luts[own]));
+    S.luts[own] = nullptr;
+    S.luts[own] = create_device_luts(k, c->stream);
+    S.luts_k[own] = k;
+    c->luts_made++;
+    return S.luts[own];
 }
 
 // Grow-only pinned host staging of a context (the plan of the batch in flight).
@@ -3880,7 +3882,7 @@ static void run_batch(MapCtx* c, const IndexStorage* ix, const shm_params& p, co
     // / pk_mask, and pk_words code words are readable there (0: the batch's own)
     plan_batch(h_plan, h_offs, n, p.k, p.h_frac, caps, bp, pk_codes ? pk_base : 0);
     H.mark("plan");
-    const SketchLuts* luts = ctx_luts(c, p.k);
+    const SketchLuts* luts = ctx_luts(c, p.k, true);
     const uint64_t kcap = bp.kcap_off[(size_t)n], phtn = bp.pht_off[(size_t)n];
     // the plan goes up in one copy from its own pinned block, by the copy
     // engine, or (plan_mapped) by a kernel reading the block through its

@@ -120,8 +120,11 @@ struct MapCtx {
 MapCtx* mapctx_create(int device, size_t hbm_budget);
 void mapctx_destroy(MapCtx* c);
 
-// The sketch tables of k on the context's device (kept until another k is asked for).
-const SketchLuts* ctx_luts(MapCtx* c, int32_t k);
+// The sketch tables of k on the context's device: mapping calls keep theirs
+// until one maps at another k, sketches and index builds theirs, so that a
+// program that sketches at one k and maps at another makes both once. Either
+// uses the other's where k is the same.
+const SketchLuts* ctx_luts(MapCtx* c, int32_t k, bool mapping);
 // The context's pinned staging block, grown to at least `bytes` (its contents are the last user's).
 uint8_t* pinned_stage(MapCtx* c, size_t bytes);
 
