@@ -4555,6 +4555,45 @@ __global__ void k_mask_scatter(const uint32_t* __restrict__ pairs, uint32_t n, u
         mask[pairs[2 * i]] = pairs[2 * i + 1];
 }
 
+// What a batch's scratch grows by, at most, in device bytes: a k-mer of
+// capacity (kmer_cap: at most 2 r L + 25 of a read of L bases, and at most L)
+// has its hash, position and seed arrays and fewer than four probe slots; a
+// read its bucket tables (first and spare), its share of the jobs with their
+// lists, and its smallest probe table. What does not grow with the batch is
+// left out (refinement scratch, 1 GiB at most; the first 2^20 jobs and spare
+// slots, 0.2 GiB). A buffer that grows again takes a quarter more.
+ScratchCost scratch_cost(const shm_params& p) {
+    const double kmer = sizeof(uint64_t) + 2 * sizeof(uint32_t) + sizeof(SeedRec) + 4.0 * sizeof(ulonglong2) +
+                        (p.metric == SHM_BUCKET_LCS ? 2.0 * sizeof(uint32_t) : 0.0);
+    const double job = sizeof(BucketJob) + 3 * sizeof(uint32_t) + 2.0 * sizeof(SweepCand);
+    ScratchCost c;
+    c.base = 1.25 * kmer * std::min(1.0, 2.0 * std::max(0.0, p.h_frac));
+    c.read = 1.25 * (25 * kmer + 16 * sizeof(ulonglong2) + (double)(fast_bt_slots() + 1024) * (sizeof(BSlot) + 4) +
+                     64 * job + 512);
+    return c;
+}
+
+// The bases a batch of up to `reads` reads and `bases` bases may have for its
+// scratch to fit 3/5 of the device memory that is free or already the
+// context's scratch. At high hash ratios a k-mer of capacity a base makes
+// 2^31 bases more than a device holds; up to SCRATCH_SURE bytes the batch is
+// taken as it is (every batch at the default limits and a ratio below 0.02) and
+// the driver is not asked.
+constexpr double SCRATCH_SURE = 16e9;
+static int64_t batch_bases(MapCtx* c, const shm_params& p, int64_t reads, int64_t bases) {
+    const ScratchCost k = scratch_cost(p);
+    if (k.read * (double)reads + k.base * (double)bases <= SCRATCH_SURE) return bases;
+    const MapScratch& S = *c->scr;
+    size_t held = 0, free_b = 0, total_b = 0;
+    auto add = [&](const auto& b) { held += b.cap * sizeof(*b.p); };
+    add(S.km_h), add(S.km_rs), add(S.sd), add(S.sd_hpre), add(S.pht), add(S.lcs_pos), add(S.lcs_cnt);
+    add(S.bt), add(S.bt_list), add(S.jobs), add(S.cidx), add(S.cfar), add(S.cfar_q), add(S.sweep_scr);
+    SHM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const double most = 0.6 * (double)(free_b + held) - k.read * (double)reads;
+    const double b = std::max(most / k.base, 16e6);
+    return b < (double)bases ? (int64_t)b : bases;
+}
+
 // Batches of at most max_reads reads and max_bases bases (one read at a time
 // in the plain form).
 static std::vector<std::pair<int32_t, int32_t>> cut_batches(const int64_t* offs, int32_t n, bool plain,
@@ -4596,7 +4635,10 @@ void map_device(MapCtx* c, const IndexStorage* ix, const shm_params& p, const ui
                 int32_t n, shm_map_record* d_out, bool plain) {
     SHM_CUDA(cudaSetDevice(c->device));
     const Tuning tu = tuning();
-    const auto batches = cut_batches(h_offs, n, plain, (int32_t)tu.dev_batch_reads, tu.dev_batch_bases,
+    const int64_t most_bases = std::min<int64_t>(tu.dev_batch_bases, n ? h_offs[n] - h_offs[0] : 0);
+    const auto batches = cut_batches(h_offs, n, plain, (int32_t)tu.dev_batch_reads,
+                                     plain ? most_bases
+                                           : batch_bases(c, p, std::min<int64_t>(n, tu.dev_batch_reads), most_bases),
                                      (int32_t)tu.dev_first_batch_reads);
     std::vector<BatchSlot> slots = batch_slots(c, batches, h_offs);
     const std::vector<uint8_t*> plans = plan_blocks(c, batches);
@@ -4778,13 +4820,15 @@ static StreamSink* stream_sink(MapCtx* c, size_t piece_words, int ring, bool raw
 // map slower than the host packs the next one.)
 static std::vector<std::pair<int32_t, int32_t>> cut_stream_batches(const int64_t* offs, int32_t r0, int32_t r1,
                                                                    int64_t first_bases, int64_t last_bases,
-                                                                   int64_t max_bases, int32_t max_reads) {
+                                                                   int64_t max_bases, int32_t max_reads,
+                                                                   int64_t scratch_bases = INT64_MAX) {
     std::vector<std::pair<int32_t, int32_t>> b;
     int64_t tgt = std::max<int64_t>(1, first_bases);
     for (int32_t i = r0; i < r1;) {
         const int64_t rest = offs[r1] - offs[i];
         int64_t lim = rest <= 2 * tgt ? std::max(rest / 2, last_bases) : tgt;
         if (rest - lim < last_bases) lim = rest;  // no last batch smaller than last_bases (its fixed cost)
+        lim = std::min(lim, scratch_bases);  // (batch_bases: no batch of several reads above it)
         int32_t j = i + 1;
         while (j < r1 && j - i < max_reads && offs[j + 1] - offs[i] <= lim) j++;
         b.emplace_back(i, j);
@@ -4826,10 +4870,13 @@ static bool map_host_stream(MapCtx* c, const IndexStorage* ix, const shm_params&
     // every device batch of the call, part by part (their plans and result slots)
     std::vector<std::pair<int32_t, int32_t>> batches;
     std::vector<size_t> part_first;
+    const int64_t whole = std::min<int64_t>(offs[n] - offs[0], tu.dev_batch_bases);
+    const int64_t fits = batch_bases(c, p, std::min<int64_t>(n, tu.dev_batch_reads), whole);
+    const int64_t scratch_bases = fits < whole ? fits : INT64_MAX;
     for (auto [r0, r1] : parts) {
         part_first.push_back(batches.size());
         auto b = cut_stream_batches(offs, r0, r1, tu.host_stream_first_kib * 1024, tu.host_stream_last_kib * 1024,
-                                    tu.dev_batch_bases, (int32_t)tu.dev_batch_reads);
+                                    tu.dev_batch_bases, (int32_t)tu.dev_batch_reads, scratch_bases);
         batches.insert(batches.end(), b.begin(), b.end());
     }
     part_first.push_back(batches.size());
@@ -5026,9 +5073,11 @@ bool map_host(MapCtx* c, const IndexStorage* ix, const shm_params& p, const uint
         return map_host_stream(c, ix, p, seqs, offs, n, out, sink);
     MapScratch& S = *c->scr;
     cudaStream_t s = c->stream;
-    const auto batches =
-        cut_batches(offs, n, plain, (int32_t)tuning().host_batch_reads, tuning().host_batch_bases,
-                    (int32_t)tuning().host_first_batch_reads, true);
+    const Tuning tu = tuning();
+    const int64_t most_bases = plain ? tu.host_batch_bases
+                                     : batch_bases(c, p, std::min<int64_t>(n, tu.host_batch_reads), tu.host_batch_bases);
+    const auto batches = cut_batches(offs, n, plain, (int32_t)tu.host_batch_reads, most_bases,
+                                     (int32_t)tu.host_first_batch_reads, true);
     int64_t max_nb = 0;
     int32_t max_n = 0;
     for (auto [i, j] : batches) {
@@ -5266,4 +5315,11 @@ extern "C" int shm_internal_cut_stream(const int64_t* offs, int32_t n, int64_t f
         out[2 * i + 1] = b[i].second;
     }
     return (int)b.size();
+}
+
+// Test hook: the bound on a batch's growing scratch, a base and a read.
+extern "C" void shm_internal_scratch_cost(const shm_params* p, double* base, double* read) {
+    const shm::ScratchCost c = shm::scratch_cost(*p);
+    *base = c.base;
+    *read = c.read;
 }

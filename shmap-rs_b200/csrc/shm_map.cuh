@@ -128,6 +128,12 @@ const SketchLuts* ctx_luts(MapCtx* c, int32_t k, bool mapping);
 // The context's pinned staging block, grown to at least `bytes` (its contents are the last user's).
 uint8_t* pinned_stage(MapCtx* c, size_t bytes);
 
+// The device bytes a batch's scratch grows by, at most, a base and a read.
+struct ScratchCost {
+    double base, read;
+};
+ScratchCost scratch_cost(const shm_params& p);
+
 // Maps reads [0, n) whose bytes are at d_seq (device) with host offsets
 // h_offs[0..n] (h_offs[0] may be nonzero: bytes are relative to d_seq - h_offs[0]).
 // Writes n records to d_out (device). plain = one read per launch sequence.
