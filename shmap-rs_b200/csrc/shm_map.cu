@@ -4576,13 +4576,15 @@ ScratchCost scratch_cost(const shm_params& p) {
 // The bases a batch of up to `reads` reads and `bases` bases may have for its
 // scratch to fit 3/5 of the device memory that is free or already the
 // context's scratch. At high hash ratios a k-mer of capacity a base makes
-// 2^31 bases more than a device holds; up to SCRATCH_SURE bytes the batch is
-// taken as it is (every batch at the default limits and a ratio below 0.02) and
-// the driver is not asked.
+// 2^31 bases more than a device holds. The driver takes 5 ms to say what is
+// free, so it is asked only where the bound is above SCRATCH_SURE bytes (no
+// batch at the default limits and a ratio below 0.02) and above every bound
+// that was found to fit before, whose scratch the context has kept.
 constexpr double SCRATCH_SURE = 16e9;
 static int64_t batch_bases(MapCtx* c, const shm_params& p, int64_t reads, int64_t bases) {
     const ScratchCost k = scratch_cost(p);
-    if (k.read * (double)reads + k.base * (double)bases <= SCRATCH_SURE) return bases;
+    const double need = k.read * (double)reads + k.base * (double)bases;
+    if (need <= std::max(SCRATCH_SURE, c->scratch_fits)) return bases;
     const MapScratch& S = *c->scr;
     size_t held = 0, free_b = 0, total_b = 0;
     auto add = [&](const auto& b) { held += b.cap * sizeof(*b.p); };
@@ -4591,7 +4593,9 @@ static int64_t batch_bases(MapCtx* c, const shm_params& p, int64_t reads, int64_
     SHM_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const double most = 0.6 * (double)(free_b + held) - k.read * (double)reads;
     const double b = std::max(most / k.base, 16e6);
-    return b < (double)bases ? (int64_t)b : bases;
+    if (b < (double)bases) return (int64_t)b;
+    c->scratch_fits = need;
+    return bases;
 }
 
 // Batches of at most max_reads reads and max_bases bases (one read at a time

@@ -98,6 +98,7 @@ struct MapCtx {
     size_t h_pinned_cap = 0;
     void* h_slots = nullptr;  // per-call batch results
     size_t h_slots_cap = 0;
+    double scratch_fits = 0;  // the largest bound on a batch's scratch that was found to fit (batch_bases)
     UploadStage* up = nullptr;  // uploads from pageable memory
     uint8_t* h_pack = nullptr;  // two slots of packed reads (codes, mask) on their way up
     size_t h_pack_cap = 0;
