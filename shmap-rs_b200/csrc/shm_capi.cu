@@ -696,7 +696,7 @@ int shm_submit(shm_server* srv, const uint8_t* seqs, const int64_t* offs, int32_
     if (n > 0 && (!seqs || !offs || !out)) return fail(SHM_ERR_INVALID, "null argument");
     int v = check_reads(offs, n);
     if (v != SHM_OK) return v;
-    const int64_t mb = shm::server_max_bases(srv->s);
+    const int64_t mb = shm::server_max_read(srv->s);
     for (int32_t i = 0; i < n; i++)
         if (offs[i + 1] - offs[i] > mb)
             return fail(SHM_ERR_INVALID, "read " + std::to_string(i) + " has " + std::to_string(offs[i + 1] - offs[i]) +
@@ -741,6 +741,12 @@ int shm_server_destroy(shm_server* srv) {
 int64_t shm_internal_ctx_state(const shm_ctx* ctx, int32_t what) {
     if (!ctx) return -1;
     return what == 0 ? ctx->m->luts_made : what == 1 ? (int64_t)ctx->m->h_pinned_cap : what == 2 ? ctx->m->tables_ahead : -1;
+}
+
+// Test hook: a server slot's batch limits for its share of the budget (serve_limits).
+void shm_internal_serve_limits(const shm_params* p, size_t share, int32_t cfg_reads, int64_t cfg_bases,
+                               int32_t* max_reads, int64_t* max_bases, int64_t* max_read) {
+    shm::serve_limits(*p, share, shm::ServeConfig{1, cfg_reads, cfg_bases, share}, max_reads, max_bases, max_read);
 }
 
 // Test hook: the admission rule of a server slot (how many of the queued

@@ -8,11 +8,11 @@
 // mapping workers are device slots. Each slot owns a device context of its own
 // (stream, scratch, pinned staging), so the slots' batches run on the device
 // at the same time. A free slot takes the queued requests in arrival order,
-// as many as fit its limits: at most max_batch_reads reads and, in bases, its
-// share of the HBM budget divided by the device bytes a base costs at the
-// index's hash ratio. A request larger than those limits is taken in parts,
-// each the longest run of its next reads that fits (a single read longer than
-// the base limit is refused when submitted), so no batch exceeds the budget.
+// as many as fit its limits: at most max_batch_reads reads and, in reads and
+// bases, what its share of the HBM budget holds (serve_limits). A request
+// larger than those limits is taken in parts, each the longest run of its next
+// reads that fits, at least one (a read too long for a slot is refused when
+// submitted).
 // Requests that arrive while the slots are busy wait in the queue and join
 // the next batch a slot takes.
 //
@@ -104,7 +104,7 @@ struct Server {
     shm_params p;
     int device;
     int32_t max_reads;
-    int64_t max_bases;
+    int64_t max_bases, max_read;
     std::mutex mu;
     std::condition_variable cv_work, cv_done;
     std::deque<Request*> queue;
@@ -237,6 +237,27 @@ static void run_slot(Server* S, Slot* sl) {
     }
 }
 
+// A batch's limits from a slot's share of the budget, by the bound on its
+// scratch (scratch_cost), the reads themselves and their records: the reads
+// the configuration allows, or as many as half the share holds, and the bases
+// that the rest holds. (128 bytes a sketched k-mer with no count of the reads,
+// as before, let 15,700 hifi-like reads take 1.8 times a share of 1 GiB.) Two
+// slots of 8 GiB at r = 0.01 are limited by the configuration alone; 512 MiB
+// hold 3,715 reads and 73 Mbases. What does not grow with the batch is beside
+// the share. max_read is the longest read a request may hold, mapped by itself
+// when it is longer than max_bases.
+void serve_limits(const shm_params& p, size_t share, const ServeConfig& cfg, int32_t* max_reads, int64_t* max_bases,
+                  int64_t* max_read) {
+    const ScratchCost k = scratch_cost(p);
+    const double read = k.read + sizeof(shm_map_record), base = k.base + 1.25;
+    *max_reads = (int32_t)std::max(1.0, std::min((double)cfg.max_batch_reads, 0.5 * (double)share / read));
+    const double bases = std::max(1.0, ((double)share - read * (double)*max_reads) / base);
+    *max_bases = bases < (double)cfg.max_batch_bases ? (int64_t)bases : cfg.max_batch_bases;
+    const double longest = std::max(1.0, (double)share / (1.0 + 128.0 * p.h_frac));
+    *max_read = longest < (double)cfg.max_batch_bases ? (int64_t)longest : cfg.max_batch_bases;
+    *max_bases = std::min(*max_bases, *max_read);
+}
+
 Server* server_create(int device, const IndexStorage* ix, const shm_params& p, const ServeConfig& cfg) {
     auto* S = new Server();
     S->ix = ix;
@@ -251,13 +272,7 @@ Server* server_create(int device, const IndexStorage* ix, const shm_params& p, c
             SHM_CUDA(cudaMemGetInfo(&fr, &tot));
             budget = fr / 2;
         }
-        // device bytes a batch costs per base: the read itself plus, per
-        // sketched k-mer (h_frac of the bases), its sketch entry, seed record,
-        // probe-table slots, bucket slots and jobs (128 bytes bounds them)
-        const double per_base = 1.0 + 128.0 * p.h_frac;
-        const int64_t by_budget = (int64_t)((double)(budget / (size_t)nslots) / per_base);
-        S->max_reads = std::max(1, cfg.max_batch_reads);
-        S->max_bases = std::max<int64_t>(1, std::min<int64_t>(cfg.max_batch_bases, by_budget));
+        serve_limits(p, budget / (size_t)nslots, cfg, &S->max_reads, &S->max_bases, &S->max_read);
         S->slots = std::vector<Slot>((size_t)nslots);
         for (Slot& sl : S->slots) {
             sl.c = mapctx_create(device, budget / (size_t)nslots);
@@ -273,7 +288,7 @@ Server* server_create(int device, const IndexStorage* ix, const shm_params& p, c
     return S;
 }
 
-int64_t server_max_bases(const Server* S) { return S->max_bases; }
+int64_t server_max_read(const Server* S) { return S->max_read; }
 
 uint64_t server_submit(Server* S, const uint8_t* seqs, const int64_t* offs, int32_t n, shm_map_record* out) {
     auto* r = new Request();

@@ -33,8 +33,11 @@ struct Server;
 // min(reads[0], max_reads) of them) that fit, at least one; else *part = 0.
 size_t admit_parts(const int64_t* reads, const int64_t* bases, size_t n, const int64_t* front_lens,
                    int64_t max_reads, int64_t max_bases, int64_t* part);
+// The limits of a slot's batches, given the device bytes that are its share.
+void serve_limits(const shm_params& p, size_t share, const ServeConfig& cfg, int32_t* max_reads, int64_t* max_bases,
+                  int64_t* max_read);
 // The longest read, in bases, a request may hold.
-int64_t server_max_bases(const Server* s);
+int64_t server_max_read(const Server* s);
 
 Server* server_create(int device, const IndexStorage* ix, const shm_params& p, const ServeConfig& cfg);
 uint64_t server_submit(Server* s, const uint8_t* seqs, const int64_t* offs, int32_t n, shm_map_record* out);
