@@ -183,6 +183,11 @@ int shm_ctx_work_stats(const shm_ctx* ctx, int64_t* out, int n) {
 
 const char* shm_work_stat_name(int i) { return i >= 0 && i < shm::N_WORK ? shm::WORK_NAMES[i] : ""; }
 
+// Selected windows that come back from shm_sketch at a time, two such pieces in
+// the context's pinned block (12 MiB), which it keeps: the whole sketch there
+// was 12 bytes a window for good, 3.75 GB after 250 Mbases at a ratio of 1.
+constexpr size_t SKETCH_PIECE = (size_t)1 << 19;
+
 int shm_sketch(shm_ctx* ctx, const uint8_t* seq, int64_t len, int32_t k, double h_frac, int32_t offset, int32_t* r,
                uint64_t* h, uint8_t* strand, int64_t cap, int64_t* n_out) {
     if (!ctx || !n_out || (len > 0 && !seq)) return fail(SHM_ERR_INVALID, "null argument");
@@ -233,12 +238,14 @@ int shm_sketch(shm_ctx* ctx, const uint8_t* seq, int64_t len, int32_t k, double 
     }
     shm::exclusive_scan_u32(d_cnt.p, d_out.p, parts, s);
     uint32_t total = 0;
-    size_t room = (size_t)nw, first = std::min(room, (size_t)(1.25 * h_frac * (double)nw) + 512);
+    const double expected = 1.25 * std::max(0.0, std::min(1.0, h_frac)) * (double)nw;
+    size_t room = (size_t)nw, first = std::min(room, (size_t)expected + 512);
     if (nw > (int64_t)1 << 22) {
         SHM_CUDA(cudaMemcpyAsync(&total, d_out.p + parts, sizeof total, cudaMemcpyDeviceToHost, s));
         SHM_CUDA(cudaStreamSynchronize(s));
         room = first = total;
     }
+    first = std::min(first, 2 * SKETCH_PIECE);
     d_h.reserve(room + 1, s);
     d_rs.reserve(room + 1, s);
     a.out_h = d_h.p;
@@ -260,20 +267,36 @@ int shm_sketch(shm_ctx* ctx, const uint8_t* seq, int64_t len, int32_t k, double 
     }
     SHM_CUDA(cudaStreamSynchronize(s));
     std::memcpy(&total, pin, sizeof total);
-    if (total > first) {  // more than expected (repeats): all of it again
-        pin = shm::pinned_stage(ctx->m, 12 * (size_t)total);
-        hh = (uint64_t*)pin;
-        rs = (uint32_t*)(hh + total);
-        SHM_CUDA(cudaMemcpyAsync(hh, d_h.p, sizeof(uint64_t) * total, cudaMemcpyDeviceToHost, s));
-        SHM_CUDA(cudaMemcpyAsync(rs, d_rs.p, sizeof(uint32_t) * total, cudaMemcpyDeviceToHost, s));
-        SHM_CUDA(cudaStreamSynchronize(s));
-    }
     *n_out = total;
     if ((int64_t)total > cap) return fail(SHM_ERR_CAPACITY, "output capacity too small");
-    for (uint32_t i = 0; i < total; i++) {
-        if (r) r[i] = (int32_t)(rs[i] >> 1);
-        if (h) h[i] = hh[i];
-        if (strand) strand[i] = (uint8_t)(rs[i] & 1u);
+    auto emit = [&](size_t at, size_t n, const uint64_t* ph, const uint32_t* prs) {
+        for (size_t i = 0; i < n; i++) {
+            if (r) r[at + i] = (int32_t)(prs[i] >> 1);
+            if (h) h[at + i] = ph[i];
+            if (strand) strand[at + i] = (uint8_t)(prs[i] & 1u);
+        }
+    };
+    emit(0, std::min<size_t>(first, total), hh, rs);
+    // the rest in pieces, one on its way while the one before is unpacked
+    if (total > first) {
+        shm::StreamEvent ev[2];
+        pin = shm::pinned_stage(ctx->m, 2 * 12 * SKETCH_PIECE);
+        auto piece = [&](size_t at) { return std::min<size_t>(SKETCH_PIECE, total - at); };
+        auto ask = [&](size_t at, int slot) {
+            uint64_t* ph = (uint64_t*)(pin + 12 * SKETCH_PIECE * (size_t)slot);
+            SHM_CUDA(cudaMemcpyAsync(ph, d_h.p + at, sizeof(uint64_t) * piece(at), cudaMemcpyDeviceToHost, s));
+            SHM_CUDA(cudaMemcpyAsync(ph + SKETCH_PIECE, d_rs.p + at, sizeof(uint32_t) * piece(at),
+                                     cudaMemcpyDeviceToHost, s));
+            SHM_CUDA(cudaEventRecord(ev[slot].e, s));
+        };
+        ask(first, 0);
+        int slot = 0;
+        for (size_t at = first; at < total; at += SKETCH_PIECE, slot ^= 1) {
+            if (total - at > SKETCH_PIECE) ask(at + SKETCH_PIECE, slot ^ 1);
+            SHM_CUDA(cudaEventSynchronize(ev[slot].e));
+            const uint64_t* ph = (const uint64_t*)(pin + 12 * SKETCH_PIECE * (size_t)slot);
+            emit(at, piece(at), ph, (const uint32_t*)(ph + SKETCH_PIECE));
+        }
     }
     return SHM_OK;
     SHM_GUARD_END

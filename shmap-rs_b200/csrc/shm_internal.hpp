@@ -110,6 +110,15 @@ struct PoolBuf {
     PoolBuf& operator=(const PoolBuf&) = delete;
 };
 
+// An event for waits (no timing) of one call.
+struct StreamEvent {
+    cudaEvent_t e = nullptr;
+    StreamEvent() { SHM_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)); }
+    ~StreamEvent() { cudaEventDestroy(e); }
+    StreamEvent(const StreamEvent&) = delete;
+    StreamEvent& operator=(const StreamEvent&) = delete;
+};
+
 struct IndexStorage {
     DevIndex dev{};
     PoolBuf<uint32_t> seg_off, key_off, hits, hit_fw, dir, ref_rs;
