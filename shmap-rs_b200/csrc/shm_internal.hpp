@@ -146,9 +146,6 @@ IndexStorage* load_index(const char* path, cudaStream_t s);
 // The checks load_index makes, on the host alone (no device is touched).
 void check_index_file(const char* path);
 
-// The segments' bases are read from h_seq (host) or, when d_seq is given,
-// from device memory (d_seq + seg_off[i], 32 readable bytes past the end).
-// luts: the tables of k (create_device_luts).
 // Pinned staging for copies from pageable host memory, one a context (see
 // shm_upload.cu), and the copy: dst holds the bytes once s has reached this
 // point; pageable src may be changed on return, pinned src once s has got there.
@@ -157,6 +154,9 @@ UploadStage* upload_stage_create();
 void upload_stage_destroy(UploadStage* u);
 void upload(UploadStage* u, int device, void* dst, const void* src, size_t bytes, cudaStream_t s);
 
+// The segments' bases are read from h_seq (host) or, when d_seq is given,
+// from device memory (d_seq + seg_off[i], 32 readable bytes past the end).
+// luts: the tables of k (create_device_luts).
 IndexStorage* build_index(const uint8_t* h_seq, const int64_t* seg_off, int32_t n_seg,
                           const std::vector<std::string>& names, int32_t k, double h_frac, int32_t max_matches,
                           const SketchLuts* luts, UploadStage* up, cudaStream_t s, const uint8_t* d_seq = nullptr);

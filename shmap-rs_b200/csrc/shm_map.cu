@@ -1192,9 +1192,10 @@ __device__ void seedprep_cta(const BatchView& v, int32_t q, SeedCta<C, NT>& T) {
         pout = pout == T.P0 ? T.P1 : T.P0;
     }
 
-    // seeding prefix (seeding.rs:101), as in seedprep_count
-    const bool chip = refine_on_chip(v.P, m, halflen);
-    const bool pht = !chip && v.P.metric != MET_BUCKET_SH;
+    // seeding prefix (seeding.rs:101), as in seedprep_count; no read of this
+    // form is refined on chip
+    static_assert(RCHIP_M <= (int)SEEDC_C, "reads refined on chip are prepared by a warp");
+    const bool pht = v.P.metric != MET_BUCKET_SH;
     uint32_t po_carry = 0, l_np = 0, l_s0 = 0, l_max = 0;
     uint64_t pc_carry = 0, l_sm = 0, l_eb = 0;
     for (uint32_t c0 = 0; c0 < n_u; c0 += NT) {
@@ -1207,7 +1208,6 @@ __device__ void seedprep_cta(const BatchView& v, int32_t q, SeedCta<C, NT>& T) {
         const uint64_t pc = pc_carry + block_scan_excl<uint64_t>((uint64_t)cnt, T.sw64, &T.t64);
         if (valid) {
             v.sd[kb + i] = SeedRec{T.Ra()[g], cnt, os, po};
-            if (chip) v.sd_h[kb + i] = T.Sh[g];
             pout[i] = (uint16_t)po;  // (below m <= C)
             if ((int64_t)po < (int64_t)S) {
                 v.sd_hpre[kb + i] = (uint32_t)pc;
@@ -1666,12 +1666,11 @@ __global__ void __launch_bounds__(256, 4) k_contrib2(BatchView v) {
     }
 }
 
-// Empties the first *total slots (the total is read on the device).
 // Clears the batch's bucket tables, the first `pool` slots at most: a read
 // whose table would end past the pool is flagged (mapped again) before any
 // kernel touches it.
-// A read with a capped table, at least a processed seed and BT_PRE hits for each
-// of its slots is put down for a second table at once: it would fill the first
+// A read with a capped table and, for each of its slots, at least a processed
+// seed and BT_PRE hits is put down for a second table at once: it would fill the first
 // and have its contributions made twice (12,500 dense reads, a fifth of them
 // in satellites: 4.25 ms, 3.2 so). By hits alone the rule also takes reads of
 // few seeds, whose hits share buckets and whose first table does (150,000 hifi
