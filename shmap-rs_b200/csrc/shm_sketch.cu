@@ -851,23 +851,26 @@ static int launch_bits(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t
 bool sketch_bits_takes(int32_t k, uint64_t thr) { return k >= SKB_KMIN && k <= SKB_KMAX && thr <= (uint64_t)1 << 62; }
 // ... and of the reads those where a warp's tile of windows is all there is to
 // do (few bases, short reads, whose lists' counters the rolling kernels do not
-// wait for). Sketch stage in ms, planes / rolled:
+// wait for). Sketch stage in ms, planes / rolled (k = 25):
 //   bases / read length   r = 0.25      0.3           0.4           0.5           0.7           1
-//     150 / 150           0.01 / 0.03   0.01 / 0.03   0.01 / 0.03   0.01 / 0.03   0.19 / 0.04   0.21 / 0.05
-//     9 k / 9 k           0.05 / 0.06   0.06 / 0.07   0.08 / 0.05   0.10 / 0.05   0.19 / 0.06   0.23 / 0.06
-//     300 k / 150         0.09 / 0.10   0.11 / 0.08   0.14 / 0.08   0.17 / 0.09   0.25 / 0.09   0.38 / 0.10
-//     300 k / 10 k        0.06 / 0.11   0.07 / 0.11   0.10 / 0.12   0.12 / 0.14   0.23 / 0.20   0.28 / 0.30
-//     3 M / 1.5 k         -             0.09 / 0.12   0.11 / 0.11   0.14 / 0.12   0.24 / 0.13   0.31 / 0.13
-//     3 M / 10 k          0.08 / 0.15   0.08 / 0.19   0.11 / 0.25   0.13 / 0.33   0.23 / 0.48   0.29 / 0.67
+//     150 / 150           0.01 / 0.03   0.01 / 0.04   0.01 / 0.04   0.01 / 0.04   0.01 / 0.05   0.01 / 0.07
+//     3,840 / 3,840       0.06 / 0.09   0.07 / 0.09   0.09 / 0.07   0.11 / 0.07   0.16 / 0.08   0.24 / 0.08
+//     9 k / 9 k           0.06 / 0.09   0.07 / 0.09   0.09 / 0.07   0.12 / 0.08   0.16 / 0.08   0.25 / 0.10
+//     300 k / 150         0.09 / 0.10   0.10 / 0.10   0.14 / 0.09   0.18 / 0.10   0.26 / 0.11   0.38 / 0.10
+//     300 k / 10 k        0.06 / 0.08   0.07 / 0.09   0.09 / 0.10   0.12 / 0.12   0.17 / 0.16   0.27 / 0.19
+//     3 M / 1.5 k         0.07 / 0.11   0.08 / 0.12   0.11 / 0.11   0.14 / 0.12   0.20 / 0.15   0.31 / 0.15
+//     3 M / 10 k          0.07 / 0.16   0.08 / 0.21   0.10 / 0.29   0.13 / 0.37   0.19 / 0.55   0.29 / 0.78
 //     30 M / 150          -             0.54 / 0.41   0.71 / 0.46   0.89 / 0.52   1.27 / 0.64   1.82 / 0.78
 //     30 M / 1.5 k        -             0.28 / 0.45   0.38 / 0.49   0.48 / 0.54   0.71 / 0.64   1.09 / 0.48
 //     30 M / 10 k         0.23 / 0.50   0.27 / 0.62   0.36 / 0.82   0.46 / 1.05   0.67 / 1.50   1.05 / 1.92
 bool sketch_bits_reads(int32_t k, uint64_t thr, int64_t bases, int32_t n) {
     if (k < SKB_KMIN || k > SKB_KMAX) return false;
     if (thr <= (uint64_t)1 << 62) return true;
+    // a tile (3,840 windows) or less: 12 us and 60 ns a selected window, one warp's
+    // rounds, against some 65 us
+    if (bases <= 3840) return (uint64_t)bases * (thr >> 32) <= (uint64_t)900 << 32;
     if (thr > (uint64_t)1 << 63) return bases > 300000 && bases > 2000 * (int64_t)n;
-    // (a tile has 3,840 windows)
-    return bases <= 3840 || (bases > 500 * (int64_t)n && (thr <= UINT64_MAX / 3 || bases > 100000));
+    return bases > 500 * (int64_t)n && (thr <= UINT64_MAX / 3 || bases > 100000);
 }
 void launch_sketch_bits(const SketchArgs& a, const SketchTabs* tabs, cudaStream_t s) { launch_bits(a, tabs, s); }
 uint32_t ordered_warps(const SketchArgs& a) {
