@@ -2948,6 +2948,9 @@ __global__ void __launch_bounds__(REFINE_WARPS * 32, 4) k_refine_rarity(BatchVie
 // bucket_SH's does. (The tails out of line and only where they can be needed:
 // 20 reads of 0.9 Mb take 6.2 ms with them inline, 5.8 so, 2,000 hifi reads 1.38
 // without them, 1.57 with them out of line.)
+// Reads on tails are refined in the first pass whole: a window of theirs is tens
+// of milliseconds of one warp, and the second pass waited for the first one's
+// (20 reads of 0.9 Mb: 41 ms so, 40 to 73 by min_diff with their leads first).
 constexpr int LCS_WARPS = 8;
 template <bool TAILS>
 __global__ void __launch_bounds__(LCS_WARPS * 32, 5) k_refine_lcs(BatchView v, RefScratch rsc, int pass,
@@ -2959,11 +2962,12 @@ __global__ void __launch_bounds__(LCS_WARPS * 32, 5) k_refine_lcs(BatchView v, R
     uint32_t* const mask = s_mask[wib];
     for (uint32_t jq; (jq = next_far(v, lane, pass)) != UINT32_MAX;) {
         BucketJob* J = v.jobs + jq;
-        if (!refined_in(v, *J, jq, pass)) continue;
+        const bool tails = TAILS && !lcs_ranked(v.r_m[J->read], v.roff[J->read + 1] - v.roff[J->read], bm_words);
+        if (tails ? pass != 0 : !refined_in(v, *J, jq, pass)) continue;
         if (lane == 0) atomicAdd(&v.mx->refined, 1ULL);
         const int32_t q = J->read, m = v.r_m[q];
         int32_t len;
-        if (TAILS && !lcs_ranked(m, v.roff[q + 1] - v.roff[q], bm_words)) len = lcs_one(v, J, q, D, D + m, lane);
+        if (tails) len = lcs_one(v, J, q, D, D + m, lane);
         else if (m <= 512) len = lcs_bits<1, true>(v, J, q, mask, lane);
         else if (m <= 1024) len = lcs_bits<1, false>(v, J, q, mask, lane);
         else if (m <= 2048) len = lcs_bits<2, false>(v, J, q, mask, lane);

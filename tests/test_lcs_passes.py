@@ -1,5 +1,6 @@
 """bucket_LCS refines in two passes, the reads' leads first, only where that
-leaves candidates out: not under absolute positions."""
+leaves candidates out: not under absolute positions, and not the reads of more
+than 4,096 k-mers, whose windows are too long to wait for one another."""
 import numpy as np
 import pytest
 
@@ -33,5 +34,6 @@ def test_candidates_refined(gpu_ctx, n, opts, all_refined):
     assert not mm, mm
     cands, refined = (after[f] - before[f] for f in ("candidates", "refined_candidates"))
     assert cands > len(rec)
+    all_refined = all_refined or n - k + 1 > 4_096
     assert refined == cands if all_refined else refined < cands, (refined, cands)
     g.close()
