@@ -1041,6 +1041,71 @@ __device__ __forceinline__ void block_scan_words(uint32_t* X, uint32_t n, uint32
     __syncthreads();
 }
 
+// Inserts n k-mers into hash order, by one thread.
+__device__ __forceinline__ void seed_insert(uint64_t* Sh, uint32_t* Srs, uint32_t n) {
+    for (uint32_t x = 1; x < n; x++) {
+        const uint64_t hx = Sh[x];
+        const uint32_t rx = Srs[x];
+        uint32_t y = x;
+        while (y > 0 && Sh[y - 1] > hx) {
+            Sh[y] = Sh[y - 1];
+            Srs[y] = Srs[y - 1];
+            y--;
+        }
+        Sh[y] = hx;
+        Srs[y] = rx;
+    }
+}
+
+// A bucket of seedprep_cta's hash order that is larger than SEED_BUCKET, by a
+// warp: one hash after another in ascending order, its k-mers counted and its
+// smallest r << 1 | strand found, which is all that is wanted of them, then
+// both written over the bucket. Reads of tandem arrays have a few hashes
+// hundreds of times each; one thread inserting them took a step a k-mer, and
+// where two such hashes fell into one bucket a step a pair (a read of 1,500
+// k-mers of 12 bases from an array: the stage 0.33 ms so, 0.14 by a warp, as
+// other reads; 6,000 dense reads 1.11 and 1.06). More than 32 hashes in a
+// bucket, at one a bucket on average, are inserted. Classes of up to 1,024
+// k-mers insert, as the warps of the smaller reads do: their arrays' reads are
+// tens of microseconds beside others, and with them done sooner the class below
+// started into the warps' kernel (40,000 hifi reads 0.80 ms, 0.76 so).
+constexpr uint32_t SEED_BUCKET = 16, SEED_INSERT_C = 1024;
+__device__ __noinline__ void seed_bucket_warp(uint64_t* Sh, uint32_t* Srs, uint32_t n, int lane) {
+    uint64_t mine_h = 0, prev = 0;  // lane u keeps hash u
+    uint32_t mine_n = 0, mine_r = 0, done = 0;
+    int u = 0;
+    for (; done < n && u < 32; u++) {
+        uint64_t lo = ~0ULL;
+        for (uint32_t x = lane; x < n; x += 32)
+            if ((u == 0 || Sh[x] > prev) && Sh[x] < lo) lo = Sh[x];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) lo = min((unsigned long long)lo, __shfl_xor_sync(0xffffffffu, (unsigned long long)lo, o));
+        uint32_t c = 0, r = UINT32_MAX;
+        for (uint32_t x = lane; x < n; x += 32)
+            if (Sh[x] == lo) {
+                c++;
+                r = min(r, Srs[x]);
+            }
+        c = __reduce_add_sync(0xffffffffu, c);
+        r = __reduce_min_sync(0xffffffffu, r);
+        if (lane == u) mine_h = lo, mine_n = c, mine_r = r;
+        done += c;
+        prev = lo;
+    }
+    __syncwarp();
+    if (done < n) {
+        if (lane == 0) seed_insert(Sh, Srs, n);
+        return;
+    }
+    for (int j = 0; j < u; j++) {
+        const uint64_t h = __shfl_sync(0xffffffffu, mine_h, j);
+        const uint32_t c = __shfl_sync(0xffffffffu, mine_n, j), r = __shfl_sync(0xffffffffu, mine_r, j);
+        for (uint32_t x = lane; x < c; x += 32) Sh[x] = h, Srs[x] = r;
+        Sh += c;
+        Srs += c;
+    }
+}
+
 template <uint32_t C, int NT>
 __device__ void seedprep_cta(const BatchView& v, int32_t q, SeedCta<C, NT>& T) {
     constexpr int NW = NT / 32, ND = 1 << SEEDC_DIGIT;
@@ -1056,6 +1121,7 @@ __device__ void seedprep_cta(const BatchView& v, int32_t q, SeedCta<C, NT>& T) {
     const uint32_t Ht = max((uint32_t)NT, (uint32_t)pow2_ceil(m));  // <= C
     const uint64_t mul = v.P.slot_mul[31 - __clz(Ht)];
     for (uint32_t i = tid; i < Ht; i += NT) T.Rc[i] = 0;
+    if (C > SEED_INSERT_C && tid == 0) T.RH[0] = 0;  // large buckets, listed in P1
     __syncthreads();
 #pragma unroll 4
     for (uint32_t i = tid; i < m; i += NT) atomicAdd(&T.Rc[(uint32_t)__umul64hi(v.km_h[kb + i], mul)], 1u);
@@ -1071,20 +1137,21 @@ __device__ void seedprep_cta(const BatchView& v, int32_t q, SeedCta<C, NT>& T) {
     __syncthreads();
     for (uint32_t b = tid; b < Ht; b += NT) {  // bucket b spans [Rc[b-1], Rc[b])
         const uint32_t s0 = b ? T.Rc[b - 1] : 0u, e1 = T.Rc[b];
-        for (uint32_t x = s0 + 1; x < e1; x++) {
-            const uint64_t hx = T.Sh[x];
-            const uint32_t rx = T.Srs[x];
-            uint32_t y = x;
-            while (y > s0 && T.Sh[y - 1] > hx) {
-                T.Sh[y] = T.Sh[y - 1];
-                T.Srs[y] = T.Srs[y - 1];
-                y--;
-            }
-            T.Sh[y] = hx;
-            T.Srs[y] = rx;
+        if (C > SEED_INSERT_C && e1 - s0 > SEED_BUCKET) {
+            T.P1[atomicAdd(&T.RH[0], 1u)] = (uint16_t)b;
+            continue;
         }
+        if (e1 > s0) seed_insert(T.Sh + s0, T.Srs + s0, e1 - s0);
     }
     __syncthreads();
+    if (C > SEED_INSERT_C && T.RH[0]) {
+        const uint32_t n_big = T.RH[0];
+        for (uint32_t i = wid; i < n_big; i += NW) {
+            const uint32_t b = T.P1[i], s0 = b ? T.Rc[b - 1] : 0u;
+            seed_bucket_warp(T.Sh + s0, T.Srs + s0, T.Rc[b] - s0, lane);
+        }
+        __syncthreads();
+    }
     // groups of equal hashes, compacted in place (src/shmap/seeding.rs:45-67):
     // a thread's elements are in registers before anything is written; Rc gets
     // each group's first element, Srs its smallest r << 1 | strand
