@@ -24,9 +24,13 @@
 //     coalesced at their place; each header's position and the number of
 //     sequence bytes before it;
 //  4. per header: its name's length, then (after a scan) the name itself.
-// Bound by the two reads and the write of the bytes. (Byte by byte, in three
-// passes over chunks staged by single bytes, 249 MB in two files took 6.5 ms;
-// now 0.43 ms: counts 0.12, carry 0.06, write 0.25.)
+// Not bound by memory: 125 MB of 100-base lines are counted in 0.061 ms and
+// written in 0.129, at 2.1 and 1.9 TB/s of the 6.5 a copy reaches. Both passes
+// issue in 61 to 71% of the cycles (0.31 and 0.75 warp instructions a byte:
+// the masks and the per-line steps) and wait at the barriers of the chunk's
+// scans; the carry between them, 0.037 ms, is one block's chain of loads over
+// the chunks. (Byte by byte, in three passes over chunks staged by single
+// bytes, 249 MB in two files took 6.5 ms; now 0.43.)
 #include <cstring>
 #include <string>
 #include <vector>
