@@ -65,6 +65,9 @@ inline void pool_put(void* p, size_t bytes, cudaStream_t s) {
     if (bytes > POOL_MOST) cudaFree(p);  // (waits for the device)
     else cudaFreeAsync(p, s);
 }
+// The bytes of the pool that objects hold for long (PoolBuf) changed by delta:
+// what the pool keeps of freed memory comes on top of them.
+void pool_live(int64_t delta);
 
 // A temporary of work queued on one stream: given back on that stream, behind
 // its last use.
@@ -99,11 +102,16 @@ struct PoolBuf {
         if (p) throw shm_cuda_error(cudaErrorInvalidValue);  // made once
         bytes = n * sizeof(T);
         p = (T*)pool_get(bytes, s);
+        if (bytes <= POOL_MOST) pool_live((int64_t)bytes);
     }
     ~PoolBuf() {
         if (!p) return;
         cudaDeviceSynchronize();
         pool_put(p, bytes, nullptr);
+        if (bytes <= POOL_MOST) try {
+                pool_live(-(int64_t)bytes);
+            } catch (...) {  // (the driver is gone)
+            }
     }
     PoolBuf() = default;
     PoolBuf(const PoolBuf&) = delete;

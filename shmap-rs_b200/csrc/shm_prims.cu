@@ -16,25 +16,49 @@ namespace shm {
 // keeps up to POOL_KEEP bytes of freed memory, so that a call after a
 // synchronize does not map memory again (an index of 155 Mbp took 16 ms to
 // build, most of it in some forty cudaMalloc and cudaFree calls; what is freed
-// beyond that goes back to the device at the next synchronize).
+// beyond that goes back to the device at the next synchronize). The driver's
+// threshold counts what is in use too, so it moves with the bytes of the
+// objects that live in the pool (pool_live): at a fixed one, a program that
+// kept an index of 3.1 Gbp had every freed block unmapped at the next
+// synchronize, and FASTA of 155 Mbp and 4,000 reads beside it took 18 ms to
+// parse, index and map (and now and then 60 to 800), 11.9 so.
 constexpr uint64_t POOL_KEEP = (uint64_t)1 << 30;
-static cudaMemPool_t prim_pool() {
-    static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
+struct DevPool {
+    cudaMemPool_t pool = nullptr;
+    uint64_t live = 0;  // bytes of PoolBufs
+    void set_threshold() {
+        uint64_t keep = live + POOL_KEEP;
+        SHM_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+};
+static std::mutex g_pool_mu;
+// The current device's pool (under g_pool_mu).
+static DevPool& dev_pool() {
+    static DevPool pools[64];
     int dev = 0;
     SHM_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> g(mu);
     if (dev < 0 || dev >= 64) throw shm_cuda_error(cudaErrorInvalidDevice);
-    if (!pools[dev]) {
+    DevPool& d = pools[dev];
+    if (!d.pool) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
-        SHM_CUDA(cudaMemPoolCreate(&pools[dev], &props));
-        uint64_t keep = POOL_KEEP;
-        SHM_CUDA(cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep));
+        SHM_CUDA(cudaMemPoolCreate(&d.pool, &props));
+        d.set_threshold();
     }
-    return pools[dev];
+    return d;
+}
+static cudaMemPool_t prim_pool() {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    return dev_pool().pool;
+}
+
+void pool_live(int64_t delta) {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    DevPool& d = dev_pool();
+    d.live += (uint64_t)delta;
+    d.set_threshold();
 }
 
 void* pool_get(size_t bytes, cudaStream_t s) {
@@ -332,3 +356,17 @@ bool radix_sort_pairs(uint64_t* k0, uint32_t* v0, uint64_t* k1, uint32_t* v1, si
 }
 
 }  // namespace shm
+
+// Test hook (not part of the C ABI of include/shmap_gpu.h): bytes of the current
+// device's pool, reserved and in use.
+extern "C" int shm_internal_pool_bytes(uint64_t* reserved, uint64_t* used) {
+    try {
+        const cudaMemPool_t p = shm::prim_pool();
+        return cudaMemPoolGetAttribute(p, cudaMemPoolAttrReservedMemCurrent, reserved) == cudaSuccess &&
+                       cudaMemPoolGetAttribute(p, cudaMemPoolAttrUsedMemCurrent, used) == cudaSuccess
+                   ? 0
+                   : -1;
+    } catch (...) {
+        return -1;
+    }
+}
